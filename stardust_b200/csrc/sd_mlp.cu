@@ -382,134 +382,336 @@ __global__ void __launch_bounds__(tc::kThreads, 4) k_mlp_infer_tc(const float* _
     }
 }
 
-// ---- training: generic BF16 GEMM with FP32 accumulation ------------------------------
-// C_part[split][m][n] = sum_{k in split} opA[m][k] * opB[k][n]
-//   opA[m][k] = TA ? A[k*lda + m] : A[m*lda + k],  opB[k][n] = TB ? B[n*ldb + k] : B[k*ldb + n]
-// One warp per 16x8 output tile; M a multiple of 16, N a multiple of 8; K is
-// arbitrary (products past K, or past the split's end, read as zero).
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(128) k_gemm(const __nv_bfloat16* __restrict__ A, int lda,
-                                              const __nv_bfloat16* __restrict__ B, int ldb, float* __restrict__ C,
-                                              int M, int N, int K, int ksplit) {
-    const int lane = threadIdx.x & 31;
-    const int tile = blockIdx.x * 4 + (threadIdx.x >> 5);
-    const int tn = N / 8, tiles = (M / 16) * tn;
-    if (tile >= tiles) return;
-    const int m0 = (tile / tn) * 16, n0 = (tile % tn) * 8;
-    const int split = blockIdx.y;
-    const int kbeg = split * ksplit, kend = min(K, kbeg + ksplit);
-    const int g = lane >> 2, t = lane & 3;
-    const __nv_bfloat16 zero = __float2bfloat16_rn(0.f);
-    auto a_at = [&](int m, int k) -> __nv_bfloat16 {
-        if (k >= kend) return zero;
-        return TA ? A[(size_t)k * lda + m] : A[(size_t)m * lda + k];
-    };
-    auto b_at = [&](int k, int nn) -> __nv_bfloat16 {
-        if (k >= kend) return zero;
-        return TB ? B[(size_t)nn * ldb + k] : B[(size_t)k * ldb + nn];
-    };
-    auto pk = [](__nv_bfloat16 lo, __nv_bfloat16 hi) {
-        return (unsigned)__bfloat16_as_ushort(lo) | ((unsigned)__bfloat16_as_ushort(hi) << 16);
-    };
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int k0 = kbeg; k0 < kend; k0 += 16) {
-        unsigned a[4];
-        a[0] = pk(a_at(m0 + g, k0 + 2 * t), a_at(m0 + g, k0 + 2 * t + 1));
-        a[1] = pk(a_at(m0 + g + 8, k0 + 2 * t), a_at(m0 + g + 8, k0 + 2 * t + 1));
-        a[2] = pk(a_at(m0 + g, k0 + 2 * t + 8), a_at(m0 + g, k0 + 2 * t + 9));
-        a[3] = pk(a_at(m0 + g + 8, k0 + 2 * t + 8), a_at(m0 + g + 8, k0 + 2 * t + 9));
-        const unsigned b0 = pk(b_at(k0 + 2 * t, n0 + g), b_at(k0 + 2 * t + 1, n0 + g));
-        const unsigned b1 = pk(b_at(k0 + 2 * t + 8, n0 + g), b_at(k0 + 2 * t + 9, n0 + g));
-        mma16816(acc, a, b0, b1);
-    }
-    float* c = C + (size_t)split * M * N;
-    c[(size_t)(m0 + g) * N + n0 + 2 * t] = acc[0];
-    c[(size_t)(m0 + g) * N + n0 + 2 * t + 1] = acc[1];
-    c[(size_t)(m0 + g + 8) * N + n0 + 2 * t] = acc[2];
-    c[(size_t)(m0 + g + 8) * N + n0 + 2 * t + 1] = acc[3];
+// ---- training: one batch's loss and gradients ----------------------------------------
+// k_train_tile takes tiles of 128 rows, eight warps of 16 rows each. Forward, loss
+// and backward of a warp's rows chain through registers: the accumulators of one
+// m16n8k16 product, packed to BF16, are the A fragments of the next, so no
+// activation passes through shared memory on the way. What the weight gradients
+// contract over the rows (X, h1, h2, dz1, dz2, dy) is also left in shared memory as
+// BF16 rows, and after one barrier the warps split the output tiles of
+//   dW1 = X^T dz1 (32 x 64), dW2 = h1^T dz2 (64 x 64), dW3 = h2^T dy (64 x 8)
+// over the tile's 128 rows, reading both operands with transposing ldmatrix.
+// Accumulators live across the CTA's tiles; each CTA then writes one FP32 partial of
+// the whole gradient and k_train_reduce adds the partials in CTA order, so the
+// result does not depend on timing.
+//
+// A batch is a few megaflops: the time is the latency of one tile's chain plus the
+// launches. One launch per matrix product, bias, activation and column sum (23 a
+// batch, products reading 2-byte elements a whole row apart) took 289 us for a batch
+// of 16,384 rows with its Adam step; these two kernels and the step take 26 us.
+namespace tr {
+constexpr int kThreads = 256, kWarps = 8, kRows = 128;
+constexpr int kS = 72;   // BF16 elements of a 64-wide row: 144 bytes, so 8 rows of 16 bytes fall in 32 banks
+constexpr int kSX = 40;  // of a 32-wide row
+constexpr int kPart = kParams + 8;  // floats of one CTA's partial: the gradient and the squared error
+
+struct Smem {
+    __nv_bfloat16 w1[kIn][kS], w2[kH][kS], w3[kH][kOut];
+    __nv_bfloat16 x[kRows][kSX], h1[kRows][kS], h2[kRows][kS], dz1[kRows][kS], dz2[kRows][kS], dy[kRows][kOut];
+    float b[2 * kH + kOut];
+    float colsum[kWarps][2 * kH + kOut + 1];
+};
+
+__device__ __forceinline__ uint32_t addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void ldm4(unsigned (&r)[4], uint32_t a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(a));
+}
+__device__ __forceinline__ void ldm4t(unsigned (&r)[4], uint32_t a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(a));
 }
 
-// sum the split partials in fixed order: out[i] = sum_s part[s][i]
-__global__ void k_sum_splits(const float* __restrict__ part, int splits, size_t count, float* __restrict__ out) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    float s = 0.f;
-    for (int p = 0; p < splits; ++p) s += part[(size_t)p * count + i];
-    out[i] = s;
-}
-
-// Z = acc + bias (FP32, kept for the backward pass); H = bf16(SiLU(Z)).
-__global__ void k_bias_silu(const float* __restrict__ acc, const float* __restrict__ bias, int rows, int cols,
-                            float* __restrict__ z, __nv_bfloat16* __restrict__ h) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)rows * cols) return;
-    const float v = acc[i] + bias[i % cols];
-    z[i] = v;
-    h[i] = __float2bfloat16_rn(silu(v));
-}
-
-// Output layer: Y = acc + b3; dY = 2 (Y - T) / (3 rows) on the 3 real outputs
-// (bf16 for the products), squared error per row into err[row].
-__global__ void k_out_grad(const float* __restrict__ acc, const float* __restrict__ b3, const float* __restrict__ tgt,
-                           int rows, __nv_bfloat16* __restrict__ dy, float* __restrict__ err) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    float e = 0.f;
-    for (int c = 0; c < kOut; ++c) {
-        float d = 0.f;
-        if (c < 3) {
-            const float y = acc[(size_t)r * kOut + c] + b3[c];
-            const float diff = y - tgt[(size_t)r * 3 + c];
-            e += diff * diff;
-            d = 2.f * diff / (3.f * (float)rows);
+// acc (16 x 64) += A (16 x 16 KS, fragments) * W[k][n] (rows of kS elements)
+template <int KS>
+__device__ __forceinline__ void mul_w(float (&acc)[8][4], const unsigned (&a)[KS][4], const __nv_bfloat16* w,
+                                      int lane) {
+#pragma unroll
+    for (int s = 0; s < KS; ++s)
+#pragma unroll
+        for (int np = 0; np < 4; ++np) {
+            unsigned b[4];  // two n-tiles: {k 0..7, k 8..15} of each
+            ldm4t(b, addr(w + (16 * s + (lane & 15)) * kS + 16 * np + 8 * (lane >> 4)));
+            mma16816(acc[2 * np], a[s], b[0], b[1]);
+            mma16816(acc[2 * np + 1], a[s], b[2], b[3]);
         }
-        dy[(size_t)r * kOut + c] = __float2bfloat16_rn(d);
+}
+
+// z = acc + bias; h = bf16(SiLU(z)) as the next product's A fragments and as rows of `rows`
+__device__ __forceinline__ void activate(float (&z)[8][4], const float* bias, unsigned (&h)[4][4],
+                                         __nv_bfloat16 (*rows)[kS], int row, int t) {
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+        const float b0 = bias[8 * nt + 2 * t], b1 = bias[8 * nt + 2 * t + 1];
+        z[nt][0] += b0;
+        z[nt][1] += b1;
+        z[nt][2] += b0;
+        z[nt][3] += b1;
+        const unsigned lo = pack_bf16(silu(z[nt][0]), silu(z[nt][1]));
+        const unsigned hi = pack_bf16(silu(z[nt][2]), silu(z[nt][3]));
+        h[nt >> 1][(nt & 1) * 2] = lo;
+        h[nt >> 1][(nt & 1) * 2 + 1] = hi;
+        *reinterpret_cast<unsigned*>(&rows[row][8 * nt + 2 * t]) = lo;
+        *reinterpret_cast<unsigned*>(&rows[row + 8][8 * nt + 2 * t]) = hi;
     }
-    err[r] = e;
 }
 
-// dZ = bf16(dH * SiLU'(Z))
-__global__ void k_silu_back(const float* __restrict__ dh, const float* __restrict__ z, size_t count,
-                            __nv_bfloat16* __restrict__ dz) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    dz[i] = __float2bfloat16_rn(dh[i] * silu_grad(z[i]));
+// dz = bf16(dh * SiLU'(z)): A fragments, rows, and this thread's share of the column sums
+__device__ __forceinline__ void back_silu(const float (&dh)[8][4], const float (&z)[8][4], unsigned (&dz)[4][4],
+                                          __nv_bfloat16 (*rows)[kS], int row, int t, float (&sum)[8][2]) {
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+        const unsigned lo = pack_bf16(dh[nt][0] * silu_grad(z[nt][0]), dh[nt][1] * silu_grad(z[nt][1]));
+        const unsigned hi = pack_bf16(dh[nt][2] * silu_grad(z[nt][2]), dh[nt][3] * silu_grad(z[nt][3]));
+        dz[nt >> 1][(nt & 1) * 2] = lo;
+        dz[nt >> 1][(nt & 1) * 2 + 1] = hi;
+        *reinterpret_cast<unsigned*>(&rows[row][8 * nt + 2 * t]) = lo;
+        *reinterpret_cast<unsigned*>(&rows[row + 8][8 * nt + 2 * t]) = hi;
+        // a BF16 value is the high half of a float
+        sum[nt][0] += __uint_as_float(lo << 16) + __uint_as_float(hi << 16);
+        sum[nt][1] += __uint_as_float(lo & 0xffff0000u) + __uint_as_float(hi & 0xffff0000u);
+    }
 }
 
-// column sums of a bf16 [rows][cols] matrix, one block per column, fixed order
-__global__ void __launch_bounds__(256) k_colsum(const __nv_bfloat16* __restrict__ a, int rows, int cols,
-                                                float* __restrict__ out) {
-    __shared__ float red[256];
-    float s = 0.f;
-    for (int r = threadIdx.x; r < rows; r += 256) s += __bfloat162float(a[(size_t)r * cols + blockIdx.x]);
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+// A fragment of M^T for 16 rows: elements (m0.., r0..) of a row-major [row][m] matrix
+__device__ __forceinline__ uint32_t at_a(const __nv_bfloat16* m, int stride, int r0, int m0, int lane) {
+    return addr(m + (r0 + (lane & 7) + 8 * (lane >> 4)) * stride + m0 + 8 * ((lane >> 3) & 1));
+}
+// B fragments of two n-tiles for 16 rows of a row-major [row][n] matrix
+__device__ __forceinline__ uint32_t at_b(const __nv_bfloat16* m, int stride, int r0, int n0, int lane) {
+    return addr(m + (r0 + (lane & 15)) * stride + n0 + 8 * (lane >> 4));
+}
+
+// 16 x 8 accumulator tile to rows m0.. of a row-major float matrix
+__device__ __forceinline__ void put(float* c, int ld, int m0, int n0, const float (&a)[4], int lane) {
+    const int g = lane >> 2, t = lane & 3;
+    float* q = c + (m0 + g) * ld + n0 + 2 * t;
+    q[0] = a[0];
+    q[1] = a[1];
+    q[8 * ld] = a[2];
+    q[8 * ld + 1] = a[3];
+}
+}  // namespace tr
+
+__global__ void __launch_bounds__(tr::kThreads, 1) k_train_tile(const float* __restrict__ params,
+                                                                const __nv_bfloat16* __restrict__ X,
+                                                                const float* __restrict__ tgt, int rows,
+                                                                float* __restrict__ part) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    tr::Smem& s = *reinterpret_cast<tr::Smem*>(smem_raw);
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
+    for (int e = tid; e < kIn * kH; e += tr::kThreads) s.w1[e / kH][e % kH] = __float2bfloat16_rn(params[oW1 + e]);
+    for (int e = tid; e < kH * kH; e += tr::kThreads) s.w2[e / kH][e % kH] = __float2bfloat16_rn(params[oW2 + e]);
+    for (int e = tid; e < kH * kOut; e += tr::kThreads) s.w3[e / kOut][e % kOut] = __float2bfloat16_rn(params[oW3 + e]);
+    if (tid < kH) {
+        s.b[tid] = params[oB1 + tid];
+        s.b[kH + tid] = params[oB2 + tid];
+    }
+    if (tid < kOut) s.b[2 * kH + tid] = params[oB3 + tid];
+
+    const bool aligned = (reinterpret_cast<uintptr_t>(X) & 15u) == 0;
+    float dw1[2][4] = {}, dw2[4][4] = {}, dw3[4] = {};  // this warp's tiles of the weight gradients
+    float sum1[8][2] = {}, sum2[8][2] = {}, sum3[2] = {0.f, 0.f}, err = 0.f;
+    const int tiles = (rows - 1) / tr::kRows + 1;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int r0 = tile * tr::kRows;
+        __syncthreads();  // the last tile's rows are used up (first pass: orders the weights with the next barrier)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int e = tid + q * tr::kThreads, r = e >> 2, c = e & 3;
+            uint4 v = make_uint4(0u, 0u, 0u, 0u);
+            if (r0 + r < rows) {
+                const __nv_bfloat16* src = X + (size_t)(r0 + r) * kIn + 8 * c;
+                if (aligned) {
+                    v = *reinterpret_cast<const uint4*>(src);
+                } else {  // features at any 2-byte address
+                    const unsigned short* h = reinterpret_cast<const unsigned short*>(src);
+                    v = make_uint4(h[0] | (unsigned)h[1] << 16, h[2] | (unsigned)h[3] << 16,
+                                   h[4] | (unsigned)h[5] << 16, h[6] | (unsigned)h[7] << 16);
+                }
+            }
+            *reinterpret_cast<uint4*>(&s.x[r][8 * c]) = v;
+        }
         __syncthreads();
-    }
-    if (threadIdx.x == 0) out[blockIdx.x] = red[0];
-}
-
-__global__ void k_sum_f32(const float* __restrict__ a, int n, float* __restrict__ out) {
-    __shared__ float red[256];
-    float s = 0.f;
-    for (int i = threadIdx.x; i < n; i += 256) s += a[i];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+        const int row = 16 * w + g;  // this thread's rows of the tile: row, row + 8
+        if (r0 + 16 * w < rows) {    // rows come in multiples of 16: a warp has all of its 16 or none
+            float z1[8][4] = {}, z2[8][4] = {};
+            unsigned h[4][4];
+            {
+                unsigned a[2][4];
+                const uint32_t xa = tr::addr(&s.x[16 * w + (lane & 15)][8 * (lane >> 4)]);
+                tr::ldm4(a[0], xa);
+                tr::ldm4(a[1], xa + 32);
+                tr::mul_w<2>(z1, a, &s.w1[0][0], lane);
+            }
+            tr::activate(z1, s.b, h, s.h1, row, t);
+            tr::mul_w<4>(z2, h, &s.w2[0][0], lane);
+            tr::activate(z2, s.b + kH, h, s.h2, row, t);
+            float y[4] = {};
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                unsigned b[4];  // k-steps 2q and 2q + 1
+                tr::ldm4t(b, tr::addr(&s.w3[32 * q + lane][0]));
+                mma16816(y, h[2 * q], b[0], b[1]);
+                mma16816(y, h[2 * q + 1], b[2], b[3]);
+            }
+            // dY = 2 (Y - T) / (3 rows) on the 3 real outputs
+            float d[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int c = 2 * t + (q & 1), r = row + 8 * (q >> 1);
+                d[q] = 0.f;
+                if (c < 3) {
+                    const float diff = y[q] + s.b[2 * kH + c] - tgt[(size_t)(r0 + r) * 3 + c];
+                    err += diff * diff;
+                    d[q] = 2.f * diff / (3.f * (float)rows);
+                }
+            }
+            const unsigned lo = pack_bf16(d[0], d[1]), hi = pack_bf16(d[2], d[3]);
+            *reinterpret_cast<unsigned*>(&s.dy[row][2 * t]) = lo;
+            *reinterpret_cast<unsigned*>(&s.dy[row + 8][2 * t]) = hi;
+            sum3[0] += __uint_as_float(lo << 16) + __uint_as_float(hi << 16);
+            sum3[1] += __uint_as_float(lo & 0xffff0000u) + __uint_as_float(hi & 0xffff0000u);
+            // dh2 = dY W3^T: k = the 8 outputs, the upper half of the k-step zero
+            float dh[8][4] = {};
+            const unsigned ay[4] = {lo, hi, 0u, 0u};
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                unsigned b[4];  // units 32 q + 8 j: row n, 8 outputs along k
+                tr::ldm4(b, tr::addr(&s.w3[32 * q + lane][0]));
+#pragma unroll
+                for (int j = 0; j < 4; ++j) mma16816(dh[4 * q + j], ay, b[j], 0u);
+            }
+            unsigned dz[4][4];
+            tr::back_silu(dh, z2, dz, s.dz2, row, t, sum2);
+            // dh1 = dz2 W2^T: B[k = unit of layer 2][n = unit of layer 1] = W2[n][k]
+            float dg[8][4] = {};
+#pragma unroll
+            for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    unsigned b[4];  // k-steps 2q, 2q + 1
+                    tr::ldm4(b, tr::addr(&s.w2[8 * nt + (lane & 7)][32 * q + 8 * (lane >> 3)]));
+                    mma16816(dg[nt], dz[2 * q], b[0], b[1]);
+                    mma16816(dg[nt], dz[2 * q + 1], b[2], b[3]);
+                }
+            tr::back_silu(dg, z1, dz, s.dz1, row, t, sum1);
+        } else {  // rows past the batch add nothing: their gradients' factors are zero
+            for (int e = lane; e < 16 * kH / 2; e += 32) {
+                const int r = 16 * w + e / (kH / 2), c = 2 * (e % (kH / 2));
+                *reinterpret_cast<unsigned*>(&s.h1[r][c]) = 0u;
+                *reinterpret_cast<unsigned*>(&s.h2[r][c]) = 0u;
+                *reinterpret_cast<unsigned*>(&s.dz1[r][c]) = 0u;
+                *reinterpret_cast<unsigned*>(&s.dz2[r][c]) = 0u;
+            }
+            for (int e = lane; e < 16 * kOut / 2; e += 32)
+                *reinterpret_cast<unsigned*>(&s.dy[16 * w + e / (kOut / 2)][2 * (e % (kOut / 2))]) = 0u;
+        }
         __syncthreads();
+        const int m2 = 16 * (w >> 1), n2 = 32 * (w & 1);  // dW2: 16 x 32 per warp
+        const int m1 = 16 * (w >> 2), n1 = 16 * (w & 3);  // dW1: 16 x 16 per warp
+        const int m3 = 16 * (w & 3);                      // dW3: 16 x 8 per warp, 64 rows each
+#pragma unroll 2
+        for (int k = 0; k < tr::kRows / 16; ++k) {
+            unsigned a[4], b[4];
+            tr::ldm4t(a, tr::at_a(&s.h1[0][0], tr::kS, 16 * k, m2, lane));
+            tr::ldm4t(b, tr::at_b(&s.dz2[0][0], tr::kS, 16 * k, n2, lane));
+            mma16816(dw2[0], a, b[0], b[1]);
+            mma16816(dw2[1], a, b[2], b[3]);
+            tr::ldm4t(b, tr::at_b(&s.dz2[0][0], tr::kS, 16 * k, n2 + 16, lane));
+            mma16816(dw2[2], a, b[0], b[1]);
+            mma16816(dw2[3], a, b[2], b[3]);
+            tr::ldm4t(a, tr::at_a(&s.x[0][0], tr::kSX, 16 * k, m1, lane));
+            tr::ldm4t(b, tr::at_b(&s.dz1[0][0], tr::kS, 16 * k, n1, lane));
+            mma16816(dw1[0], a, b[0], b[1]);
+            mma16816(dw1[1], a, b[2], b[3]);
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {  // warps 0..3: the tile's first 64 rows, 4..7: the rest
+            const int k = 64 * (w >> 2) + 32 * q;
+            unsigned a[4], b[4];
+            tr::ldm4t(b, tr::addr(&s.dy[k + lane][0]));
+            tr::ldm4t(a, tr::at_a(&s.h2[0][0], tr::kS, k, m3, lane));
+            mma16816(dw3, a, b[0], b[1]);
+            tr::ldm4t(a, tr::at_a(&s.h2[0][0], tr::kS, k + 16, m3, lane));
+            mma16816(dw3, a, b[2], b[3]);
+        }
     }
-    if (threadIdx.x == 0) *out = red[0];
+
+    // the CTA's partial: weight tiles straight from the accumulators; column sums and the
+    // squared error over the lanes of a warp, then over the warps
+    float* p = part + (size_t)blockIdx.x * tr::kPart;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) tr::put(p + oW2, kH, 16 * (w >> 1), 32 * (w & 1) + 8 * j, dw2[j], lane);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) tr::put(p + oW1, kH, 16 * (w >> 2), 16 * (w & 3) + 8 * j, dw1[j], lane);
+    auto over_rows = [](float v) {  // lanes that share t hold the same columns
+        v += __shfl_xor_sync(0xffffffffu, v, 4);
+        v += __shfl_xor_sync(0xffffffffu, v, 8);
+        return v + __shfl_xor_sync(0xffffffffu, v, 16);
+    };
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const float a = over_rows(sum1[nt][c]), b = over_rows(sum2[nt][c]);
+            if (g == 0) {
+                s.colsum[w][8 * nt + 2 * t + c] = a;
+                s.colsum[w][kH + 8 * nt + 2 * t + c] = b;
+            }
+        }
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        const float a = over_rows(sum3[c]);
+        if (g == 0) s.colsum[w][2 * kH + 2 * t + c] = a;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) err += __shfl_xor_sync(0xffffffffu, err, o);
+    if (lane == 0) s.colsum[w][2 * kH + kOut] = err;
+    __syncthreads();  // the last tile's rows are used up: h1's storage takes the upper half of dW3
+    float* d3 = reinterpret_cast<float*>(&s.h1[0][0]);
+    if (w >= 4) tr::put(d3, kOut, 16 * (w & 3), 0, dw3, lane);
+    if (tid <= 2 * kH + kOut) {
+        float v = 0.f;
+#pragma unroll
+        for (int q = 0; q < tr::kWarps; ++q) v += s.colsum[q][tid];
+        const int o = tid < kH ? oB1 + tid : (tid < 2 * kH ? oB2 + tid - kH : oB3 + tid - 2 * kH);
+        p[o] = v;  // the squared error lands after b3, at kParams
+    }
+    __syncthreads();
+    if (w < 4) {
+        float lo[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) lo[q] = dw3[q] + d3[(16 * w + g + 8 * (q >> 1)) * kOut + 2 * t + (q & 1)];
+        tr::put(p + oW3, kOut, 16 * w, 0, lo, lane);
+    }
 }
 
-__global__ void k_to_bf16(const float* __restrict__ a, int n, __nv_bfloat16* __restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = __float2bfloat16_rn(a[i]);
+// grad[i] = sum over the CTAs' partials, in a fixed order: 4 threads take a quarter of
+// them each; *sse from the entry after the gradient.
+__global__ void __launch_bounds__(256) k_train_reduce(const float* __restrict__ part, int parts,
+                                                      float* __restrict__ grad, float* __restrict__ sse) {
+    __shared__ float red[4][64];
+    const int c = threadIdx.x & 63, q = threadIdx.x >> 6, i = blockIdx.x * 64 + c;
+    const int per = (parts + 3) / 4, p0 = q * per, p1 = min(parts, p0 + per);
+    float v = 0.f;
+    if (i <= kParams) {
+#pragma unroll 8
+        for (int p = p0; p < p1; ++p) v += part[(size_t)p * tr::kPart + i];
+    }
+    red[q][c] = v;
+    __syncthreads();
+    if (q == 0 && i <= kParams) {
+        v = (red[0][c] + red[1][c]) + (red[2][c] + red[3][c]);
+        if (i < kParams) grad[i] = v;
+        else *sse = v;
+    }
 }
 
-__global__ void k_adam(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
+__global__ void k_adam(
+float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
                        const float* __restrict__ grad, int n, float lr, float b1, float b2, float eps, float c1,
                        float c2) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -541,19 +743,11 @@ int launch_mlp_infer(const float* params, const float4* pos, const int* perm, in
     return SD_OK;
 }
 
-// Workspace of one training batch of `rows` samples (rows a multiple of 16).
-static size_t mlp_train_ws(int rows, int splits) {
-    const size_t r = (size_t)rows;
-    size_t b = 0;
-    b += align_up(r * kH * 4, 256) * 4;         // z1, z2, dh (fp32) + acc scratch
-    b += align_up(r * kH * 2, 256) * 4;         // h1, h2, dz2, dz1 (bf16)
-    b += align_up(r * kOut * 4, 256);           // y acc
-    b += align_up(r * kOut * 2, 256);           // dy (bf16)
-    b += align_up(r * 4, 256);                  // per-row error
-    b += align_up((size_t)kParams * 2, 256);    // bf16 weights
-    b += align_up((size_t)splits * kH * kH * 4, 256);  // split partials of weight grads
-    b += 256;
-    return b;
+// CTAs of a training batch: one per tile of 128 rows, at most one per SM (a CTA's
+// partial gradient is 27 KB that the reduction reads again).
+static int train_ctas(int rows) {
+    const int tiles = rows > 0 ? (rows - 1) / tr::kRows + 1 : 1;
+    return tiles < 148 ? tiles : 148;
 }
 
 }  // namespace sd
@@ -590,12 +784,8 @@ int sd_mlp_infer(const float* params, const float* pos, const int32_t* perm, int
                             reinterpret_cast<float4*>(out), (cudaStream_t)stream);
 }
 
-// split-K slices of the weight-gradient products (K = rows): one per 1024 rows
-static int mlp_splits(int rows) { return (rows + 1023) / 1024; }
-
 size_t sd_mlp_train_workspace_bytes(int rows) {
-    const int splits = mlp_splits(rows);
-    return mlp_train_ws(rows, splits);
+    return align_up(sizeof(float) * tr::kPart * (size_t)train_ctas(rows), 256);
 }
 
 // Loss and gradients of one batch: features X (bf16 [rows][32]), targets T
@@ -606,84 +796,17 @@ int sd_mlp_loss_grad(const float* params, const void* features_bf16, const float
                      float* sse, void* ws, size_t ws_bytes, void* stream) {
     if (!params || !features_bf16 || !targets || !grad || !sse || !ws || rows <= 0 || rows % 16)
         return fail(SD_E_ARG, "mlp_loss_grad: bad arguments (rows must be a positive multiple of 16)");
-    const int splits = mlp_splits(rows);
-    if (ws_bytes < mlp_train_ws(rows, splits)) return fail(SD_E_ARG, "mlp_loss_grad: workspace too small");
+    if (ws_bytes < sd_mlp_train_workspace_bytes(rows)) return fail(SD_E_ARG, "mlp_loss_grad: workspace too small");
     cudaStream_t st = (cudaStream_t)stream;
-    const size_t r = (size_t)rows;
-    char* p = (char*)ws;
-    auto take = [&](size_t bytes) {
-        char* q = p;
-        p += align_up(bytes, 256);
-        return q;
-    };
-    float* z1 = (float*)take(r * kH * 4);
-    float* z2 = (float*)take(r * kH * 4);
-    float* dh = (float*)take(r * kH * 4);
-    float* accb = (float*)take(r * kH * 4);
-    __nv_bfloat16* h1 = (__nv_bfloat16*)take(r * kH * 2);
-    __nv_bfloat16* h2 = (__nv_bfloat16*)take(r * kH * 2);
-    __nv_bfloat16* dz2 = (__nv_bfloat16*)take(r * kH * 2);
-    __nv_bfloat16* dz1 = (__nv_bfloat16*)take(r * kH * 2);
-    float* yacc = (float*)take(r * kOut * 4);
-    __nv_bfloat16* dy = (__nv_bfloat16*)take(r * kOut * 2);
-    float* err = (float*)take(r * 4);
-    __nv_bfloat16* wb = (__nv_bfloat16*)take((size_t)kParams * 2);
-    float* part = (float*)take((size_t)splits * kH * kH * 4);
-    const __nv_bfloat16* X = (const __nv_bfloat16*)features_bf16;
-
-    auto blocks = [](size_t count) { return (unsigned)((count + 255) / 256); };
-    k_to_bf16<<<blocks(kParams), 256, 0, st>>>(params, kParams, wb);
+    const int ctas = train_ctas(rows);
+    float* part = reinterpret_cast<float*>(ws);
+    // the shared-memory limit is per device, so it is set on each call (a host-side look-up)
+    if (SD_CUDA(cudaFuncSetAttribute(k_train_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(tr::Smem))))
+        return SD_E_CUDA;
+    k_train_tile<<<ctas, tr::kThreads, sizeof(tr::Smem), st>>>(
+        params, reinterpret_cast<const __nv_bfloat16*>(features_bf16), targets, rows, part);
     SD_LAUNCHED(st);
-    const __nv_bfloat16 *W1 = wb + oW1, *W2 = wb + oW2, *W3 = wb + oW3;
-    // gemm helper: C[M][N] = opA * opB over K (split-K into `sp` slices, summed in fixed order)
-    auto gemm = [&](bool ta, bool tb, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, float* C,
-                    int M, int N, int K) -> int {
-        const int tiles = (M / 16) * (N / 8);
-        const int sp = (K >= 2048) ? splits : 1;
-        const int ks = ((K / sp + 15) / 16) * 16;
-        dim3 grid((tiles + 3) / 4, sp);
-        float* dst = (sp == 1) ? C : part;
-        if (ta && tb) k_gemm<true, true><<<grid, 128, 0, st>>>(A, lda, B, ldb, dst, M, N, K, ks);
-        else if (ta) k_gemm<true, false><<<grid, 128, 0, st>>>(A, lda, B, ldb, dst, M, N, K, ks);
-        else if (tb) k_gemm<false, true><<<grid, 128, 0, st>>>(A, lda, B, ldb, dst, M, N, K, ks);
-        else k_gemm<false, false><<<grid, 128, 0, st>>>(A, lda, B, ldb, dst, M, N, K, ks);
-        SD_LAUNCHED(st);
-        if (sp > 1) {
-            k_sum_splits<<<blocks((size_t)M * N), 256, 0, st>>>(part, sp, (size_t)M * N, C);
-            SD_LAUNCHED(st);
-        }
-        return SD_OK;
-    };
-    int rc;
-    // forward
-    if ((rc = gemm(false, false, X, kIn, W1, kH, accb, rows, kH, kIn))) return rc;
-    k_bias_silu<<<blocks(r * kH), 256, 0, st>>>(accb, params + oB1, rows, kH, z1, h1);
-    SD_LAUNCHED(st);
-    if ((rc = gemm(false, false, h1, kH, W2, kH, accb, rows, kH, kH))) return rc;
-    k_bias_silu<<<blocks(r * kH), 256, 0, st>>>(accb, params + oB2, rows, kH, z2, h2);
-    SD_LAUNCHED(st);
-    if ((rc = gemm(false, false, h2, kH, W3, kOut, yacc, rows, kOut, kH))) return rc;
-    k_out_grad<<<blocks(r), 256, 0, st>>>(yacc, params + oB3, targets, rows, dy, err);
-    SD_LAUNCHED(st);
-    k_sum_f32<<<1, 256, 0, st>>>(err, rows, sse);
-    SD_LAUNCHED(st);
-    // backward: layer 3
-    if ((rc = gemm(true, false, h2, kH, dy, kOut, grad + oW3, kH, kOut, rows))) return rc;
-    k_colsum<<<kOut, 256, 0, st>>>(dy, rows, kOut, grad + oB3);
-    SD_LAUNCHED(st);
-    if ((rc = gemm(false, true, dy, kOut, W3, kOut, dh, rows, kH, kOut))) return rc;
-    k_silu_back<<<blocks(r * kH), 256, 0, st>>>(dh, z2, r * kH, dz2);
-    SD_LAUNCHED(st);
-    // layer 2
-    if ((rc = gemm(true, false, h1, kH, dz2, kH, grad + oW2, kH, kH, rows))) return rc;
-    k_colsum<<<kH, 256, 0, st>>>(dz2, rows, kH, grad + oB2);
-    SD_LAUNCHED(st);
-    if ((rc = gemm(false, true, dz2, kH, W2, kH, dh, rows, kH, kH))) return rc;
-    k_silu_back<<<blocks(r * kH), 256, 0, st>>>(dh, z1, r * kH, dz1);
-    SD_LAUNCHED(st);
-    // layer 1
-    if ((rc = gemm(true, false, X, kIn, dz1, kH, grad + oW1, kIn, kH, rows))) return rc;
-    k_colsum<<<kH, 256, 0, st>>>(dz1, rows, kH, grad + oB1);
+    k_train_reduce<<<(kParams + 1 + 63) / 64, 256, 0, st>>>(part, ctas, grad, sse);
     SD_LAUNCHED(st);
     return SD_OK;
 }

@@ -102,6 +102,33 @@ def test_gpu_loss_grad_matches_oracle(cuda, lib, oracle, rows):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("rows,shift", [(16, 0), (112, 1), (128, 0), (144, 3), (148 * 128, 0), (148 * 128 + 16, 1)])
+def test_gpu_loss_grad_tiles(cuda, lib, oracle, rows, shift):
+    # one warp, a part tile, a whole one, one row group past it, one tile per CTA, and a
+    # CTA's second tile; features at addresses that are not a multiple of 16 bytes.
+    # BF16 roundings that fall the other way (2^-9 each) bound the difference, as above.
+    params = _params(12, 0.2)
+    X, T = _batch(rows, 5)
+    buf = cuda.zeros(rows * 32 + 8, dtype=cuda.bfloat16, device="cuda")
+    Xb = buf[shift:shift + rows * 32]
+    Xb.copy_(cuda.from_numpy(X).reshape(-1))
+    Td, prm = cuda.from_numpy(T).cuda(), cuda.from_numpy(params).cuda()
+    grad = cuda.full((6792,), float("nan"), dtype=cuda.float32, device="cuda")
+    sse = cuda.empty(1, dtype=cuda.float32, device="cuda")
+    ws = cuda.full((int(lib.sd_mlp_train_workspace_bytes(rows)),), 255, dtype=cuda.uint8, device="cuda")
+    L.check(lib.sd_mlp_loss_grad(prm.data_ptr(), Xb.data_ptr(), Td.data_ptr(), rows, grad.data_ptr(), sse.data_ptr(),
+                                 ws.data_ptr(), ws.numel(), None), "loss_grad")
+    g = grad.cpu().numpy()
+    assert np.isfinite(g).all()
+    sse_ref, g_ref = oracle.mlp_loss_grad(params, X, T)
+    assert float(sse.cpu()) == pytest.approx(sse_ref, rel=1e-3)
+    for name, (o, sh) in oracle.MLP_OFF.items():
+        a, b = g[o:o + int(np.prod(sh))], g_ref[o:o + int(np.prod(sh))]
+        rel = np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-12)
+        assert rel < 3e-2, (name, rel)
+
+
+@pytest.mark.gpu
 def test_gpu_adam_step(cuda, lib):
     n = 6792
     rng = np.random.default_rng(0)
