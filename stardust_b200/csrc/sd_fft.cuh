@@ -157,8 +157,9 @@ struct PlainLoad {
 };
 
 // Stages from sub-transform length Ns on, stopping before the stage at STOP; the
-// stage at Ns = 1 reads through `load`.
-template <int N, int Ns, int NT, int TWS, bool INV, int STOP = N, class Load = PlainLoad>
+// stage at Ns = 1 reads through `load`. HALF: positions N/2 and up of the input are
+// zero and are not read (they are the upper half of the first stage's radix).
+template <int N, int Ns, int NT, int TWS, bool INV, int STOP = N, class Load = PlainLoad, bool HALF = false>
 __device__ __forceinline__ void stages16(float2* s, const float2* tw, Load load = Load()) {
     if constexpr (Ns < N && Ns < STOP) {
         constexpr int R = radix_of<N / Ns, N, NT>::value;
@@ -173,6 +174,10 @@ __device__ __forceinline__ void stages16(float2* s, const float2* tw, Load load 
                 const int l = u & 15, j = u >> 4, k = j % Ns;
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
+                    if (HALF && Ns == 1 && r >= R / 2) {
+                        v[p][r] = make_float2(0.f, 0.f);
+                        continue;
+                    }
                     float2 x = (Ns == 1) ? load(s, l, j + r * NB) : s[(j + r * NB) * 16 + l];
                     if (Ns > 1 && r > 0) {
                         float2 w = tw[(k * r * (N / (Ns * R))) * TWS];
@@ -201,10 +206,10 @@ __device__ __forceinline__ void stages16(float2* s, const float2* tw, Load load 
 }
 
 // Transform the 16 interleaved lines of length N in s. The caller synchronises
-// before the call; the routine ends with a barrier.
-template <int N, int NT, int TWS, bool INV>
+// before the call; the routine ends with a barrier. HALF: the input's upper half is zero.
+template <int N, int NT, int TWS, bool INV, bool HALF = false>
 __device__ __forceinline__ void lines16(float2* s, const float2* tw) {
-    stages16<N, 1, NT, TWS, INV>(s, tw);
+    stages16<N, 1, NT, TWS, INV, N, PlainLoad, HALF>(s, tw);
 }
 
 // Forward transform, a pointwise multiply, inverse transform of the 16 lines.
@@ -214,15 +219,16 @@ __device__ __forceinline__ void lines16(float2* s, const float2* tw) {
 // mul(line, position, value) and the inverse's first stage run in registers with
 // no shared-memory round trip or barrier between them; the inverse then goes on
 // from sub-length R. The caller synchronises before the call; it ends with a
-// barrier.
-template <int N, int NT, int TWS, class Mul>
+// barrier. HALF: the input's upper half is zero (N takes at least two stages).
+template <int N, int NT, int TWS, bool HALF = false, class Mul>
 __device__ __forceinline__ void convolve16(float2* s, const float2* tw, Mul mul) {
     constexpr int NsL = last_stage_ns(N, NT);
     constexpr int R = N / NsL;
     constexpr int NB = N / R;  // == NsL
     constexpr int TOT = 16 * NB;
     constexpr int PER = (TOT + NT - 1) / NT;
-    stages16<N, 1, NT, TWS, false, NsL>(s, tw);
+    static_assert(!HALF || NsL > 1, "a half-zero input is pruned in a first stage of its own");
+    stages16<N, 1, NT, TWS, false, NsL, PlainLoad, HALF>(s, tw);
     float2 v[PER][R];
 #pragma unroll
     for (int p = 0; p < PER; ++p) {

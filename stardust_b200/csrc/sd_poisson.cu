@@ -736,10 +736,11 @@ __global__ void __launch_bounds__(kDepositThreads, G >= 128 ? 3 : 2)
 
 // Stage bricks into shared memory with cp.async. DIR 1: y-lines of CTA (bx,bz);
 // DIR 2: z-lines of CTA (bx,by). Lines: DIR 1 -> z_l*4 + kx_l, DIR 2 -> y_l*4 + kx_l.
-template <int G, int DIR>
+// HALF: only the lower half of each line (load_lines, store_lines).
+template <int G, int DIR, bool HALF = false>
 __device__ __forceinline__ void load_lines(float2* s, const float2* __restrict__ spec, int b0, int b1) {
     using T = Geo<G>;
-    constexpr int NB = (DIR == 1) ? T::NBY : T::NBZ;
+    constexpr int NB = ((DIR == 1) ? T::NBY : T::NBZ) / (HALF ? 2 : 1);
     for (int u = threadIdx.x; u < NB * 32; u += kFftThreads) {
         const int b = u >> 5, c = u & 31;
         const int e = 2 * c;
@@ -758,10 +759,10 @@ __device__ __forceinline__ void load_lines(float2* s, const float2* __restrict__
     __syncthreads();
 }
 
-template <int G, int DIR>
+template <int G, int DIR, bool HALF = false>
 __device__ __forceinline__ void store_lines(const float2* s, float2* __restrict__ spec, int bx, int b1) {
     using T = Geo<G>;
-    constexpr int NB = (DIR == 1) ? T::NBY : T::NBZ;
+    constexpr int NB = ((DIR == 1) ? T::NBY : T::NBZ) / (HALF ? 2 : 1);
     for (int u = threadIdx.x; u < NB * 32; u += kFftThreads) {
         const int b = u >> 5, c = u & 31;
         const int e = 2 * c;
@@ -779,25 +780,33 @@ __device__ __forceinline__ void store_lines(const float2* s, float2* __restrict_
 }
 
 // ---- passes B and D: y-lines of CTA (bx, bz), in place -------------------------
-template <int G, bool INV>
-__global__ void __launch_bounds__(kFftThreads) k_pass_y(float2* __restrict__ spec, const float2* __restrict__ tw_g) {
+// HALF (isolated boundary): the density fills the low corner of the box and the
+// potential is read only there, so the forward transform's inputs past half the box
+// are zero (never written, not read) and the inverse's outputs past it are not
+// stored; the grid covers the lower half of the z slabs. At 512 the pruned forward
+// transform takes 85 registers left alone, two CTAs an SM; bounded to three 112 -> 102 us
+// (the other instances have three by themselves).
+template <int G, bool INV, bool HALF>
+__global__ void __launch_bounds__(kFftThreads, G == 512 && HALF && !INV ? 3 : 0)
+    k_pass_y(float2* __restrict__ spec, const float2* __restrict__ tw_g) {
     extern __shared__ float2 sm[];
     float2* tw = sm;
     float2* s = sm + G;
     const int bx = blockIdx.x, bz = blockIdx.y;
     for (int i = threadIdx.x; i < G; i += kFftThreads) tw[i] = tw_g[i];
-    load_lines<G, 1>(s, spec, bx, bz);
-    fft::lines16<G, kFftThreads, 1, INV>(s, tw);
-    store_lines<G, 1>(s, spec, bx, bz);
+    load_lines<G, 1, HALF && !INV>(s, spec, bx, bz);
+    fft::lines16<G, kFftThreads, 1, INV, HALF && !INV>(s, tw);
+    store_lines<G, 1, HALF && INV>(s, spec, bx, bz);
 }
 
 // ---- pass C: z-lines of CTA (bx, by): forward, Green's function, inverse ---------
 // MODE 0: the periodic Green's function (analytic, Sim.cu:528-557).
 // MODE 1: forward transform only (builds the isolated boundary's Green spectrum).
-// MODE 2: multiply by a tabulated real Green spectrum table[|ky|][kx][|kz|]
-//         ((H+1)^3 floats) times table_scale, then inverse (isolated boundary,
-//         kMulSpec, Sim.cu:578-584).
-template <int G, int MODE>
+// MODE 2: multiply by a tabulated real Green spectrum table[|ky|][kx / 4][|kz|][kx % 4]
+//         (columns past kx = H hold zeros) times table_scale, then inverse (isolated
+//         boundary, kMulSpec, Sim.cu:578-584). A CTA's values are 4 contiguous runs.
+// HALF: the lines' upper half is zero on input and not needed on output (see k_pass_y).
+template <int G, int MODE, bool HALF>
 __global__ void __launch_bounds__(kFftThreads) k_pass_c(float2* __restrict__ spec, const float2* __restrict__ tw_g,
                                                         const float* __restrict__ gexp_g, float scale,
                                                         const float* __restrict__ table, float table_scale) {
@@ -820,7 +829,22 @@ __global__ void __launch_bounds__(kFftThreads) k_pass_c(float2* __restrict__ spe
         line_g[l] = (kx <= H) ? -scale * (gexp_g[kx] * gexp_g[abs(kyf)]) : 0.f;  // the global table: no barrier yet
         line_k2[l] = kx * kx + kyf * kyf;
     }
-    load_lines<G, 2>(s, spec, bx, by);  // ends with a barrier
+    // MODE 2: the table's values of these 16 lines, 4 runs of H + 1 groups of 4 bins, come
+    // into shared memory with the lines. Fetched at the multiply, each thread's 16 or 32
+    // values came one L2 access after another, a sector for each 16 bytes. The runs are
+    // 8 banks apart, so the two kz a warp multiplies by do not conflict.
+    constexpr int kRun = 4 * (H + 1) + 4;
+    float* line_t = reinterpret_cast<float*>(s + 16 * G);
+    if (MODE == 2) {
+        const float4* t4 = reinterpret_cast<const float4*>(table);
+#pragma unroll
+        for (int yl = 0; yl < 4; ++yl) {
+            const int ky = by * 4 + yl, kyf = (ky <= G / 2) ? ky : G - ky;
+            for (int kz = threadIdx.x; kz <= H; kz += kFftThreads)
+                fft::cp_async16(line_t + yl * kRun + 4 * kz, t4 + ((size_t)kyf * T::NBX + bx) * (H + 1) + kz);
+        }
+    }
+    load_lines<G, 2, HALF>(s, spec, bx, by);  // ends with a barrier
     if (MODE == 1) {
         fft::lines16<G, kFftThreads, 1, false>(s, tw);
         store_lines<G, 2>(s, spec, bx, by);
@@ -837,27 +861,27 @@ __global__ void __launch_bounds__(kFftThreads) k_pass_c(float2* __restrict__ spe
             const int k2 = line_k2[l] + kzf * kzf;
             m = (k2 != 0) ? __fdividef(line_g[l] * gexp[abs(kzf)], (float)k2) : 0.f;
         } else {
-            const int kx = bx * 4 + (l & 3), ky = by * 4 + (l >> 2);
-            const int kyf = (ky <= G / 2) ? ky : G - ky;
-            m = (kx <= H) ? table[((size_t)kyf * (H + 1) + kx) * (H + 1) + abs(kzf)] * table_scale : 0.f;
+            m = line_t[(l >> 2) * kRun + 4 * abs(kzf) + (l & 3)] * table_scale;
         }
         return make_float2(x.x * m, x.y * m);
     };
-    fft::convolve16<G, kFftThreads, 1>(s, tw, green);
-    store_lines<G, 2>(s, spec, bx, by);
+    fft::convolve16<G, kFftThreads, 1, HALF>(s, tw, green);
+    store_lines<G, 2, HALF>(s, spec, bx, by);
 }
 
-// Real part of a forward spectrum (bricked) into table[|ky|][kx][|kz|], ky, kz, kx <= H.
+// Real part of a forward spectrum (bricked) into table[|ky|][kx / 4][|kz|][kx % 4].
 template <int G>
 __global__ void k_green_table(const float2* __restrict__ spec, float* __restrict__ table) {
     using T = Geo<G>;
     constexpr int H = T::H;
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t n = (size_t)(H + 1) * (H + 1) * (H + 1);
+    const size_t n = (size_t)(H + 1) * T::PX * (H + 1);
     if (i >= n) return;
-    const int kz = (int)(i % (H + 1)), kx = (int)((i / (H + 1)) % (H + 1)), ky = (int)(i / ((size_t)(H + 1) * (H + 1)));
-    const size_t e = T::brick(kx >> 2, ky >> 2, kz >> 2) + (size_t)((kz & 3) * 16 + (ky & 3) * 4 + (kx & 3));
-    table[i] = spec[e].x;
+    const size_t g = i >> 2;
+    const int kz = (int)(g % (H + 1)), bx = (int)(g / (H + 1) % T::NBX), ky = (int)(g / ((size_t)(H + 1) * T::NBX));
+    const int kx = 4 * bx + (int)(i & 3);
+    const size_t e = T::brick(bx, ky >> 2, kz >> 2) + (size_t)((kz & 3) * 16 + (ky & 3) * 4 + (kx & 3));
+    table[i] = kx <= H ? spec[e].x : 0.f;
 }
 
 // Real-space isolated kernel on the transform box (kGreen, Sim.cu:563-576):
@@ -874,7 +898,9 @@ __global__ void k_green_kernel(float* __restrict__ g, int S, float soft) {
 }
 
 // ---- pass E: kx bins -> real rows (y = 4by + y_l, z = 4bz + z_l) ----------------
-template <int G>
+// HALF (isolated boundary): only the lower half of each row is needed and stored;
+// the grid covers the rows of the low corner.
+template <int G, bool HALF>
 __global__ void __launch_bounds__(kFftThreads, 5) k_pass_e(const float2* __restrict__ spec, float* __restrict__ phi,
                                                         const float2* __restrict__ tw_g) {
     using T = Geo<G>;
@@ -925,8 +951,9 @@ __global__ void __launch_bounds__(kFftThreads, 5) k_pass_e(const float2* __restr
     constexpr int RS = H + 2;
     static_assert(16 * RS <= 16 * T::PX, "row staging fits the line buffer");
     fft::lines16_rows<H, kFftThreads, 2, true, RS>(s, tw, c2r_load);
-    for (int u = threadIdx.x; u < 16 * (H / 2); u += kFftThreads) {
-        const int l = u / (H / 2), mp = u % (H / 2);
+    constexpr int Q = HALF ? H / 4 : H / 2;  // float4 of a row
+    for (int u = threadIdx.x; u < 16 * Q; u += kFftThreads) {
+        const int l = u / Q, mp = u % Q;
         const size_t row = ((size_t)(bz * 4 + (l >> 2)) * G + by * 4 + (l & 3)) * G;
         const float4 ab = *reinterpret_cast<const float4*>(s + l * RS + 2 * mp);
         *reinterpret_cast<float4*>(phi + row + 4 * mp) = ab;
@@ -943,6 +970,8 @@ struct Launcher {
     }
     static size_t smem_bd() { return sizeof(float2) * ((size_t)G + 16 * (size_t)G); }
     static size_t smem_c() { return sizeof(float2) * ((size_t)G + (T::H + 2) / 2 + 1 + 16 * (size_t)G); }
+    // and the table's values; the lines before them end on a 16-byte boundary
+    static size_t smem_ct() { return smem_c() + sizeof(float) * 16 * (size_t)(T::H + 2); }
     // the line buffer (16 * PX float2) overlays the 32-bit sum words (2 * 16 * (G + 4));
     // at G = 512 the warp-per-line transform's twiddle tables follow the sums
     static size_t smem_bal() {
@@ -957,40 +986,47 @@ struct Launcher {
         return nb < 8 ? 8 : (nb > 296 ? 296 : nb);
     }
 
+    static constexpr bool kIsoBox = G >= 32;  // the transform box of an isolated grid of side G / 2 >= 16
+
     static int configure() {
         int rc = SD_OK;
         // prefer the largest shared-memory carveout so several 70 KB CTAs fit per SM
-        const int carve = (int)cudaSharedmemCarveoutMaxShared;
-        rc |= SD_CUDA(cudaFuncSetAttribute(k_pass_a<G, 0>, cudaFuncAttributePreferredSharedMemoryCarveout, carve));
-        rc |= SD_CUDA(cudaFuncSetAttribute(k_pass_a<G, 1>, cudaFuncAttributePreferredSharedMemoryCarveout, carve));
-        rc |= SD_CUDA(cudaFuncSetAttribute(k_pass_y<G, false>, cudaFuncAttributePreferredSharedMemoryCarveout, carve));
-        rc |= SD_CUDA(cudaFuncSetAttribute(k_pass_y<G, true>, cudaFuncAttributePreferredSharedMemoryCarveout, carve));
-        rc |= SD_CUDA(cudaFuncSetAttribute(k_pass_c<G, 0>, cudaFuncAttributePreferredSharedMemoryCarveout, carve));
-        rc |= SD_CUDA(cudaFuncSetAttribute(k_pass_c<G, 1>, cudaFuncAttributePreferredSharedMemoryCarveout, carve));
-        rc |= SD_CUDA(cudaFuncSetAttribute(k_pass_c<G, 2>, cudaFuncAttributePreferredSharedMemoryCarveout, carve));
-        rc |= SD_CUDA(cudaFuncSetAttribute(k_pass_e<G>, cudaFuncAttributePreferredSharedMemoryCarveout, carve));
-        rc |= SD_CUDA(cudaFuncSetAttribute(k_pass_a_deposit_bal<G>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                           carve));
-        rc |= SD_CUDA(cudaFuncSetAttribute(k_pass_a<G, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a()));
-        rc |= SD_CUDA(cudaFuncSetAttribute(k_pass_a<G, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a()));
-        rc |= SD_CUDA(cudaFuncSetAttribute(k_pass_y<G, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem_bd()));
-        rc |= SD_CUDA(cudaFuncSetAttribute(k_pass_y<G, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem_bd()));
-        rc |= SD_CUDA(cudaFuncSetAttribute(k_pass_c<G, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_c()));
-        rc |= SD_CUDA(cudaFuncSetAttribute(k_pass_c<G, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_c()));
-        rc |= SD_CUDA(cudaFuncSetAttribute(k_pass_c<G, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_c()));
-        rc |= SD_CUDA(cudaFuncSetAttribute(k_pass_e<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_ae()));
-        rc |= SD_CUDA(cudaFuncSetAttribute(k_pass_a_deposit_bal<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem_bal()));
+        auto set = [&rc](auto* kernel, size_t smem) {
+            rc |= SD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                               (int)cudaSharedmemCarveoutMaxShared));
+            rc |= SD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        };
+        set(k_pass_a<G, 0>, smem_a());
+        set(k_pass_a<G, 1>, smem_a());
+        set(k_pass_y<G, false, false>, smem_bd());
+        set(k_pass_y<G, true, false>, smem_bd());
+        set(k_pass_c<G, 0, false>, smem_c());
+        set(k_pass_c<G, 1, false>, smem_c());
+        set(k_pass_e<G, false>, smem_ae());
+        set(k_pass_a_deposit_bal<G>, smem_bal());
+        if constexpr (kIsoBox) {
+            set(k_pass_y<G, false, true>, smem_bd());
+            set(k_pass_y<G, true, true>, smem_bd());
+            set(k_pass_c<G, 2, true>, smem_ct());
+            set(k_pass_e<G, true>, smem_ae());
+        }
         return rc == SD_OK ? SD_OK : SD_E_CUDA;
     }
 
     static int run(const PoissonPlan& p, const long long* acc, const float* rho, const float4* pos, const int* perm,
                    const int* row_start, float* keep, float2* spec, float* phi, cudaStream_t s, cudaEvent_t* ev,
                    const PoissonIso* iso, const DepositWork* dw) {
-        const dim3 grid_rows(T::NBY, T::NBZ), grid_y(T::NBX, T::NBZ), grid_z(T::NBX, T::NBY);
         const int src_g = (iso && iso->src_g > 0) ? iso->src_g : G;
+        // isolated boundary: the density fills an eighth of the box and the potential is
+        // read only there. Pass A runs on the quarter of the rows that hold particles,
+        // the y passes on the half of the slabs, every line reads and stores the half
+        // that is not zero or wanted, pass E makes a quarter of the rows: a third of the
+        // full box's traffic (a 256^3 box: A 39 -> 19 us, B 27 -> 13, C 42 -> 29, D 27 -> 13,
+        // E 33 -> 9; a 512^3 box: 266 -> 90, 210 -> 112, 402 -> 253, 210 -> 88, 234 -> 55).
+        const bool half = kIsoBox && iso && iso->table && 2 * src_g == G;
+        if (iso && iso->table && !half) return fail(SD_E_ARG, "poisson: the isolated density has half the box's side");
+        const int hy = half ? T::NBY / 2 : T::NBY, hz = half ? T::NBZ / 2 : T::NBZ;
+        const dim3 grid_rows(hy, hz), grid_y(T::NBX, hz), grid_z(T::NBX, T::NBY);
         if (pos) {
             if (!dw || !dw->acc || !dw->ints || dw->split <= 0) return fail(SD_E_ARG, "fused deposit: no work plan");
             k_deposit_plan<G><<<DepPlan<G>::NC, 256, 0, s>>>(row_start, dw->ints, dw->split);
@@ -1004,25 +1040,38 @@ struct Launcher {
             k_pass_a<G, 0><<<grid_rows, kFftThreads, smem_a(), s>>>(rho, nullptr, keep, spec, p.tw, src_g);
         SD_LAUNCHED(s);
         if (ev) cudaEventRecord(ev[0], s);
-        k_pass_y<G, false><<<grid_y, kFftThreads, smem_bd(), s>>>(spec, p.tw);
+        if constexpr (kIsoBox) {
+            if (half) {
+                k_pass_y<G, false, true><<<grid_y, kFftThreads, smem_bd(), s>>>(spec, p.tw);
+                SD_LAUNCHED(s);
+                if (ev) cudaEventRecord(ev[1], s);
+                k_pass_c<G, 2, true><<<grid_z, kFftThreads, smem_ct(), s>>>(spec, p.tw, p.gexp, p.scale, iso->table,
+                                                                           iso->table_scale);
+                SD_LAUNCHED(s);
+                if (ev) cudaEventRecord(ev[2], s);
+                k_pass_y<G, true, true><<<grid_y, kFftThreads, smem_bd(), s>>>(spec, p.tw);
+                SD_LAUNCHED(s);
+                if (ev) cudaEventRecord(ev[3], s);
+                k_pass_e<G, true><<<grid_rows, kFftThreads, smem_ae(), s>>>(spec, phi, p.tw);
+                SD_LAUNCHED(s);
+                return SD_OK;
+            }
+        }
+        k_pass_y<G, false, false><<<grid_y, kFftThreads, smem_bd(), s>>>(spec, p.tw);
         SD_LAUNCHED(s);
         if (ev) cudaEventRecord(ev[1], s);
         if (iso && iso->forward_only) {
-            k_pass_c<G, 1><<<grid_z, kFftThreads, smem_c(), s>>>(spec, p.tw, p.gexp, p.scale, nullptr, 0.f);
+            k_pass_c<G, 1, false><<<grid_z, kFftThreads, smem_c(), s>>>(spec, p.tw, p.gexp, p.scale, nullptr, 0.f);
             SD_LAUNCHED(s);
             return SD_OK;
         }
-        if (iso && iso->table)
-            k_pass_c<G, 2><<<grid_z, kFftThreads, smem_c(), s>>>(spec, p.tw, p.gexp, p.scale, iso->table,
-                                                                 iso->table_scale);
-        else
-            k_pass_c<G, 0><<<grid_z, kFftThreads, smem_c(), s>>>(spec, p.tw, p.gexp, p.scale, nullptr, 0.f);
+        k_pass_c<G, 0, false><<<grid_z, kFftThreads, smem_c(), s>>>(spec, p.tw, p.gexp, p.scale, nullptr, 0.f);
         SD_LAUNCHED(s);
         if (ev) cudaEventRecord(ev[2], s);
-        k_pass_y<G, true><<<grid_y, kFftThreads, smem_bd(), s>>>(spec, p.tw);
+        k_pass_y<G, true, false><<<grid_y, kFftThreads, smem_bd(), s>>>(spec, p.tw);
         SD_LAUNCHED(s);
         if (ev) cudaEventRecord(ev[3], s);
-        k_pass_e<G><<<grid_rows, kFftThreads, smem_ae(), s>>>(spec, phi, p.tw);
+        k_pass_e<G, false><<<grid_rows, kFftThreads, smem_ae(), s>>>(spec, phi, p.tw);
         SD_LAUNCHED(s);
         return SD_OK;
     }
@@ -1136,7 +1185,7 @@ int launch_poisson_ex(const PoissonPlan& p, const long long* acc, const float* r
 
 size_t green_table_elems(int S) {
     const size_t h = (size_t)S / 2 + 1;
-    return h * h * h;
+    return h * h * (h + 3);
 }
 
 int build_green_table(const PoissonPlan& p, float softening_cells, float* kernel_grid, float2* spec, float* table,

@@ -51,6 +51,21 @@ def test_isolated_potential_and_accel_match_fp64(cuda, oracle, G):
     assert rel_rms(a, a64) < 5e-5
 
 
+@pytest.mark.parametrize("G", [16, 128, 256])
+def test_isolated_transform_sizes(cuda, oracle, G):
+    # the smallest and the largest transform boxes, 2 G a side: the parts of the lines
+    # and rows that are neither read nor stored. The bound on phi as above (FP32 FFT).
+    n = 3_001
+    pos, vel = scene(n, G)
+    with iso_sim(n, G, keep_density=1) as s:
+        s.set_particles(pos, vel)
+        for _ in range(2):  # the second solve finds the first one's spectrum and potential
+            s.accel()
+        phi, rho = s.potential(), s.density()
+    phi64 = oracle.poisson_isolated_f64(rho.astype(np.float64), 1.5)
+    assert np.abs(phi - phi64).max() < 2e-5 * np.abs(phi64).max()
+
+
 def test_isolated_newton_units_scale_by_grid(cuda):
     G, n = 32, 20_000
     pos, vel = scene(n, 3)
