@@ -76,6 +76,19 @@ __device__ __forceinline__ uint32_t order_key(float4 p, int G, int order) {
     return (uint32_t)((cz * G + cy) * G + cx) + 1u;
 }
 
+// Row table of sorted keys: entry r is the first position whose key is at least
+// row_low(r, shift). Tiled keys are rows themselves (shift < 0; entries 0..G^2).
+// Row-major and Morton keys hold 2^shift = G cells of a row (or of a run of the
+// Morton curve) next to each other: entry 0 is the empty slots (key 0), entry r + 1
+// starts row r (entries 0..G^2 + 1). row_of is the last entry whose low key is not
+// above a key.
+__host__ __device__ __forceinline__ uint32_t row_low(int r, int shift) {
+    return shift < 0 ? (uint32_t)r : (r ? ((uint32_t)(r - 1) << shift) + 1u : 0u);
+}
+__host__ __device__ __forceinline__ uint32_t row_of(uint32_t key, int shift) {
+    return shift < 0 ? key : (key ? ((key - 1u) >> shift) + 1u : 0u);
+}
+
 __device__ __forceinline__ unsigned lanemask_lt() {
     unsigned m;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));

@@ -99,8 +99,17 @@ size_t green_table_elems(int S);
 // kernel_grid (S^3 floats) and spec are scratch.
 int build_green_table(const PoissonPlan& p, float softening_cells, float* kernel_grid, float2* spec, float* table,
                       cudaStream_t s);
-// row_start[r] = first index i with sorted row keys[i] >= r, for r in [0, rows]
-int launch_row_bounds(const uint32_t* keys, int n, int rows, int* row_start, cudaStream_t s);
+// row_start[r] = first index i with sorted keys[i] >= row_low(r, shift), for r in
+// [0, rows] (sd_common.cuh; rows = row_last(G, order), shift = row_shift(G, order))
+int launch_row_bounds(const uint32_t* keys, int n, int rows, int shift, int* row_start, cudaStream_t s);
+// the row table's last entry and its key shift (see row_low)
+inline int row_shift(int G, int order) {
+    if (order == SD_ORDER_TILED) return -1;
+    int b = 0;
+    while ((1 << b) < G) ++b;
+    return b;
+}
+inline int row_last(int G, int order) { return order == SD_ORDER_TILED ? G * G : G * G + 1; }
 
 size_t gather_partials(int n);
 // one-time per-device set-up of the gather's default grid (call outside stream capture)
@@ -166,7 +175,7 @@ ResortBufs resort_layout(void* base, int n, int G, uint32_t* spare_k0, int32_t* 
 // keys: the new key of every position, positions sorted by their old keys, whose
 // row table is row_start; writes the stable sort's permutation to vals_out and
 // the new keys' row table over row_start.
-int launch_resort(const ResortBufs& r, const uint32_t* keys, int n, int G, int key_bits, int* row_start,
+int launch_resort(const ResortBufs& r, const uint32_t* keys, int n, int G, int order, int key_bits, int* row_start,
                   int32_t* vals_out, void* sort_ws, size_t sort_ws_bytes, cudaStream_t s);
 
 // Grid hydrodynamics add-ons (sd_hydro.cu): per-cell fixed-point sums for cooling

@@ -1,10 +1,11 @@
-// sd_resort.cu -- the step's sort as a merge, for the tiled order.
+// sd_resort.cu -- the step's sort as a merge.
 //
-// Between two steps a particle's row key changes only when it crosses a row:
-// a fraction of a percent of the particles on the 16M/512^3 field. The previous
-// step left the particles sorted by their old keys, its row table
-// (row_start[r] = first position with old key >= r) and, from its gather, the
-// new key of every position plus a bit per position saying whether it changed.
+// Between two steps a particle's key changes only when it crosses a row (tiled
+// order) or a cell (row-major, Morton): a percent of the particles or less on the
+// 16M/512^3 field. The previous step left the particles sorted by their old keys,
+// its row table (row_start[r] = first position with old key >= row_low(r)) and,
+// from its gather, the new key of every position plus a bit per position saying
+// whether it changed.
 // The stable sort of the new keys is then the merge of
 //   U  the unchanged positions, already in (key, position) order, and
 //   C  the changed ones, radix-sorted by key (stable, so in position order
@@ -14,9 +15,11 @@
 //   changed  (k, i) at rank r in C:  r + #U before it, where the unchanged
 //            positions before it are those below row_start[k] plus those in
 //            [row_start[k], row_start[k+1]) below i, less the changed ones
-//            among them (prefix counts of the change bits);
-//   unchanged (k, j):  j - #changed below j + #C with key < k (a row table of
-//            the sorted C) + #C with key k and position < j.
+//            among them (prefix counts of the change bits); where a row holds many
+//            keys (row-major, Morton), a binary search of the row's unchanged
+//            positions, whose keys are still in order, takes the place of i;
+//   unchanged (k, j):  j - #changed below j + #C with row below k's (a row table of
+//            the sorted C) + #C of the same row and (key, position) below (k, j).
 // The new row table needs no pass over the keys either: the positions below
 // row r are the unchanged ones below the old row_start[r] plus the changed
 // ones with key < r. The permutation is the one the radix sort gives; the
@@ -163,42 +166,71 @@ __device__ __forceinline__ unsigned changed_below(const unsigned* __restrict__ w
     return word_pre[x >> 5] + __popc(words[x >> 5] & m);
 }
 
+// First unchanged position at or after q (hi when there is none before hi).
+__device__ __forceinline__ int next_unchanged(const unsigned* __restrict__ words, int q, int hi) {
+    int w = q >> 5;
+    unsigned u = ~words[w] & (0xffffffffu << (q & 31));
+    while (u == 0u) {
+        if ((++w << 5) >= hi) return hi;
+        u = ~words[w];
+    }
+    return min(hi, (w << 5) + __ffs(u) - 1);
+}
+
+// WIDE: rows hold many keys (shift >= 0); otherwise the key is the row.
+template <bool WIDE>
 __global__ void k_merge_changed(const uint32_t* __restrict__ ck, const int32_t* __restrict__ ci,
-                                const int* __restrict__ n_changed, const int* __restrict__ row_start_old,
-                                const unsigned* __restrict__ words, const unsigned* __restrict__ word_pre,
-                                int32_t* __restrict__ vals_out) {
+                                const int* __restrict__ n_changed, const uint32_t* __restrict__ keys, int shift,
+                                const int* __restrict__ row_start_old, const unsigned* __restrict__ words,
+                                const unsigned* __restrict__ word_pre, int32_t* __restrict__ vals_out) {
     const int nc = *n_changed;
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nc; r += gridDim.x * blockDim.x) {
         const uint32_t k = ck[r];
         const int i = ci[r];
-        const int lb = row_start_old[k], ub = row_start_old[k + 1];
-        const unsigned cl = changed_below(words, word_pre, lb);
-        unsigned u = (unsigned)lb - cl;
-        if (i > lb) {
-            const int m = min(ub, i);
-            u += (unsigned)(m - lb) - (changed_below(words, word_pre, m) - cl);
+        const uint32_t row = WIDE ? row_of(k, shift) : k;
+        const int lb = row_start_old[row], ub = row_start_old[row + 1];
+        if (WIDE) {
+            // the row's unchanged positions are in (key, position) order: find the first
+            // that is not before (k, i), stepping over the changed ones
+            int lo = lb, hi = ub;
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                const int q = next_unchanged(words, mid, hi);
+                const uint32_t kq = q < hi ? keys[q] : 0xffffffffu;
+                if (kq < k || (kq == k && q < i)) lo = q + 1;
+                else hi = mid;
+            }
+            vals_out[r + lo - (int)changed_below(words, word_pre, lo)] = i;
+        } else {
+            const unsigned cl = changed_below(words, word_pre, lb);
+            unsigned u = (unsigned)lb - cl;
+            if (i > lb) {
+                const int m = min(ub, i);
+                u += (unsigned)(m - lb) - (changed_below(words, word_pre, m) - cl);
+            }
+            vals_out[r + u] = i;
         }
-        vals_out[r + u] = i;
     }
 }
 
-// Thread per row r in [0, rows]: c_rows[r] = first rank of C with key >= r, and
+// Thread per row r in [0, rows]: c_rows[r] = first rank of C with key >= row_low(r), and
 // the new row start = unchanged positions below the old one + c_rows[r]. The
 // search starts where r would fall if C were spread evenly over the rows and
 // gallops outwards to a bracket, which a few steps find for an even spread.
-__global__ void k_rows(const uint32_t* __restrict__ ck, const int* __restrict__ n_changed, int rows,
+__global__ void k_rows(const uint32_t* __restrict__ ck, const int* __restrict__ n_changed, int rows, int shift,
                        const unsigned* __restrict__ words, const unsigned* __restrict__ word_pre,
                        int* __restrict__ c_rows, int* __restrict__ row_start) {
     const int nc = *n_changed;
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r <= rows; r += gridDim.x * blockDim.x) {
-        // bracket [lo, hi] with ck[lo - 1] < r <= ck[hi] (ck[-1] = -inf, ck[nc] = +inf)
+        const uint32_t low = row_low(r, shift);
+        // bracket [lo, hi] with ck[lo - 1] < low <= ck[hi] (ck[-1] = -inf, ck[nc] = +inf)
         const int g = (int)(((long long)r * nc) / (rows > 0 ? rows : 1));
         int lo, hi;
-        if (g < nc && ck[g] < (uint32_t)r) {  // the answer lies above g
+        if (g < nc && ck[g] < low) {  // the answer lies above g
             int step = 1;
             lo = g + 1;
             hi = g + 1;
-            while (hi < nc && ck[hi] < (uint32_t)r) {
+            while (hi < nc && ck[hi] < low) {
                 lo = hi + 1;
                 hi = min(nc, hi + step);
                 step <<= 1;
@@ -207,7 +239,7 @@ __global__ void k_rows(const uint32_t* __restrict__ ck, const int* __restrict__ 
             int step = 1;
             hi = g;
             lo = g;
-            while (lo > 0 && ck[lo - 1] >= (uint32_t)r) {
+            while (lo > 0 && ck[lo - 1] >= low) {
                 hi = lo - 1;
                 lo = max(0, lo - step);
                 step <<= 1;
@@ -215,7 +247,7 @@ __global__ void k_rows(const uint32_t* __restrict__ ck, const int* __restrict__ 
         }
         while (lo < hi) {
             const int mid = (lo + hi) >> 1;
-            if (ck[mid] < (uint32_t)r) lo = mid + 1;
+            if (ck[mid] < low) lo = mid + 1;
             else hi = mid;
         }
         c_rows[r] = lo;
@@ -227,10 +259,12 @@ __global__ void k_rows(const uint32_t* __restrict__ ck, const int* __restrict__ 
 // Warp per 8 words (256 positions, lane-major: position = base + 32 q + lane), all
 // loads issued before use. The changed positions were placed by k_merge_changed.
 // Clears the change bits for the next gather.
+template <bool WIDE>
 __global__ void __launch_bounds__(kMergeThreads) k_merge_unchanged(const uint32_t* __restrict__ keys,
                                                                    unsigned* __restrict__ words,
                                                                    const unsigned* __restrict__ word_pre,
-                                                                   const int* __restrict__ c_rows,
+                                                                   const int* __restrict__ c_rows, int shift,
+                                                                   const uint32_t* __restrict__ ck,
                                                                    const int32_t* __restrict__ ci, int n,
                                                                    int32_t* __restrict__ vals_out) {
     const int lane = threadIdx.x & 31;
@@ -249,19 +283,25 @@ __global__ void __launch_bounds__(kMergeThreads) k_merge_unchanged(const uint32_
     int lo[8], hi[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-        lo[q] = c_rows[k[q]];
-        hi[q] = c_rows[k[q] + 1];
+        const uint32_t row = WIDE ? row_of(k[q], shift) : k[q];
+        lo[q] = c_rows[row];
+        hi[q] = c_rows[row + 1];
     }
     const unsigned lt = lanemask_lt();
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
         const int j = base + q * 32 + lane;
         if (j < n && !((bits[q] >> lane) & 1u)) {
-            // C entries with key k lie at ranks [c_rows[k], c_rows[k+1]) in position order
+            // C entries of k's row lie at ranks [c_rows[row], c_rows[row+1]) in (key, position) order
             int a = lo[q], b = hi[q];
-            while (a < b) {  // first rank whose position is above j
+            while (a < b) {  // first rank that is above (k, j)
                 const int mid = (a + b) >> 1;
-                if (ci[mid] < j) a = mid + 1;
+                bool before = ci[mid] < j;
+                if (WIDE) {
+                    const uint32_t kc = ck[mid];
+                    before = kc < k[q] || (kc == k[q] && before);
+                }
+                if (before) a = mid + 1;
                 else b = mid;
             }
             vals_out[j - (int)(pre[q] + __popc(bits[q] & lt)) + a] = j;
@@ -284,7 +324,7 @@ size_t resort_words(int n) { return padded_words(n); }
 size_t resort_bytes(int n, int G) {
     const size_t words = padded_words(n), chunks = words / kChunkWords;
     return align_up(sizeof(unsigned) * words, 256) * 2 + align_up(sizeof(unsigned) * chunks, 256) +
-           align_up(sizeof(int32_t) * ((size_t)G * G + 1), 256) + align_up(sizeof(int), 256) +
+           align_up(sizeof(int32_t) * ((size_t)G * G + 2), 256) + align_up(sizeof(int), 256) +
            3 * align_up(sizeof(uint32_t) * (size_t)n, 256);
 }
 
@@ -299,7 +339,7 @@ ResortBufs resort_layout(void* base, int n, int G, uint32_t* spare_k0, int32_t* 
     r.chunk_cnt = (unsigned*)b;
     b += align_up(sizeof(unsigned) * chunks, 256);
     r.c_rows = (int*)b;
-    b += align_up(sizeof(int32_t) * ((size_t)G * G + 1), 256);
+    b += align_up(sizeof(int32_t) * ((size_t)G * G + 2), 256);
     r.n_changed = (int*)b;
     b += align_up(sizeof(int), 256);
     r.ck_out = (uint32_t*)b;
@@ -313,11 +353,11 @@ ResortBufs resort_layout(void* base, int n, int G, uint32_t* spare_k0, int32_t* 
     return r;
 }
 
-int launch_resort(const ResortBufs& r, const uint32_t* keys, int n, int G, int key_bits, int* row_start,
+int launch_resort(const ResortBufs& r, const uint32_t* keys, int n, int G, int order, int key_bits, int* row_start,
                   int32_t* vals_out, void* sort_ws, size_t sort_ws_bytes, cudaStream_t s) {
     if (n <= 0) return SD_OK;
     const int chunks = (int)(padded_words(n) / kChunkWords);
-    const int rows = G * G;
+    const int rows = row_last(G, order), shift = row_shift(G, order);
     k_chg_count<<<chunks, kChgThreads, 0, s>>>(r.words, r.chunk_cnt);
     SD_LAUNCHED(s);
     k_chg_compact<<<chunks, kChgThreads, 0, s>>>(r.words, r.chunk_cnt, keys, r.word_pre, r.ck_in, r.ci_in,
@@ -327,15 +367,17 @@ int launch_resort(const ResortBufs& r, const uint32_t* keys, int n, int G, int k
     int rc = launch_sort_pairs(r.ck_in, r.ci_in, r.ck_out, r.ci_out, r.ck_tmp, r.ci_tmp, n, key_bits, sort_ws,
                                sort_ws_bytes, s, true, false, r.n_changed);
     if (rc) return rc;
-    k_merge_changed<<<148 * 4, 256, 0, s>>>(r.ck_out, r.ci_out, r.n_changed, row_start, r.words, r.word_pre,
-                                            vals_out);
+    auto changed = shift < 0 ? k_merge_changed<false> : k_merge_changed<true>;
+    changed<<<148 * 4, 256, 0, s>>>(r.ck_out, r.ci_out, r.n_changed, keys, shift, row_start, r.words, r.word_pre,
+                                    vals_out);
     SD_LAUNCHED(s);
-    k_rows<<<(rows + 1 + 255) / 256, 256, 0, s>>>(r.ck_out, r.n_changed, rows, r.words, r.word_pre, r.c_rows,
+    k_rows<<<(rows + 1 + 255) / 256, 256, 0, s>>>(r.ck_out, r.n_changed, rows, shift, r.words, r.word_pre, r.c_rows,
                                                    row_start);
     SD_LAUNCHED(s);
     const int warps = (n + 255) / 256;
-    k_merge_unchanged<<<(warps + kMergeThreads / 32 - 1) / (kMergeThreads / 32), kMergeThreads, 0, s>>>(
-        keys, r.words, r.word_pre, r.c_rows, r.ci_out, n, vals_out);
+    auto unchanged = shift < 0 ? k_merge_unchanged<false> : k_merge_unchanged<true>;
+    unchanged<<<(warps + kMergeThreads / 32 - 1) / (kMergeThreads / 32), kMergeThreads, 0, s>>>(
+        keys, r.words, r.word_pre, r.c_rows, shift, r.ck_out, r.ci_out, n, vals_out);
     SD_LAUNCHED(s);
     return SD_OK;
 }

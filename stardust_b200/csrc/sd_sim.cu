@@ -214,7 +214,7 @@ int allocate(sd_sim* s) {
     // the sort's count buffers start zero and every sort leaves them zero
     if (!rc && SD_CUDA(cudaMemset(s->sort_ws, 0, s->sort_ws_bytes))) rc = SD_E_CUDA;
     rc = rc ? rc : alloc_dev(s->acc, cells);
-    rc = rc ? rc : alloc_dev(s->row_start, (size_t)s->G * s->G + 1);
+    rc = rc ? rc : alloc_dev(s->row_start, (size_t)s->G * s->G + 2);
     rc = rc ? rc : alloc_dev(s->dep_ints, deposit_work_ints(s->G));
     rc = rc ? rc : alloc_dev(s->spec, poisson_spectrum_elems(S));
     rc = rc ? rc : alloc_dev(s->phi, box);
@@ -296,23 +296,29 @@ void invalidate_keys(sd_sim* s) {
 }
 
 bool incr_possible(const sd_sim* s) {
-    return s->allow_incr && s->cfg.full_sort != 1 && s->cfg.order == SD_ORDER_TILED && !isolated(s);
+    return s->allow_incr && s->cfg.full_sort != 1 && !isolated(s);
 }
 
 // Above this share of changed keys the full radix sort is cheaper than the merge
 // (4M particles on 256^3 with a third of the keys changing: merge 0.146 ms, full
 // sort with its row table 0.093 ms; 16M on 512^3 with 0.8 % changing: merge
-// 0.12 ms, full sort 0.23 ms). Below kMergeMinParticles the merge's dozen launches
-// cost more than a full sort whatever changes (262,144 particles on 64^3 with 9 %
-// changing: merge 0.107 ms, full sort and row table 0.05 ms).
+// 0.12 ms, full sort 0.23 ms). Below merge_min_particles the merge's dozen launches
+// cost more than a full sort whatever changes (tiled, 262,144 particles on 64^3 with
+// 9 % changing: merge 0.107 ms, full sort and row table 0.05 ms). The tiled order's
+// two-pass sort breaks even at 2^22 (a step on 256^3: 3,000,000 particles full 0.370,
+// merge 0.373 ms; 4,194,304 0.415 and 0.414 ms); the three passes of the row-major and
+// Morton cell keys earlier. In captured steps on 128^3 at 2^20 (0.205 and 0.164 ms), in
+// eager steps, which issue the merge's extra launches from the host, at 2^21 (2,000,000
+// particles 0.411 and 0.421 ms); 3,000,000 on 256^3 captured 0.569 and 0.479 ms,
+// 8,000,003 1.00 and 0.72 ms.
 constexpr double kMergeMaxFraction = 0.10;
 constexpr int kMergeProbe = 64;
-constexpr int kMergeMinParticles = 1 << 22;
+int merge_min_particles(const sd_sim* s) { return s->cfg.order == SD_ORDER_TILED ? 1 << 22 : 1 << 21; }
 
 // The next sorted step leaves change bits for a merge (otherwise first-pass counts).
 bool merge_next(const sd_sim* s) {
     if (!s->rs_base || !incr_possible(s)) return false;
-    return s->cfg.full_sort == -1 || (!s->merge_off && s->N >= kMergeMinParticles);
+    return s->cfg.full_sort == -1 || (!s->merge_off && s->N >= merge_min_particles(s));
 }
 
 // Read the share of keys the last merge found changed (written to pinned memory
@@ -334,7 +340,47 @@ void update_merge_policy(sd_sim* s) {
     }
 }
 
-// Merge-sort buffers exist while the configuration can merge-sort (zeroed when made).
+// The changed-key counts' host slots: one static page, page-locked once per context,
+// one int per handle while it lives. A pinned allocation of its own for each handle
+// cost 1-3 ms at init. Handles past the page's 1,024 get an allocation.
+alignas(4096) int g_chg_slots[1024];
+bool g_chg_used[1024];
+std::mutex g_chg_mu;
+
+int* take_chg_slot() {
+    std::lock_guard<std::mutex> lk(g_chg_mu);
+    // again after a device reset, which ends the registration; otherwise already registered
+    const cudaError_t e = cudaHostRegister(g_chg_slots, sizeof(g_chg_slots), cudaHostRegisterPortable);
+    if (e != cudaSuccess) cudaGetLastError();
+    if (e == cudaSuccess || e == cudaErrorHostMemoryAlreadyRegistered)
+        for (int i = 0; i < 1024; ++i)
+            if (!g_chg_used[i]) {
+                g_chg_used[i] = true;
+                return g_chg_slots + i;
+            }
+    int* p = nullptr;
+    if (cudaHostAlloc((void**)&p, sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return p;
+}
+
+// the handle's work is done (sd_destroy): nothing writes the slot any more
+void give_chg_slot(int* p) {
+    if (!p) return;
+    const uintptr_t at = (uintptr_t)p, base = (uintptr_t)g_chg_slots;
+    if (at < base || at >= base + sizeof(g_chg_slots)) {
+        cudaFreeHost(p);
+        return;
+    }
+    std::lock_guard<std::mutex> lk(g_chg_mu);
+    g_chg_used[p - g_chg_slots] = false;
+}
+
+// Merge-sort buffers are made (zeroed) when the configuration merge-sorts and kept
+// while it can; they cover every allocated slot, as a later request may only narrow
+// the range in use.
 int ensure_resort(sd_sim* s) {
     if (!incr_possible(s)) {
         if (s->rs_base) cudaFree(s->rs_base);
@@ -342,25 +388,22 @@ int ensure_resort(sd_sim* s) {
         s->incr_ready = s->chg_dirty = false;
         return SD_OK;
     }
-    if (s->rs_base) return SD_OK;
+    if (s->rs_base || (s->cfg.full_sort != -1 && s->N < merge_min_particles(s))) return SD_OK;
     if (!s->chg_host) {
-        if (cudaHostAlloc((void**)&s->chg_host, sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
-            cudaGetLastError();
-            s->chg_host = nullptr;
-            return fail(SD_E_NOMEM, "cudaHostAlloc of the changed-key count failed");
-        }
+        s->chg_host = take_chg_slot();
+        if (!s->chg_host) return fail(SD_E_NOMEM, "cudaHostAlloc of the changed-key count failed");
         *s->chg_host = -1;
     }
     s->chg_frac = -1.0;
     s->merge_off = false;
-    const size_t b = resort_bytes(s->N, s->G);
+    const size_t b = resort_bytes(s->capacity, s->G);
     if (cudaMalloc(&s->rs_base, b) != cudaSuccess) {
         cudaGetLastError();
         s->rs_base = nullptr;
         return fail(SD_E_NOMEM, "cudaMalloc of the merge-sort buffers failed");
     }
     // the full sort's scratch (sorted keys, temporaries) is idle while a merge runs
-    s->rs = resort_layout(s->rs_base, s->N, s->G, s->keys2, s->vals2, s->keys3);
+    s->rs = resort_layout(s->rs_base, s->capacity, s->G, s->keys2, s->vals2, s->keys3);
     s->incr_ready = s->chg_dirty = false;
     return SD_CUDA(cudaMemset(s->rs_base, 0, b));
 }
@@ -481,8 +524,8 @@ int do_step(sd_sim* s, float dt, bool sort, bool timed) {
     bool merged = false;  // the merge also left the new row table
     if (sort) {
         if (s->incr_ready && s->keys_valid && s->rs_base) {
-            rc = launch_resort(s->rs, s->keys, s->N, s->G, key_bits_for(s->G, s->cfg.order), s->row_start, s->vals,
-                               s->sort_ws, s->sort_ws_bytes, s->stream);
+            rc = launch_resort(s->rs, s->keys, s->N, s->G, s->cfg.order, key_bits_for(s->G, s->cfg.order),
+                               s->row_start, s->vals, s->sort_ws, s->sort_ws_bytes, s->stream);
             if (rc) return sim_error(s, rc);
             // the share of changed keys, for the choice between merge and full sort
             if (s->chg_host && SD_CUDA(cudaMemcpyAsync(s->chg_host, s->rs.n_changed, sizeof(int),
@@ -513,12 +556,13 @@ int do_step(sd_sim* s, float dt, bool sort, bool timed) {
     // (The isolated boundary always takes the atomic deposit, which clamps corners
     // onto the edge cells.)
     const bool fused = sort && s->cfg.order == SD_ORDER_TILED && !isolated(s);
-    if (fused) {
-        if (!merged && (rc = launch_row_bounds(s->keys2, s->N, s->G * s->G, s->row_start, s->stream)))
-            return sim_error(s, rc);
-    } else if ((rc = launch_deposit_fixed(s->pos, s->N, s->G, s->acc, s->stream, isolated(s) ? 0 : 1))) {
+    // the row table of the sorted keys, for the fused deposit and the next step's merge
+    if (!merged && (fused || incr_next) &&
+        (rc = launch_row_bounds(s->keys2, s->N, row_last(s->G, s->cfg.order), row_shift(s->G, s->cfg.order),
+                                s->row_start, s->stream)))
         return sim_error(s, rc);
-    }
+    if (!fused && (rc = launch_deposit_fixed(s->pos, s->N, s->G, s->acc, s->stream, isolated(s) ? 0 : 1)))
+        return sim_error(s, rc);
     if (timed) cudaEventRecord(s->ev[2], s->stream);
     PoissonIso io;
     DepositWork dw;
@@ -930,7 +974,7 @@ int sd_destroy(sd_sim* s) {
         if (e) cudaEventDestroy(e);
     if (s->out_ev) cudaEventDestroy(s->out_ev);
     if (s->up_stream) cudaStreamDestroy(s->up_stream);
-    if (s->chg_host) cudaFreeHost(s->chg_host);
+    give_chg_slot(s->chg_host);
     for (auto& e : s->ev)
         if (e) cudaEventDestroy(e);
     for (auto& e : s->pev)
@@ -1288,6 +1332,7 @@ int sd_step_auto(sd_sim* s) {
     float dt = 0.0016f * dt_scale_for(s->cfg.time_scale);
     const float dt_max = (vmax > 1e-6f) ? (0.8f * cell / vmax) : dt;
     if (dt > dt_max) dt = dt_max;
+    update_merge_policy(s);
     rc = do_step(s, dt, sort_due(s), true);
     if (rc) return rc;
     s->tm.dt_used = dt;

@@ -451,10 +451,10 @@ __global__ void k_copy_keys(const uint32_t* __restrict__ kin, const int32_t* __r
     vout[i] = vin ? vin[i] : i;
 }
 
-// Sorted row keys (tiled order: key = row, below `rows`) -> row_start[r] = first
-// position whose key is >= r, r = 0..rows (row_start[rows] = n). Thread per
-// position i in [0, n]: the rows r in (key[i-1], key[i]] start at i (position 0
-// takes the rows up to key[0], position n the rows after key[n-1]). One coalesced
+// Sorted keys -> row_start[r] = first position whose key is >= row_low(r, shift),
+// r = 0..rows (row_start[rows] = n). Thread per position i in [0, n]: the rows in
+// (row of key[i-1], row of key[i]] start at i (position 0 takes the rows up to
+// key[0]'s, position n the rows after key[n-1]'s). One coalesced
 // pass over the keys instead of a lower-bound search per row (a chain of dependent
 // loads): a short run of empty rows is written by its own thread, a longer one is
 // queued and written by the whole CTA, so no thread walks a long empty stretch of
@@ -463,7 +463,7 @@ __global__ void k_copy_keys(const uint32_t* __restrict__ kin, const int32_t* __r
 // two-galaxy scene on 256^3: search 0.013 ms, this pass 0.017 ms; 262,144 keys of
 // the disk on 64^3: search 0.011 ms, this pass 0.007 ms).
 constexpr int kRowShortRun = 8;
-__global__ void __launch_bounds__(256) k_row_marks(const uint32_t* __restrict__ keys, int n, int rows,
+__global__ void __launch_bounds__(256) k_row_marks(const uint32_t* __restrict__ keys, int n, int rows, int shift,
                                                    int* __restrict__ row_start) {
     __shared__ int q_lo[256], q_hi[256], q_val[256];
     __shared__ int q_count;
@@ -471,8 +471,8 @@ __global__ void __launch_bounds__(256) k_row_marks(const uint32_t* __restrict__ 
     __syncthreads();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i <= n) {
-        const int prev = (i == 0) ? -1 : (int)__ldg(keys + i - 1);
-        const int cur = (i == n) ? rows : (int)__ldg(keys + i);
+        const int prev = (i == 0) ? -1 : (int)row_of(__ldg(keys + i - 1), shift);
+        const int cur = (i == n) ? rows : (int)row_of(__ldg(keys + i), shift);
         const int run = cur - prev;  // rows prev + 1 .. cur
         if (run > kRowShortRun) {
             const int slot = atomicAdd(&q_count, 1);
@@ -489,13 +489,15 @@ __global__ void __launch_bounds__(256) k_row_marks(const uint32_t* __restrict__ 
 }
 
 // One thread per row: a lower-bound search over the keys.
-__global__ void k_row_bounds(const uint32_t* __restrict__ keys, int n, int rows, int* __restrict__ row_start) {
+__global__ void k_row_bounds(const uint32_t* __restrict__ keys, int n, int rows, int shift,
+                             int* __restrict__ row_start) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r > rows) return;
+    const uint32_t low = row_low(r, shift);
     int lo = 0, len = n;
     while (len > 0) {
         const int half = len >> 1;
-        if (__ldg(keys + lo + half) < (uint32_t)r) {
+        if (__ldg(keys + lo + half) < low) {
             lo += half + 1;
             len -= half + 1;
         } else {
@@ -507,11 +509,11 @@ __global__ void k_row_bounds(const uint32_t* __restrict__ keys, int n, int rows,
 
 }  // namespace
 
-int launch_row_bounds(const uint32_t* keys, int n, int rows, int* row_start, cudaStream_t s) {
+int launch_row_bounds(const uint32_t* keys, int n, int rows, int shift, int* row_start, cudaStream_t s) {
     if (n <= (1 << 20))
-        k_row_marks<<<(n + 1 + 255) / 256, 256, 0, s>>>(keys, n, rows, row_start);
+        k_row_marks<<<(n + 1 + 255) / 256, 256, 0, s>>>(keys, n, rows, shift, row_start);
     else
-        k_row_bounds<<<(rows + 1 + 255) / 256, 256, 0, s>>>(keys, n, rows, row_start);
+        k_row_bounds<<<(rows + 1 + 255) / 256, 256, 0, s>>>(keys, n, rows, shift, row_start);
     SD_LAUNCHED(s);
     return SD_OK;
 }

@@ -432,6 +432,41 @@ def test_merge_sort_equals_full_sort(cuda, G, n, speed):
         assert np.array_equal(v0.view(np.int32), v1.view(np.int32))
 
 
+@pytest.mark.parametrize("order", [L.SD_ORDER_ROWMAJOR, L.SD_ORDER_MORTON])
+@pytest.mark.parametrize("G,n,speed", [(16, 1_000, 3.0), (16, 40_000, 0.3), (64, 262_144, 1.0), (128, 300_000, 0.2),
+                                       (64, 1_500_000, 40.0)])
+def test_merge_sort_of_cell_keys_equals_full_sort(cuda, order, G, n, speed):
+    """The row-major and Morton orders merge too: rows of many keys, empty slots in a
+    row of their own, particles lost on the way (non-finite), steps that do not sort
+    in between. Every particle comes out as the full sort leaves it, bit for bit."""
+    pos, vel = _mover_scene(n, G, speed)
+    vel[::4999, 0] = np.inf  # lost in the first step
+    outs = []
+    for full in (1, -1):
+        with make_sim(cuda, n, G, gravity=200.0, softening_cells=1.0, order=order, full_sort=full) as s:
+            s.set_particles(pos, vel)
+            got = []
+            for _ in range(4):
+                s.step(1e-3)
+            got.append(s.get_particles())
+            s.steps(1e-3, 5)
+            got.append(s.get_particles())
+            cfg = s.config()
+            cfg.sort_interval = 2
+            s.reconfigure(cfg)
+            for _ in range(3):
+                s.step(1e-3)
+            cfg.sort_interval = 1
+            s.reconfigure(cfg)
+            s.steps(1e-3, 4)
+            got.append(s.get_particles())
+            assert s.merge_sorting() == (full == -1)
+            outs.append(got)
+    for (p0, v0), (p1, v1) in zip(outs[0], outs[1]):
+        assert np.array_equal(p0.view(np.int32), p1.view(np.int32))
+        assert np.array_equal(v0.view(np.int32), v1.view(np.int32))
+
+
 def test_merge_sort_with_particles_lost_and_keys_unchanged(cuda):
     """A step where nothing crosses a row (all keys unchanged) and steps where
     some particles are lost (non-finite) merge like the full sort."""

@@ -79,3 +79,51 @@ def test_an_unmarked_change_breaks_the_merge():
     marked[i] = False
     perm, _ = merge_by_counts(old, new, marked, 64)
     assert not np.array_equal(perm, np.argsort(new, kind="stable"))
+
+
+def merge_wide(old, new, marked, rows, shift):
+    """The permutation where a row holds 2^shift keys (key 0, the empty slots, is a row
+    of its own): a binary search of the row's unchanged positions places a changed key."""
+    n = len(old)
+    low = np.concatenate([[0], (np.arange(rows + 1) << shift) + 1])
+    row = np.where(new > 0, ((np.maximum(new, 1) - 1) >> shift) + 1, 0)
+    rs_old = np.searchsorted(old, low, side="left")
+    below = np.concatenate([[0], np.cumsum(marked)])
+    ci = np.nonzero(marked)[0]
+    o = np.argsort(new[ci], kind="stable")
+    ck, ci = new[ci][o], ci[o]
+    c_rows = np.searchsorted(ck, low, side="left")
+    perm = np.full(n, -1, np.int64)
+    for r, (k, i) in enumerate(zip(ck, ci)):
+        lo, hi = rs_old[row[i]], rs_old[row[i] + 1]
+        while lo < hi:
+            mid = (lo + hi) >> 1
+            q = mid
+            while q < hi and marked[q]:
+                q += 1
+            if q < hi and (new[q], q) < (k, i):
+                lo = q + 1
+            else:
+                hi = mid
+        perm[r + lo - below[lo]] = i
+    for j in np.nonzero(~marked)[0]:
+        a, b = c_rows[row[j]], c_rows[row[j] + 1]
+        a += sum((ck[q], ci[q]) < (new[j], j) for q in range(a, b))
+        perm[j - below[j] + a] = j
+    return perm, rs_old - below[rs_old] + c_rows, low
+
+
+@pytest.mark.parametrize("n,rows,shift,frac,stale", [(1, 16, 4, 1.0, 0.0), (700, 16, 4, 0.05, 0.0), (2000, 64, 3, 0.3, 0.1),
+                                                     (900, 16, 5, 1.0, 0.0), (800, 256, 4, 0.02, 0.5)])
+def test_wide_rows(n, rows, shift, frac, stale):
+    rng = np.random.default_rng(n)
+    old = np.sort(rng.integers(0, (rows << shift) + 1, n))
+    old[: n // 20] = 0
+    new = old.copy()
+    moved = rng.random(n) < frac
+    new[moved] = np.clip(old[moved] + rng.choice([-(1 << shift), -1, 1, 1 << shift], moved.sum()), 0, rows << shift)
+    new[moved & (rng.random(n) < 0.05)] = 0  # lost
+    marked = (new != old) | (rng.random(n) < stale)
+    perm, rs, low = merge_wide(old, new, marked, rows, shift)
+    assert np.array_equal(perm, np.argsort(new, kind="stable"))
+    assert np.array_equal(rs, np.searchsorted(np.sort(new), low, side="left"))
