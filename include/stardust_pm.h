@@ -53,7 +53,7 @@ enum { SD_BOUNDARY_ISOLATED = 0, SD_BOUNDARY_PERIODIC = 1 };
 enum {
     SD_ORDER_ROWMAJOR = 0, /* reference key: (cz*G+cy)*G+cx of the containing cell */
     SD_ORDER_MORTON = 1,   /* 30-bit Morton code of the containing cell */
-    SD_ORDER_TILED = 2     /* CIC base-cell rows in 4x4 row tiles (fused deposit/gather) */
+    SD_ORDER_TILED = 2     /* CIC base-cell rows in 4x4 row tiles */
 };
 
 /* Time integrator. SD_INT_KD is the reference's kick-then-drift
@@ -417,10 +417,10 @@ int sd_set_mlp(sd_sim* sim, const float* params_device, float out_scale);
  * density is the same fixed-point sum as when it runs alone (bit-exact). */
 typedef struct sd_ensemble sd_ensemble;
 typedef struct sd_scene_tuning {
-    int order;          /* SD_ORDER_TILED (fused deposit) or SD_ORDER_ROWMAJOR (atomic deposit) */
+    int order;          /* SD_ORDER_TILED or SD_ORDER_ROWMAJOR */
     int gather_blocks;  /* gather grid cap in CTAs (0: one CTA per 256 particles, at most 4096) */
     float step_ms;      /* median step time of the chosen variant alone; -1 before tuning */
-    int deposit_split;  /* window particles per CTA share of the fused deposit (0 with the atomic deposit) */
+    int deposit_split;  /* window particles per CTA share of the fused deposit (0: the default, in row-major order) */
 } sd_scene_tuning;
 int sd_ensemble_create(sd_ensemble** out, int device);
 int sd_ensemble_destroy(sd_ensemble* ens);

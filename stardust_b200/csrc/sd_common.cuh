@@ -22,6 +22,11 @@ __device__ __forceinline__ void cic_axis(float p, int G, int& i, float& f) {
     f = __fsub_rn(g, fl);
 }
 
+// Containing cell along one axis, clamped (kCellKey, Sim.cu:2482-2485).
+__device__ __forceinline__ int cell_axis(float p, int G) {
+    return min(max((int)__fmul_rn(p, (float)G), 0), G - 1);
+}
+
 // Cell index of a CIC corner: wrapped (periodic) or clamped to the edge cell
 // (isolated; gidx3, Sim.cu:96-100 -- weights past the edge land on it).
 __device__ __forceinline__ int cic_cell(int i, int G, bool periodic) {
@@ -42,6 +47,24 @@ __device__ __forceinline__ long long fixed_weight(float w) {
 
 __device__ __forceinline__ float fixed_to_float(long long s) {
     return __fmul_rn(__ll2float_rn(s), SD_FIXED_INV);
+}
+
+// The 8 corners of one particle into an int64 fixed-point grid of side G.
+__device__ __forceinline__ void deposit_particle(float4 p, int G, unsigned long long* __restrict__ acc, bool periodic) {
+    if (p.x < 0.f) return;
+    int ix, iy, iz;
+    float fx, fy, fz;
+    cic_axis(p.x, G, ix, fx);
+    cic_axis(p.y, G, iy, fy);
+    cic_axis(p.z, G, iz, fz);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const int cx = cic_cell(ix + (k & 1), G, periodic);
+        const int cy = cic_cell(iy + ((k >> 1) & 1), G, periodic);
+        const int cz = cic_cell(iz + ((k >> 2) & 1), G, periodic);
+        const long long q = fixed_weight(cic_weight(k, fx, fy, fz));
+        atomicAdd(acc + ((size_t)cz * G + cy) * G + cx, (unsigned long long)q);
+    }
 }
 
 __device__ __forceinline__ uint32_t part1by2(uint32_t v) {
@@ -67,10 +90,7 @@ __device__ __forceinline__ uint32_t order_key(float4 p, int G, int order) {
         const int tile = (iz >> 2) * tiles + (iy >> 2);
         return (uint32_t)(tile * 16 + (iz & 3) * 4 + (iy & 3));
     }
-    // containing cell, clamped (kCellKey, Sim.cu:2482-2485)
-    const int cx = min(max((int)__fmul_rn(p.x, (float)G), 0), G - 1);
-    const int cy = min(max((int)__fmul_rn(p.y, (float)G), 0), G - 1);
-    const int cz = min(max((int)__fmul_rn(p.z, (float)G), 0), G - 1);
+    const int cx = cell_axis(p.x, G), cy = cell_axis(p.y, G), cz = cell_axis(p.z, G);
     if (order == 1)
         return (part1by2((uint32_t)cx) | (part1by2((uint32_t)cy) << 1) | (part1by2((uint32_t)cz) << 2)) + 1u;
     return (uint32_t)((cz * G + cy) * G + cx) + 1u;
@@ -87,6 +107,19 @@ __host__ __device__ __forceinline__ uint32_t row_low(int r, int shift) {
 }
 __host__ __device__ __forceinline__ uint32_t row_of(uint32_t key, int shift) {
     return shift < 0 ? key : (key ? ((key - 1u) >> shift) + 1u : 0u);
+}
+
+// Whether the fused deposit's windows miss a live particle: its stencil's base row is
+// not where its key's row says (only positions outside the box; see k_deposit_plan).
+__device__ __forceinline__ bool stray_row(float p, int G, int order, bool periodic) {
+    int i;
+    float f;
+    cic_axis(p, G, i, f);
+    if (order == 0 && periodic) {
+        const int c = cell_axis(p, G);
+        return i != c && i != c - 1;
+    }
+    return order == 2 && !periodic && (i < -1 || i >= G);
 }
 
 __device__ __forceinline__ unsigned lanemask_lt() {

@@ -22,7 +22,9 @@ long long launches();
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // Stage launchers (defined in the .cu files). All return SD_OK or SD_E_*.
-int launch_cell_keys(const float4* pos, int n, int G, int order, uint32_t* keys, cudaStream_t s);
+// stray (optional): the fused deposit's flag for positions outside the box (deposit_stray_flag)
+int launch_cell_keys(const float4* pos, int n, int G, int order, uint32_t* keys, cudaStream_t s, int* stray = nullptr,
+                     int periodic = 1);
 size_t sort_workspace_bytes(int n);
 int launch_sort_pairs(const uint32_t* keys_in, const int32_t* vals_in, uint32_t* keys_out, int32_t* vals_out,
                       uint32_t* keys_tmp, int32_t* vals_tmp, int n, int key_bits, void* ws, size_t ws_bytes,
@@ -63,7 +65,7 @@ size_t poisson_spectrum_elems(int G);  // complex elements of the (bricked, padd
 // float density. The spectrum buffer is transformed in place.
 int launch_poisson(const PoissonPlan& p, const long long* rho_fixed, const float* rho_float, float* rho_keep,
                    float2* spec, float* phi, cudaStream_t s);
-// pos != nullptr: the first pass deposits the particles itself (SD_ORDER_TILED
+// pos != nullptr: the first pass deposits the particles itself (tiled or row-major
 // order, row_start from launch_row_bounds) instead of reading a density grid.
 // ev (optional): 4 events recorded after passes A, B, C and D.
 // Isolated-boundary options of the Poisson solve (Hockney-Eastwood, kGreen/kMulSpec,
@@ -77,7 +79,9 @@ struct PoissonIso {
     bool forward_only = false;
 };
 // Work plan of the fused deposit (pos != nullptr). A row bundle's CTA reads the
-// particles of the 25 base rows whose stencils reach its 16 rows; a bundle whose
+// particles of the rows whose stencils reach its 16 rows (25 base rows in the tiled
+// order, 36 cell rows in the row-major order, `wide`; row_start then points at the
+// row table's entry 1, the first row); a bundle whose
 // window holds more than `split` particles is shared by several CTAs, which add
 // their exact int64 partial rows into `acc` (the fixed-point grid, zero between
 // uses) and the last of them to finish transforms the rows. `ints` is scratch of
@@ -86,8 +90,11 @@ struct DepositWork {
     long long* acc = nullptr;
     int* ints = nullptr;
     int split = 0;
+    bool wide = false;
+    int n = 0;  // particles
 };
 size_t deposit_work_ints(int G);
+int* deposit_stray_flag(int* ints, int G);
 // the particles per CTA above which a window is split: mult times a window's mean count
 // (mult 0: 10 where the grid has at least 1024 row bundles, 5 below)
 int deposit_split(int n, int G, int mult = 0);

@@ -53,21 +53,7 @@ __global__ void __launch_bounds__(256) k_deposit_fixed(const float4* __restrict_
                                                        unsigned long long* __restrict__ acc, int periodic) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const float4 p = pos[i];
-    if (p.x < 0.f) return;
-    int ix, iy, iz;
-    float fx, fy, fz;
-    cic_axis(p.x, G, ix, fx);
-    cic_axis(p.y, G, iy, fy);
-    cic_axis(p.z, G, iz, fz);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const int cx = cic_cell(ix + (k & 1), G, periodic);
-        const int cy = cic_cell(iy + ((k >> 1) & 1), G, periodic);
-        const int cz = cic_cell(iz + ((k >> 2) & 1), G, periodic);
-        const long long q = fixed_weight(cic_weight(k, fx, fy, fz));
-        atomicAdd(acc + ((size_t)cz * G + cy) * G + cx, (unsigned long long)q);
-    }
+    deposit_particle(pos[i], G, acc, periodic);
 }
 
 __global__ void k_fixed_to_float(long long* __restrict__ acc, size_t cells, float* __restrict__ rho, int clear) {

@@ -319,37 +319,70 @@ __global__ void __launch_bounds__(kFftThreads) k_pass_a(const float* __restrict_
 //   arrive[NB]   CTAs of a shared bundle done so far (zero between uses)
 //   cta_sum[NC], cta_pre[NC + 1]   per-block totals and their exclusive prefix
 //   plan_done    blocks of the plan kernel done (zero between uses)
+//   use          nonzero: this use deposits from the fixed-point grid (see stray)
+//   stray        nonzero: a particle sits where its row's windows do not reach (set where
+//                keys are made, launch_cell_keys; cleared by the next plan)
 template <int G>
 struct DepPlan {
     static constexpr int NB = G * G / 16;
     static constexpr int NC = (NB + 255) / 256;
     static constexpr int kItems = 0, kXpre = NB, kArrive = 2 * NB, kCtaSum = 3 * NB, kCtaPre = 3 * NB + NC,
-                         kDone = 3 * NB + 2 * NC + 1, kInts = kDone + 1;
+                         kDone = 3 * NB + 2 * NC + 1, kUse = kDone + 1, kStray = kUse + 1, kInts = kStray + 1;
 };
 
-// The 25 base rows whose CIC stencils reach the 16 rows of bundle b = bz*(G/4)+by,
-// as 7 ranges of the sorted particles: r = 0 the bundle's own rows (16 consecutive
-// keys); r = 1 the rows z_l = 3 of the bundle below in z (4 consecutive keys);
-// r = 2..5 the rows y_l = 3, z_l = r - 2 of the bundle below in y; r = 6 the row
-// y_l = z_l = 3 of the bundle below in both. Neighbours wrap (periodic box).
-template <int G>
+// Where the particles of a bundle's window sit among the sorted ones, as kRanges
+// ranges. G is the side of the particles' grid, rs its row table.
+//
+// Tiled order: the 25 base rows whose CIC stencils reach the 16 rows of bundle
+// b = bz*(G/4)+by, as 7 ranges: r = 0 the bundle's own rows (16 consecutive keys);
+// r = 1 the rows z_l = 3 of the bundle below in z (4 consecutive keys); r = 2..5 the
+// rows y_l = 3, z_l = r - 2 of the bundle below in y; r = 6 the row y_l = z_l = 3 of
+// the bundle below in both. Neighbours wrap: in a periodic box the stencils do, in an
+// isolated one a base row -1 is stored as row G - 1 (and one that does not reach this
+// bundle adds nothing to it).
+//
+// Row-major order (WIDE): a particle's cell is its base cell or the one above, so the
+// window is the 6 x 6 rows of cells around the bundle: for each plane z = 4 bz - 1 ..
+// 4 bz + 4 the rows y = 4 by - 1 .. 4 by + 4, one range, and a second one for the row
+// that wraps. 36 rows read for 16 against 25, still less than a pass of 64-bit atomics
+// over the grid and another to read and clear it (8,000,003 particles on 256^3: 238 us,
+// now 190 with the plan; 2,000,000 on 128^3: 78 and 73; 1,000,003 of a galaxy on an
+// isolated 128^3: 106 and 78).
+template <bool WIDE>
+constexpr int kRanges = WIDE ? 12 : 7;
+
+template <int G, bool WIDE, bool ISO>
 __device__ __forceinline__ void window_range(int b, int r, const int* __restrict__ rs, int& lo, int& hi) {
     constexpr int TB = G / 4;
     const int by = b & (TB - 1), bz = b / TB;
-    const int bym = (by + TB - 1) & (TB - 1), bzm = (bz + TB - 1) & (TB - 1);
     int k0, k1;
-    if (r == 0) {
-        k0 = 16 * b;
-        k1 = k0 + 16;
-    } else if (r == 1) {
-        k0 = 16 * (bzm * TB + by) + 12;
-        k1 = k0 + 4;
-    } else if (r == 6) {
-        k0 = 16 * (bzm * TB + bym) + 15;
-        k1 = k0 + 1;
+    if (WIDE) {
+        int z = 4 * bz - 1 + (r >> 1);
+        const int y0 = 4 * by - 1, y1 = 4 * by + 4;
+        int ya = max(y0, 0), yb = min(y1, G - 1);
+        bool none = ISO && (unsigned)z >= (unsigned)G;
+        if (r & 1) {
+            none = none || ISO || (y0 >= 0 && y1 < G);
+            ya = yb = (y0 < 0) ? G - 1 : 0;
+        }
+        z &= G - 1;
+        k0 = none ? 0 : z * G + ya;
+        k1 = none ? 0 : z * G + yb + 1;
     } else {
-        k0 = 16 * (bz * TB + bym) + 4 * (r - 2) + 3;
-        k1 = k0 + 1;
+        const int bym = (by + TB - 1) & (TB - 1), bzm = (bz + TB - 1) & (TB - 1);
+        if (r == 0) {
+            k0 = 16 * b;
+            k1 = k0 + 16;
+        } else if (r == 1) {
+            k0 = 16 * (bzm * TB + by) + 12;
+            k1 = k0 + 4;
+        } else if (r == 6) {
+            k0 = 16 * (bzm * TB + bym) + 15;
+            k1 = k0 + 1;
+        } else {
+            k0 = 16 * (bz * TB + bym) + 4 * (r - 2) + 3;
+            k1 = k0 + 1;
+        }
     }
     lo = rs[k0];
     hi = rs[k1];
@@ -386,17 +419,33 @@ __device__ __forceinline__ int block_excl_scan256(int v, int* total) {
 // How many CTAs share each bundle: ceil(window particles / split), at least 1,
 // and where each bundle's extra CTAs start. The last block to finish turns the
 // block totals into their prefix.
-template <int G>
-__global__ void __launch_bounds__(256) k_deposit_plan(const int* __restrict__ rs, int* __restrict__ w, int split) {
+//
+// Positions outside the box are accepted. The periodic stencil wraps them and the
+// isolated one clamps them, but the row that the row-major key (clamped) or the tiled
+// key (wrapped) puts them in is then not the stencil's, so no window finds them. Where
+// keys were made from such a position the stray flag is set, and this kernel deposits
+// every particle into the fixed-point grid itself, which the bundles read instead of
+// particles. Steps leave positions inside the box, so this is at most the first step
+// after a load; its speed does not matter, its not costing the others a launch does.
+template <int G, bool WIDE, bool ISO>
+__global__ void __launch_bounds__(256) k_deposit_plan(const int* __restrict__ rs, int* __restrict__ w, int split,
+                                                      const float4* __restrict__ pos, int n,
+                                                      unsigned long long* __restrict__ acc) {
     using P = DepPlan<G>;
     const int b = blockIdx.x * 256 + threadIdx.x;
     int extra = 0;
+    constexpr bool kMayStray = WIDE != ISO;  // row-major periodic, tiled isolated
+    const int stray = kMayStray ? w[P::kStray] : 0;
+    if (kMayStray && stray) {
+        split = 0x7fffffff;  // no shared bundles
+        for (long long i = b; i < n; i += (long long)gridDim.x * 256) deposit_particle(pos[i], G, acc, !ISO);
+    }
     if (b < P::NB) {
         int total = 0;
 #pragma unroll
-        for (int r = 0; r < 7; ++r) {
+        for (int r = 0; r < kRanges<WIDE>; ++r) {
             int lo, hi;
-            window_range<G>(b, r, rs, lo, hi);
+            window_range<G, WIDE, ISO>(b, r, rs, lo, hi);
             total += hi - lo;
         }
         const int items = total > split ? (int)(((long long)total + split - 1) / split) : 1;
@@ -422,6 +471,10 @@ __global__ void __launch_bounds__(256) k_deposit_plan(const int* __restrict__ rs
     if (threadIdx.x == 0) {
         w[P::kCtaPre + P::NC] = all;
         w[P::kDone] = 0;
+        if (kMayStray) {  // every block has read the flag
+            w[P::kUse] = stray;
+            w[P::kStray] = 0;
+        }
     }
 }
 
@@ -429,35 +482,49 @@ __global__ void __launch_bounds__(256) k_deposit_plan(const int* __restrict__ rs
 // into int64 row sums in shared memory; if the bundle is shared, add the sums into
 // the fixed-point grid and let the last CTA continue with the whole bundle; then
 // convert, transform the 16 rows along x and store the spectrum bricks.
+// ISO: the particles' grid has half the box's side and corners past its edge are
+// clamped onto the edge cells (no weight is lost); the upper half of each line is zero.
 // (Summing equal corners across a warp's lanes first, with __match_any_sync and
 // __reduce_add_sync, made dense scenes slower, not faster: 0.27 against 0.18 ms
 // at 4M particles / 256^3.)
-template <int G, bool SHARED>
+template <int G, bool ISO>
+struct DepGeo {
+    static constexpr int M = ISO ? G / 2 : G;  // side of the particles' grid
+    static constexpr int RS = M + 4;           // words between the rows of the sums
+    // float2 of the storage that the sums, the line buffer and (512) the warps' scratch share
+    static constexpr int kLines = 16 * Geo<G>::PX, kSums = 16 * RS, kWarp = 16 * 256 + xl::kStage;
+    static constexpr int kStore = G == 512 ? (kWarp > kSums ? kWarp : kSums) : (kLines > kSums ? kLines : kSums);
+};
+
+template <int G, bool ISO, bool WIDE, bool SHARED>
 __device__ __forceinline__ void deposit_bundle(int b, int slice, int items, const float4* __restrict__ pos,
                                                const int* __restrict__ perm, const int* __restrict__ row_start,
                                                float* __restrict__ rho_keep, float2* __restrict__ spec,
-                                               const DepositWork& w, unsigned* __restrict__ arrive, bool reuse) {
+                                               const DepositWork& w, unsigned* __restrict__ arrive, bool reuse,
+                                               bool from_grid) {
     using T = Geo<G>;
-    constexpr int H = T::H, NBX = T::NBX, NT = kDepositThreads, TB = G / 4;
+    using D = DepGeo<G, ISO>;
+    constexpr int M = D::M, NR = kRanges<WIDE>;
+    constexpr int H = T::H, NBX = T::NBX, NT = kDepositThreads, TB = M / 4;
     // The int64 fixed-point sums, as two 32-bit words per cell (lo[16][RS], hi[16][RS]),
     // share their storage with the complex line buffer used after the conversion.
-    // Rows are RS = G + 4 words apart, so the row-parallel 16-byte reads of the
+    // Rows are RS = M + 4 words apart, so the row-parallel 16-byte reads of the
     // conversion fall in different banks.
-    constexpr int RS = G + 4;
+    constexpr int RS = D::RS;
     extern __shared__ float2 sm[];
     const float2* tw = sm;
     unsigned* acc_lo = reinterpret_cast<unsigned*>(sm + G);
     unsigned* acc_hi = acc_lo + 16 * RS;
     float2* s = sm + G;
-    __shared__ int r_lo[7], r_off[8];
+    __shared__ int r_lo[16], r_off[17];
     __shared__ int s_last;
     const int by = b & (TB - 1), bz = b / TB;
-    const int m = G - 1;
+    const int m = M - 1;
     const int j = threadIdx.x;
     int lo = 0, len = 0;
-    if (j < 7) {
+    if (j < NR) {
         int hi;
-        window_range<G>(b, j, row_start, lo, hi);
+        window_range<M, WIDE, ISO>(b, j, row_start, lo, hi);
         len = hi - lo;
     }
     if (reuse) __syncthreads();  // the shared buffers of this CTA's previous bundle are free
@@ -465,18 +532,18 @@ __device__ __forceinline__ void deposit_bundle(int b, int slice, int items, cons
     if (threadIdx.x < 32) {
         int inc = len;
 #pragma unroll
-        for (int o = 1; o < 8; o <<= 1) {
+        for (int o = 1; o < (WIDE ? 16 : 8); o <<= 1) {
             const int t = __shfl_up_sync(0xffffffffu, inc, o);
             if (j >= o) inc += t;
         }
-        if (j < 7) {
+        if (j < NR) {
             r_lo[j] = lo;
             r_off[j + 1] = inc;
         }
         if (j == 0) r_off[0] = 0;
     }
     __syncthreads();
-    const int total = r_off[7];
+    const int total = from_grid ? 0 : r_off[NR];  // from_grid: the sums are in the fixed-point grid
     const int f_lo = SHARED ? (int)((long long)total * slice / items) : 0;
     const int f_hi = SHARED ? (int)((long long)total * (slice + 1) / items) : total;
     // A weight q <= 2^32 is added as (q >> 16) into the high word and (q & 0xffff)
@@ -494,9 +561,11 @@ __device__ __forceinline__ void deposit_bundle(int b, int slice, int items, cons
             const int f = base + q * NT + lane;
             src[q] = -1;
             if (f < f_hi) {
-                int r = (r_off[4] <= f) ? 4 : 0;  // largest r < 7 with r_off[r] <= f
-                if (r + 2 < 7 && r_off[r + 2] <= f) r += 2;
-                if (r + 1 < 7 && r_off[r + 1] <= f) r += 1;
+                // largest r < NR with r_off[r] <= f
+                int r = (WIDE && r_off[8] <= f) ? 8 : 0;
+                if (r + 4 < NR && r_off[r + 4] <= f) r += 4;
+                if (r + 2 < NR && r_off[r + 2] <= f) r += 2;
+                if (r + 1 < NR && r_off[r + 1] <= f) r += 1;
                 src[q] = r_lo[r] + (f - r_off[r]);
             }
         }
@@ -515,22 +584,41 @@ __device__ __forceinline__ void deposit_bundle(int b, int slice, int items, cons
             const bool valid = p.x >= 0.f;  // empty slots sort into row 0
             int ix, iy, iz;
             float fx, fy, fz;
-            cic_axis(p.x, G, ix, fx);
-            cic_axis(p.y, G, iy, fy);
-            cic_axis(p.z, G, iz, fz);
+            cic_axis(p.x, M, ix, fx);
+            cic_axis(p.y, M, iy, fy);
+            cic_axis(p.z, M, iz, fz);
             if (!valid) continue;
-            const int x0 = ix & m, x1 = (ix + 1) & m;
+            // the weights of cic_weight, scaled by 2^32 with their z factor (exact)
+            const float wx[2] = {__fsub_rn(1.f, fx), fx}, wy[2] = {__fsub_rn(1.f, fy), fy};
+            const float wz[2] = {__fmul_rn(__fsub_rn(1.f, fz), SD_FIXED_ONE), __fmul_rn(fz, SD_FIXED_ONE)};
+            const int x0 = cic_cell(ix, M, !ISO), x1 = cic_cell(ix + 1, M, !ISO);
+            // the bundle's rows that the stencil reaches: yl + (0, 1), zl + (0, 1), each in
+            // [0, 4) or not this bundle's. In the periodic box they lie at fixed distances
+            // from the first one's address, whether that is in the bundle or not.
+            int yl[2], zl[2];
+            if (ISO) {
+#pragma unroll
+                for (int o = 0; o < 2; ++o) {
+                    yl[o] = cic_cell(iy + o, M, false) - 4 * by;
+                    zl[o] = cic_cell(iz + o, M, false) - 4 * bz;
+                }
+            } else {
+                yl[1] = (iy + 1 - 4 * by) & m;
+                zl[1] = (iz + 1 - 4 * bz) & m;
+                yl[0] = yl[1] - 1;
+                zl[0] = zl[1] - 1;
+            }
+            const int first = (zl[0] * 4 + yl[0]) * RS;
 #pragma unroll
             for (int oyz = 0; oyz < 4; ++oyz) {
-                const int yl = ((iy + (oyz & 1)) & m) - 4 * by;
-                const int zl = ((iz + (oyz >> 1)) & m) - 4 * bz;
-                if ((unsigned)yl >= 4u || (unsigned)zl >= 4u) continue;
-                const int rowc = (zl * 4 + yl) * RS;
+                const int oy = oyz & 1, oz = oyz >> 1;
+                if ((unsigned)yl[oy] >= 4u || (unsigned)zl[oz] >= 4u) continue;
+                const int row = ISO ? (zl[oz] * 4 + yl[oy]) * RS : first + (oz * 4 + oy) * RS;
 #pragma unroll
                 for (int ox = 0; ox < 2; ++ox) {
                     const unsigned long long qv =
-                        (unsigned long long)fixed_weight(cic_weight(ox | (oyz << 1), fx, fy, fz));
-                    const int c = rowc + (ox ? x1 : x0);
+                        (unsigned long long)__float2ll_rn(__fmul_rn(__fmul_rn(wx[ox], wy[oy]), wz[oz]));
+                    const int c = row + (ox ? x1 : x0);
                     if (split16) {
                         atomicAdd(acc_hi + c, (unsigned)(qv >> 16));
                         atomicAdd(acc_lo + c, (unsigned)(qv & 0xffffu));
@@ -548,41 +636,43 @@ __device__ __forceinline__ void deposit_bundle(int b, int slice, int items, cons
     }
     __syncthreads();
     int sh = split16 ? 16 : 32;  // value of a cell: (hi << sh) + lo
-    if (SHARED && items > 1) {
+    if (SHARED && (items > 1 || from_grid)) {
         // a shared bundle: every CTA adds its rows into the fixed-point grid; the last
         // to arrive reads the complete sums back (and leaves the grid zero)
         unsigned long long* g = reinterpret_cast<unsigned long long*>(w.acc);
+        if (!from_grid) {
 #pragma unroll 1
-        for (int u = threadIdx.x; u < 16 * G; u += NT) {
-            const int l = u / G, x = u & m;
-            const unsigned long long v =
-                ((unsigned long long)acc_hi[l * RS + x] << sh) + (unsigned long long)acc_lo[l * RS + x];
-            if (v) atomicAdd(g + ((size_t)(4 * bz + (l >> 2)) * G + 4 * by + (l & 3)) * G + x, v);
+            for (int u = threadIdx.x; u < 16 * M; u += NT) {
+                const int l = u / M, x = u & m;
+                const unsigned long long v =
+                    ((unsigned long long)acc_hi[l * RS + x] << sh) + (unsigned long long)acc_lo[l * RS + x];
+                if (v) atomicAdd(g + ((size_t)(4 * bz + (l >> 2)) * M + 4 * by + (l & 3)) * M + x, v);
+            }
+            __threadfence();
+            __syncthreads();
+            if (threadIdx.x == 0) s_last = atomicAdd(arrive + b, 1u) == (unsigned)(items - 1);
+            __syncthreads();
+            if (!s_last) return;
+            __threadfence();
         }
-        __threadfence();
-        __syncthreads();
-        if (threadIdx.x == 0) s_last = atomicAdd(arrive + b, 1u) == (unsigned)(items - 1);
-        __syncthreads();
-        if (!s_last) return;
-        __threadfence();
         // all of this thread's loads first, then the shared-memory writes and the zeroing
         // stores (a store behind each load of the same address would serialise them)
         constexpr int RB = 4;  // loads in flight per thread (more spill at the 40-register bound)
 #pragma unroll 1
-        for (int u0 = threadIdx.x; u0 < 16 * G; u0 += RB * NT) {
+        for (int u0 = threadIdx.x; u0 < 16 * M; u0 += RB * NT) {
             unsigned long long rb[RB];
 #pragma unroll
             for (int q = 0; q < RB; ++q) {
-                const int u = u0 + q * NT, l = u / G, x = u & m;
-                if (u < 16 * G) rb[q] = __ldcg(g + ((size_t)(4 * bz + (l >> 2)) * G + 4 * by + (l & 3)) * G + x);
+                const int u = u0 + q * NT, l = u / M, x = u & m;
+                if (u < 16 * M) rb[q] = __ldcg(g + ((size_t)(4 * bz + (l >> 2)) * M + 4 * by + (l & 3)) * M + x);
             }
 #pragma unroll
             for (int q = 0; q < RB; ++q) {
-                const int u = u0 + q * NT, l = u / G, x = u & m;
-                if (u < 16 * G) {
+                const int u = u0 + q * NT, l = u / M, x = u & m;
+                if (u < 16 * M) {
                     acc_lo[l * RS + x] = (unsigned)rb[q];
                     acc_hi[l * RS + x] = (unsigned)(rb[q] >> 32);
-                    g[((size_t)(4 * bz + (l >> 2)) * G + 4 * by + (l & 3)) * G + x] = 0ull;
+                    g[((size_t)(4 * bz + (l >> 2)) * M + 4 * by + (l & 3)) * M + x] = 0ull;
                 }
             }
         }
@@ -597,11 +687,15 @@ __device__ __forceinline__ void deposit_bundle(int b, int slice, int items, cons
         const int l = threadIdx.x >> 5, lane = threadIdx.x & 31;
         const unsigned* lo = acc_lo + l * RS;
         const unsigned* hi = acc_hi + l * RS;
-        const size_t grow = ((size_t)(bz * 4 + (l >> 2)) * G + by * 4 + (l & 3)) * G;
+        const size_t grow = ((size_t)(bz * 4 + (l >> 2)) * M + by * 4 + (l & 3)) * M;
         float2 v[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const int m = lane + 32 * k;
+            if (ISO && k >= 4) {
+                v[k] = make_float2(0.f, 0.f);
+                continue;
+            }
             const uint2 lw = *reinterpret_cast<const uint2*>(lo + 2 * m);
             const uint2 hw = *reinterpret_cast<const uint2*>(hi + 2 * m);
             v[k] = make_float2(fixed_to_float((long long)(((unsigned long long)hw.x << sh) + lw.x)),
@@ -609,18 +703,17 @@ __device__ __forceinline__ void deposit_bundle(int b, int slice, int items, cons
             if (rho_keep) *reinterpret_cast<float2*>(rho_keep + grow + 2 * m) = v[k];
         }
         // every row is in registers: the sums' storage becomes 16 warp scratches
-        // (256 float2 each) and the brick staging (16 * 256 + kStage = 16 * RS float2)
-        static_assert(16 * 256 + xl::kStage == 16 * RS, "scratch and staging fill the sums");
+        // (256 float2 each) and the brick staging
         __syncthreads();
         float2* R = reinterpret_cast<float2*>(acc_lo);
-        xl::r2c512(v, R + l * 256, tw, sm + G + 16 * RS, R + 16 * 256, l);
+        xl::r2c512(v, R + l * 256, tw, sm + G + D::kStore, R + 16 * 256, l);
         __syncthreads();
         xl::store_bricks<G>(R + 16 * 256, spec, by, bz);
         return;
     }
     // int64 rows -> complex positions z[m] = x[2m] + i x[2m+1] on line l = z_l*4 + y_l,
     // staged through registers because the line buffer overlays the sums.
-    constexpr int CITEMS = 16 * (H / 2);
+    constexpr int CITEMS = 16 * (M / 4);
     constexpr int CPER = (CITEMS + NT - 1) / NT;
     float4 cv[CPER];
 #pragma unroll
@@ -643,7 +736,7 @@ __device__ __forceinline__ void deposit_bundle(int b, int slice, int items, cons
         if (CITEMS % NT == 0 || u < CITEMS) {
             const int l = u & 15, mp = u >> 4;
             if (rho_keep) {
-                const size_t grow = ((size_t)(bz * 4 + (l >> 2)) * G + by * 4 + (l & 3)) * G;
+                const size_t grow = ((size_t)(bz * 4 + (l >> 2)) * M + by * 4 + (l & 3)) * M;
                 *reinterpret_cast<float4*>(rho_keep + grow + 4 * mp) = cv[p];
             }
             s[(2 * mp) * 16 + l] = make_float2(cv[p].x, cv[p].y);
@@ -651,7 +744,7 @@ __device__ __forceinline__ void deposit_bundle(int b, int slice, int items, cons
         }
     }
     __syncthreads();
-    fft::lines16<H, NT, 2, false>(s, tw);
+    fft::lines16<H, NT, 2, false, ISO>(s, tw);
     constexpr int PAIRS = 16 * (H / 2 + 1);
     for (int u = threadIdx.x; u < PAIRS; u += NT) {
         const int l = u & 15, k = u >> 4;
@@ -686,23 +779,24 @@ __device__ __forceinline__ void deposit_bundle(int b, int slice, int items, cons
 // Grid: X CTAs that take the extra shares of heavy bundles (first, so they start
 // early), then one CTA per bundle for its first share. 40 registers at G = 512
 // keep three 70 KB CTAs per SM; smaller grids need more for their FFT stages.
-template <int G>
+template <int G, bool ISO, bool WIDE>
 __global__ void __launch_bounds__(kDepositThreads, G >= 128 ? 3 : 2)
     k_pass_a_deposit_bal(const float4* __restrict__ pos, const int* __restrict__ perm,
                          const int* __restrict__ row_start, float* __restrict__ rho_keep, float2* __restrict__ spec,
                          const float2* __restrict__ tw_g, DepositWork w) {
-    using P = DepPlan<G>;
+    using P = DepPlan<DepGeo<G, ISO>::M>;
     extern __shared__ float2 sm[];
     const int* items = w.ints + P::kItems;
     const int* xpre = w.ints + P::kXpre;
     const int* cta_pre = w.ints + P::kCtaPre;
     unsigned* arrive = reinterpret_cast<unsigned*>(w.ints + P::kArrive);
     const int X = (int)gridDim.x - P::NB;
+    const bool from_grid = WIDE != ISO && w.ints[P::kUse] != 0;
     const bool first = (int)blockIdx.x >= X;  // a bundle's first share, then done
     const int extras = first ? 0 : cta_pre[P::NC];
     if (!first && (int)blockIdx.x >= extras) return;  // no extra share for this CTA
     for (int i = threadIdx.x; i < G; i += kDepositThreads) sm[i] = tw_g[i];  // ordered by a later barrier
-    if constexpr (G == 512) xl::fill_twiddles(sm + G + 16 * (G + 4), tw_g);  // the twiddle tables, after the sums
+    if constexpr (G == 512) xl::fill_twiddles(sm + G + DepGeo<G, ISO>::kStore, tw_g);  // the twiddle tables, after the sums
     for (int e = first ? 0 : (int)blockIdx.x; first || e < extras; e += X) {
         int b, slice;
         if (first) {
@@ -724,12 +818,12 @@ __global__ void __launch_bounds__(kDepositThreads, G >= 128 ? 3 : 2)
         // it does not (0.513 against 0.479 ms at 16M / 512^3)
         // (at 512^3; smaller grids, whose registers the two copies would spill, keep one)
         const int nb = items[b];
-        if (G >= 512 && nb == 1)
-            deposit_bundle<G, false>(b, 0, 1, pos, perm, row_start, rho_keep, spec, w, arrive,
-                                     !first && e != (int)blockIdx.x);
+        if (G >= 512 && nb == 1 && !from_grid)
+            deposit_bundle<G, ISO, WIDE, false>(b, 0, 1, pos, perm, row_start, rho_keep, spec, w, arrive,
+                                                !first && e != (int)blockIdx.x, false);
         else
-            deposit_bundle<G, true>(b, slice, nb, pos, perm, row_start, rho_keep, spec, w, arrive,
-                                    !first && e != (int)blockIdx.x);
+            deposit_bundle<G, ISO, WIDE, true>(b, slice, nb, pos, perm, row_start, rho_keep, spec, w, arrive,
+                                               !first && e != (int)blockIdx.x, from_grid);
         if (first) break;
     }
 }
@@ -972,18 +1066,30 @@ struct Launcher {
     static size_t smem_c() { return sizeof(float2) * ((size_t)G + (T::H + 2) / 2 + 1 + 16 * (size_t)G); }
     // and the table's values; the lines before them end on a 16-byte boundary
     static size_t smem_ct() { return smem_c() + sizeof(float) * 16 * (size_t)(T::H + 2); }
-    // the line buffer (16 * PX float2) overlays the 32-bit sum words (2 * 16 * (G + 4));
-    // at G = 512 the warp-per-line transform's twiddle tables follow the sums
+    // the line buffer overlays the 32-bit sum words (DepGeo); at G = 512 the warp-per-line
+    // transform's twiddle tables follow
+    template <bool ISO>
     static size_t smem_bal() {
-        const size_t lines = sizeof(float2) * 16 * (size_t)T::PX, sums = 2 * sizeof(unsigned) * 16 * (size_t)(G + 4);
-        const size_t xtab = G == 512 ? sizeof(float2) * xl::kTw2 : 0;
-        static_assert(G != 512 || 16 * (G + 4) >= 16 * T::PX, "the sums are the larger overlay");
-        return sizeof(float2) * (size_t)G + (lines > sums ? lines : sums) + xtab;
+        return sizeof(float2) * ((size_t)G + DepGeo<G, ISO>::kStore + (G == 512 ? xl::kTw2 : 0));
     }
     // CTAs that take the extra shares of heavy bundles
+    template <bool ISO>
     static int extra_ctas() {
-        const int nb = DepPlan<G>::NB / 4;
+        const int nb = DepPlan<DepGeo<G, ISO>::M>::NB / 4;
         return nb < 8 ? 8 : (nb > 296 ? 296 : nb);
+    }
+
+    template <bool ISO, bool WIDE>
+    static int deposit(const PoissonPlan& p, const float4* pos, const int* perm, const int* row_start, float* keep,
+                       float2* spec, const DepositWork& dw, cudaStream_t s) {
+        using P = DepPlan<DepGeo<G, ISO>::M>;
+        k_deposit_plan<DepGeo<G, ISO>::M, WIDE, ISO><<<P::NC, 256, 0, s>>>(
+            row_start, dw.ints, dw.split, pos, dw.n, reinterpret_cast<unsigned long long*>(dw.acc));
+        SD_LAUNCHED(s);
+        k_pass_a_deposit_bal<G, ISO, WIDE><<<extra_ctas<ISO>() + P::NB, kDepositThreads, smem_bal<ISO>(), s>>>(
+            pos, perm, row_start, keep, spec, p.tw, dw);
+        SD_LAUNCHED(s);
+        return SD_OK;
     }
 
     static constexpr bool kIsoBox = G >= 32;  // the transform box of an isolated grid of side G / 2 >= 16
@@ -1003,12 +1109,15 @@ struct Launcher {
         set(k_pass_c<G, 0, false>, smem_c());
         set(k_pass_c<G, 1, false>, smem_c());
         set(k_pass_e<G, false>, smem_ae());
-        set(k_pass_a_deposit_bal<G>, smem_bal());
+        set(k_pass_a_deposit_bal<G, false, false>, smem_bal<false>());
+        set(k_pass_a_deposit_bal<G, false, true>, smem_bal<false>());
         if constexpr (kIsoBox) {
             set(k_pass_y<G, false, true>, smem_bd());
             set(k_pass_y<G, true, true>, smem_bd());
             set(k_pass_c<G, 2, true>, smem_ct());
             set(k_pass_e<G, true>, smem_ae());
+            set(k_pass_a_deposit_bal<G, true, false>, smem_bal<true>());
+            set(k_pass_a_deposit_bal<G, true, true>, smem_bal<true>());
         }
         return rc == SD_OK ? SD_OK : SD_E_CUDA;
     }
@@ -1029,16 +1138,24 @@ struct Launcher {
         const dim3 grid_rows(hy, hz), grid_y(T::NBX, hz), grid_z(T::NBX, T::NBY);
         if (pos) {
             if (!dw || !dw->acc || !dw->ints || dw->split <= 0) return fail(SD_E_ARG, "fused deposit: no work plan");
-            k_deposit_plan<G><<<DepPlan<G>::NC, 256, 0, s>>>(row_start, dw->ints, dw->split);
+            int rc = SD_OK;
+            if constexpr (kIsoBox) {
+                if (half)
+                    rc = dw->wide ? deposit<true, true>(p, pos, perm, row_start, keep, spec, *dw, s)
+                                  : deposit<true, false>(p, pos, perm, row_start, keep, spec, *dw, s);
+            }
+            if (!half)
+                rc = dw->wide ? deposit<false, true>(p, pos, perm, row_start, keep, spec, *dw, s)
+                              : deposit<false, false>(p, pos, perm, row_start, keep, spec, *dw, s);
+            if (rc) return rc;
+        } else {
+            if (acc)
+                k_pass_a<G, 1><<<grid_rows, kFftThreads, smem_a(), s>>>(nullptr, const_cast<long long*>(acc), keep,
+                                                                         spec, p.tw, src_g);
+            else
+                k_pass_a<G, 0><<<grid_rows, kFftThreads, smem_a(), s>>>(rho, nullptr, keep, spec, p.tw, src_g);
             SD_LAUNCHED(s);
-            k_pass_a_deposit_bal<G><<<extra_ctas() + DepPlan<G>::NB, kDepositThreads, smem_bal(), s>>>(
-                pos, perm, row_start, keep, spec, p.tw, *dw);
-        } else if (acc)
-            k_pass_a<G, 1><<<grid_rows, kFftThreads, smem_a(), s>>>(nullptr, const_cast<long long*>(acc), keep, spec,
-                                                                     p.tw, src_g);
-        else
-            k_pass_a<G, 0><<<grid_rows, kFftThreads, smem_a(), s>>>(rho, nullptr, keep, spec, p.tw, src_g);
-        SD_LAUNCHED(s);
+        }
         if (ev) cudaEventRecord(ev[0], s);
         if constexpr (kIsoBox) {
             if (half) {
@@ -1117,6 +1234,8 @@ size_t deposit_work_ints(int G) {
         default: return 0;
     }
 }
+
+int* deposit_stray_flag(int* ints, int G) { return ints + deposit_work_ints(G) - 1; }
 
 int deposit_split(int n, int G, int mult) {
     // by default ten times a window's mean particle count (a window spans 25 rows for a

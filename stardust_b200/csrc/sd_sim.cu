@@ -459,7 +459,9 @@ int mlp_correction(sd_sim* s, const int32_t* perm) {
 int ensure_sort_inputs(sd_sim* s) {
     int rc = SD_OK;
     if (!s->keys_valid) {
-        if ((rc = launch_cell_keys(s->pos, s->N, s->G, s->cfg.order, s->keys, s->stream))) return rc;
+        if ((rc = launch_cell_keys(s->pos, s->N, s->G, s->cfg.order, s->keys, s->stream,
+                                   deposit_stray_flag(s->dep_ints, s->G), isolated(s) ? 0 : 1)))
+            return rc;
         s->keys_valid = true;
         s->counts_valid = s->incr_ready = false;
     }
@@ -551,11 +553,10 @@ int do_step(sd_sim* s, float dt, bool sort, bool timed) {
     }
     if (timed) cudaEventRecord(s->ev[1], s->stream);
     const bool keep = keeps_rho(s);
-    // Tiled order right after a sort: the first FFT pass deposits the particles
-    // itself from the row table. Otherwise: int64 atomics (any particle order).
-    // (The isolated boundary always takes the atomic deposit, which clamps corners
-    // onto the edge cells.)
-    const bool fused = sort && s->cfg.order == SD_ORDER_TILED && !isolated(s);
+    // Right after a sort in the tiled or row-major order the first FFT pass deposits the
+    // particles itself from the row table. Otherwise: int64 atomics (any particle order).
+    const bool wide = s->cfg.order == SD_ORDER_ROWMAJOR;
+    const bool fused = sort && (s->cfg.order == SD_ORDER_TILED || wide);
     // the row table of the sorted keys, for the fused deposit and the next step's merge
     if (!merged && (fused || incr_next) &&
         (rc = launch_row_bounds(s->keys2, s->N, row_last(s->G, s->cfg.order), row_shift(s->G, s->cfg.order),
@@ -569,8 +570,10 @@ int do_step(sd_sim* s, float dt, bool sort, bool timed) {
     dw.acc = s->acc;
     dw.ints = s->dep_ints;
     dw.split = s->dep_split > 0 ? s->dep_split : deposit_split(s->N, s->G);
+    dw.wide = wide;
+    dw.n = s->N;
     if ((rc = launch_poisson_ex(s->plan, fused ? nullptr : s->acc, nullptr, fused ? s->pos : nullptr, perm,
-                                s->row_start, keep ? s->rho : nullptr, s->spec, s->phi, s->stream,
+                                s->row_start + (wide ? 1 : 0), keep ? s->rho : nullptr, s->spec, s->phi, s->stream,
                                 timed ? s->pev : nullptr, iso_opts(s, io), &dw)))
         return sim_error(s, rc);
     if (keep) s->rho_valid = true;

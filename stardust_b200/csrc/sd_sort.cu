@@ -47,11 +47,16 @@ constexpr int kColChunk = 1 << kSortChunkShift;  // tiles per column-scan chunk
 constexpr int kColThreads = 256;
 constexpr int kColSegs = kColThreads / 32;  // 8 segments of a column per CTA
 
+// stray (optional): set where a particle's key does not lead the fused deposit to its
+// stencil (positions outside the box).
 __global__ void __launch_bounds__(256) k_cell_keys(const float4* __restrict__ pos, int n, int G, int order,
-                                                   uint32_t* __restrict__ keys) {
+                                                   uint32_t* __restrict__ keys, int* __restrict__ stray,
+                                                   int periodic) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    keys[i] = order_key(pos[i], G, order);
+    const float4 p = pos[i];
+    keys[i] = order_key(p, G, order);
+    if (stray && p.x >= 0.f && (stray_row(p.y, G, order, periodic) || stray_row(p.z, G, order, periodic))) *stray = 1;
 }
 
 // Inclusive warp scan.
@@ -518,9 +523,10 @@ int launch_row_bounds(const uint32_t* keys, int n, int rows, int shift, int* row
     return SD_OK;
 }
 
-int launch_cell_keys(const float4* pos, int n, int G, int order, uint32_t* keys, cudaStream_t s) {
+int launch_cell_keys(const float4* pos, int n, int G, int order, uint32_t* keys, cudaStream_t s, int* stray,
+                     int periodic) {
     if (n <= 0) return SD_OK;
-    k_cell_keys<<<(n + 255) / 256, 256, 0, s>>>(pos, n, G, order, keys);
+    k_cell_keys<<<(n + 255) / 256, 256, 0, s>>>(pos, n, G, order, keys, stray, periodic);
     SD_LAUNCHED(s);
     return SD_OK;
 }
