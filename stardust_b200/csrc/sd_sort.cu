@@ -11,13 +11,15 @@
 //      row; every later pass gets its counts from the scatter before it, which
 //      knows where each key lands and adds one count per (tile, digit) run of a
 //      warp into a zeroed buffer, so the keys are not read an extra time;
-//   2. a column scan over tiles (chunk sums, a per-digit scan of the chunk sums
-//      plus the digit bases, a rescan of each chunk) turns the rows into, for
-//      every (tile, digit), the global output offset: all keys of smaller digits
-//      plus the same digit's keys in earlier tiles, which is what makes the
-//      result stable across tiles. Counts from k_digit_counts or added by a
-//      scatter bring their chunk sums with them; counts added by the gather that
-//      wrote the keys have their chunks summed;
+//   2. a column scan over tiles gives, for every (tile, digit), the global output
+//      offset: all keys of smaller digits plus the same digit's keys in earlier
+//      tiles, which is what makes the result stable across tiles. Up to
+//      kScanTiles tiles one kernel scans each digit's column and the scatter adds
+//      the smaller digits' totals; above, the columns are cut into chunks (chunk
+//      sums, a per-digit scan of the chunk sums plus the digit bases, a rescan of
+//      each chunk). Counts from k_digit_counts or added by a scatter bring their
+//      chunk sums with them; counts added by the gather that wrote the keys have
+//      their chunks summed;
 //   3. k_digit_scatter: each tile ranks its keys stably (per warp, in input order,
 //      with __match_any_sync on the digit), stages them digit-sorted in shared
 //      memory and writes each digit run contiguously; it then clears its row of
@@ -59,34 +61,25 @@ __global__ void __launch_bounds__(256) k_cell_keys(const float4* __restrict__ po
     if (stray && p.x >= 0.f && (stray_row(p.y, G, order, periodic) || stray_row(p.z, G, order, periodic))) *stray = 1;
 }
 
-// Inclusive warp scan.
-__device__ __forceinline__ unsigned warp_inclusive(unsigned v) {
-    const int lane = threadIdx.x & 31;
+// Exclusive scan across a 256-thread block (of two 32-bit sums packed in 64 bits, or
+// of one); warp_sums: a scratch value per warp.
+template <class T>
+__device__ __forceinline__ T block_exclusive(T v, T* warp_sums) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    T inc = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const unsigned t = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v += t;
+        const T t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
     }
-    return v;
-}
-
-// Exclusive scan across a 256-thread block; *total receives the block sum.
-__device__ __forceinline__ unsigned block_exclusive(unsigned v, unsigned* warp_sums, unsigned* total) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const unsigned inc = warp_inclusive(v);
     if (lane == 31) warp_sums[w] = inc;
     __syncthreads();
-    if (w == 0) {
-        const unsigned s = (lane < (int)(blockDim.x >> 5)) ? warp_sums[lane] : 0u;
-        const unsigned si = warp_inclusive(s);
-        if (lane < (int)(blockDim.x >> 5)) warp_sums[lane] = si - s;
-        if (lane == 31) warp_sums[32] = si;
-    }
+    T before = 0;
+#pragma unroll
+    for (int q = 0; q < kWarps - 1; ++q)
+        if (q < w) before += warp_sums[q];
     __syncthreads();
-    const unsigned r = warp_sums[w] + inc - v;
-    if (total) *total = warp_sums[32];
-    __syncthreads();
-    return r;
+    return before + inc - v;
 }
 
 template <int BITS>
@@ -138,18 +131,21 @@ struct ScatterSmem {
     unsigned short warp_cnt[kWarps][1 << BITS];
     unsigned local_start[1 << BITS];
     unsigned dst_base[1 << BITS];  // global start of the digit's run minus its local start
-    unsigned scan_tmp[33];
+    unsigned long long scan_tmp[kWarps];
     uint32_t skeys[kSortTile];
     int32_t svals[kSortTile];
 };
 
-// One tile of k_digit_scatter (n keys in all).
+// One tile of k_digit_scatter (n keys in all). With `totals` the offsets count the same
+// digit's keys in earlier tiles only, and the smaller digits' keys come from the totals
+// of all digits, scanned here beside the tile's own digit counts.
 template <int BITS>
 __device__ __forceinline__ void scatter_tile(ScatterSmem<BITS>& sm, int tile, const uint32_t* __restrict__ keys_in,
                                              const int32_t* __restrict__ vals_in, uint32_t* __restrict__ keys_out,
                                              int32_t* __restrict__ vals_out, int n, int shift,
-                                             unsigned* __restrict__ offsets, unsigned* __restrict__ next_counts,
-                                             unsigned* __restrict__ next_sums, int next_shift) {
+                                             unsigned* __restrict__ offsets, const unsigned* __restrict__ totals,
+                                             unsigned* __restrict__ next_counts, unsigned* __restrict__ next_sums,
+                                             int next_shift) {
     constexpr int kRadix = 1 << BITS;
     constexpr unsigned mask = kRadix - 1;
     constexpr int DPT = (kRadix + kSortThreads - 1) / kSortThreads;  // digits per thread
@@ -217,16 +213,25 @@ __device__ __forceinline__ void scatter_tile(ScatterSmem<BITS>& sm, int tile, co
     }
     __syncthreads();
     {
-        unsigned tot;
-        unsigned ex = block_exclusive(tsum, sm.scan_tmp, &tot);
+        unsigned all[DPT], asum = 0u;
+#pragma unroll
+        for (int j = 0; j < DPT; ++j) {
+            const int d = threadIdx.x * DPT + j;
+            all[j] = (totals && d < kRadix) ? totals[d] : 0u;
+            asum += all[j];
+        }
+        const unsigned long long ex2 =
+            block_exclusive<unsigned long long>(((unsigned long long)asum << 32) | tsum, sm.scan_tmp);
+        unsigned ex = (unsigned)ex2, base = (unsigned)(ex2 >> 32);
 #pragma unroll
         for (int j = 0; j < DPT; ++j) {
             const int d = threadIdx.x * DPT + j;
             if (d < kRadix) {
                 local_start[d] = ex;
-                dst_base[d] = offsets[(size_t)tile * kRadix + d] - ex;
+                dst_base[d] = base + offsets[(size_t)tile * kRadix + d] - ex;
             }
             ex += dtot[j];
+            base += all[j];
         }
     }
     __syncthreads();
@@ -266,7 +271,7 @@ __device__ __forceinline__ void scatter_tile(ScatterSmem<BITS>& sm, int tile, co
             if (pair != 0xffffffffu && (peers & lt) == 0u) {
                 const unsigned c = (unsigned)__popc(peers), t = pair >> BITS, d = pair & mask;
                 atomicAdd(next_counts + (size_t)t * kRadix + d, c);
-                atomicAdd(next_sums + (size_t)(t >> kSortChunkShift) * kRadix + d, c);
+                if (next_sums) atomicAdd(next_sums + (size_t)(t >> kSortChunkShift) * kRadix + d, c);
             }
         }
     }
@@ -280,25 +285,77 @@ __global__ void __launch_bounds__(kSortThreads) k_digit_scatter(const uint32_t* 
                                                                 uint32_t* __restrict__ keys_out,
                                                                 int32_t* __restrict__ vals_out, int n, int shift,
                                                                 unsigned* __restrict__ offsets,
+                                                                const unsigned* __restrict__ totals,
                                                                 unsigned* __restrict__ next_counts,
                                                                 unsigned* __restrict__ next_sums, int next_shift,
                                                                 const int* __restrict__ n_dev) {
     __shared__ ScatterSmem<BITS> sm;
     if (!LOOP) {
-        scatter_tile<BITS>(sm, blockIdx.x, keys_in, vals_in, keys_out, vals_out, n, shift, offsets, next_counts,
-                           next_sums, next_shift);
+        scatter_tile<BITS>(sm, blockIdx.x, keys_in, vals_in, keys_out, vals_out, n, shift, offsets, totals,
+                           next_counts, next_sums, next_shift);
         return;
     }
     n = *n_dev;  // a count made on the device; the grid covers at most the capacity
     const int ntiles = (n + kSortTile - 1) / kSortTile;
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        scatter_tile<BITS>(sm, tile, keys_in, vals_in, keys_out, vals_out, n, shift, offsets, next_counts, next_sums,
-                           next_shift);
+        scatter_tile<BITS>(sm, tile, keys_in, vals_in, keys_out, vals_out, n, shift, offsets, totals, next_counts,
+                           next_sums, next_shift);
         __syncthreads();  // the tile's shared memory is read to the end before the next one
     }
 }
 
-// Exclusive offsets of the tile-major digit counts counts[tile][digit]:
+// Exclusive scan down each digit's column of the tile-major counts[tile][digit]:
+//   counts[t][d] -> sum_{t' < t} counts[t'][d],  T[d] = the column's total.
+// CTA per 32 digits, so every access is a 128-byte row piece; warp s takes a run of up
+// to kScanRows rows into registers, the warps' sums are scanned transposed (warp w the
+// column w), and the run is written back. More than 32 kScanRows tiles go round with a
+// carry. One launch in place of three (or two) of chunk sums, their scan and a rescan:
+// 262,144 keys of 12 bits, two passes: 16.5 -> 6.1 us; 2,000,000 of 22 bits, three
+// passes: 28 -> 19 us.
+constexpr int kScanThreads = 1024;
+constexpr int kScanRows = 16;
+constexpr int kScanTiles = 2048;  // above (4M keys) the chunked scan's many CTAs are faster
+__global__ void __launch_bounds__(kScanThreads) k_col_scan(unsigned* __restrict__ counts, int tiles, int radix,
+                                                           unsigned* __restrict__ T, const int* __restrict__ n_dev) {
+    __shared__ unsigned pre[32][33];
+    __shared__ unsigned total[32];
+    if (n_dev) tiles = (*n_dev + kSortTile - 1) / kSortTile;
+    const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
+    unsigned* col = counts + blockIdx.x * 32 + lane;  // the radix is a multiple of 32
+    unsigned carry = 0u;
+    for (int t0 = 0; t0 < tiles; t0 += 32 * kScanRows) {
+        const int rows = min(tiles - t0, 32 * kScanRows), per = (rows + 31) / 32;
+        const int r0 = t0 + seg * per, cnt = min(per, t0 + rows - r0);  // cnt may be negative
+        unsigned v[kScanRows], sum = 0u;
+#pragma unroll
+        for (int j = 0; j < kScanRows; ++j) v[j] = j < cnt ? col[(size_t)(r0 + j) * radix] : 0u;
+#pragma unroll
+        for (int j = 0; j < kScanRows; ++j) sum += v[j];
+        pre[seg][lane] = sum;
+        __syncthreads();
+        unsigned inc = pre[lane][seg];  // run `lane` of column `seg`
+        const unsigned mine = inc;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
+        }
+        pre[lane][seg] = inc - mine;
+        if (lane == 31) total[seg] = inc;
+        __syncthreads();
+        unsigned run = carry + pre[seg][lane];
+#pragma unroll
+        for (int j = 0; j < kScanRows; ++j) {
+            if (j < cnt) col[(size_t)(r0 + j) * radix] = run;
+            run += v[j];
+        }
+        carry += total[lane];
+        __syncthreads();  // pre and total are read before the next round writes them
+    }
+    if (seg == 0) T[blockIdx.x * 32 + lane] = carry;
+}
+
+// The chunked scan:
 //   offset(t, d) = base(d) + sum_{t' < t} counts[t'][d],  base(d) = sum_{d' < d} total(d'),
 // over chunks of kColChunk tiles and slabs of 32 digits, so every global access
 // is a coalesced 128-byte row piece and every chain of dependent adds is short:
@@ -307,35 +364,24 @@ __global__ void __launch_bounds__(kSortThreads) k_digit_scatter(const uint32_t* 
 //                the last CTA to finish turns T into the digit bases base(d)
 //   k_col_apply  counts[t][d] -> base(d) + S[c][d] + prefix within the chunk,
 //                and clears S, ready for the adds of the next counts
-
-// Tiles holding n keys (n from the device when n_dev is set: the grids cover the capacity).
-__device__ __forceinline__ int tiles_of(int tiles, const int* n_dev) {
-    return n_dev ? (*n_dev + kSortTile - 1) / kSortTile : tiles;
-}
-
 __global__ void __launch_bounds__(kColThreads) k_col_sums(const unsigned* __restrict__ counts, int tiles, int radix,
-                                                          unsigned* __restrict__ S, const int* __restrict__ n_dev) {
+                                                          unsigned* __restrict__ S) {
     const int d = blockIdx.y * kColThreads + threadIdx.x;
-    tiles = tiles_of(tiles, n_dev);
     if (d >= radix) return;
-    for (int c = blockIdx.x; c * kColChunk < tiles; c += gridDim.x) {
-        const int t0 = c * kColChunk, t1 = min(tiles, t0 + kColChunk);
-        unsigned s = 0u;
+    const int c = blockIdx.x, t0 = c * kColChunk, t1 = min(tiles, t0 + kColChunk);
+    unsigned s = 0u;
 #pragma unroll 8
-        for (int t = t0; t < t1; ++t) s += counts[(size_t)t * radix + d];
-        S[(size_t)c * radix + d] = s;
-    }
+    for (int t = t0; t < t1; ++t) s += counts[(size_t)t * radix + d];
+    S[(size_t)c * radix + d] = s;
 }
 
 // CTA per 32-digit slab: thread (seg, lane) owns digit slab*32 + lane and a
 // contiguous run of chunks; two sweeps (sum, rewrite) around a scan of the runs.
 __global__ void __launch_bounds__(kColThreads) k_col_prefix(unsigned* __restrict__ S, int chunks, int radix,
-                                                            unsigned* __restrict__ T, unsigned* __restrict__ done,
-                                                            const int* __restrict__ n_dev) {
+                                                            unsigned* __restrict__ T, unsigned* __restrict__ done) {
     __shared__ unsigned seg_sum[kColSegs][32];
-    __shared__ unsigned scan_tmp[33];
+    __shared__ unsigned scan_tmp[kWarps];
     __shared__ bool last;
-    if (n_dev) chunks = (tiles_of(0, n_dev) + kColChunk - 1) / kColChunk;
     const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
     const int d = blockIdx.x * 32 + lane;
     const int per = (chunks + kColSegs - 1) / kColSegs;
@@ -382,7 +428,7 @@ __global__ void __launch_bounds__(kColThreads) k_col_prefix(unsigned* __restrict
         v[j] = (dd < radix) ? __ldcg(T + dd) : 0u;
         mine += v[j];
     }
-    unsigned ex = block_exclusive(mine, scan_tmp, nullptr);
+    unsigned ex = block_exclusive(mine, scan_tmp);
 #pragma unroll
     for (int j = 0; j < kPer; ++j) {
         const int dd = threadIdx.x * kPer + j;
@@ -396,45 +442,40 @@ __global__ void __launch_bounds__(kColThreads) k_col_prefix(unsigned* __restrict
 // memory, scanned down each column in 8 segments of 8 tiles.
 __global__ void __launch_bounds__(kColThreads) k_col_apply(unsigned* __restrict__ counts, int tiles, int radix,
                                                            unsigned* __restrict__ S,
-                                                           const unsigned* __restrict__ T,
-                                                           const int* __restrict__ n_dev) {
+                                                           const unsigned* __restrict__ T) {
     __shared__ unsigned tile[kColChunk][33];
     __shared__ unsigned seg_sum[kColSegs][32];
     const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
     const int d = blockIdx.y * 32 + lane;
-    tiles = tiles_of(tiles, n_dev);
-    for (int c = blockIdx.x; c * kColChunk < tiles; c += gridDim.x) {
-        const int t0 = c * kColChunk, rows = min(tiles - t0, kColChunk);
-        constexpr int kRowsPerSeg = kColChunk / kColSegs;
+    const int c = blockIdx.x, t0 = c * kColChunk, rows = min(tiles - t0, kColChunk);
+    constexpr int kRowsPerSeg = kColChunk / kColSegs;
 #pragma unroll
-        for (int j = 0; j < kRowsPerSeg; ++j) {
-            const int r = seg + j * kColSegs;
-            tile[r][lane] = (r < rows && d < radix) ? counts[(size_t)(t0 + r) * radix + d] : 0u;
-        }
-        __syncthreads();
-        unsigned sum = 0u;
+    for (int j = 0; j < kRowsPerSeg; ++j) {
+        const int r = seg + j * kColSegs;
+        tile[r][lane] = (r < rows && d < radix) ? counts[(size_t)(t0 + r) * radix + d] : 0u;
+    }
+    __syncthreads();
+    unsigned sum = 0u;
 #pragma unroll
-        for (int j = 0; j < kRowsPerSeg; ++j) sum += tile[seg * kRowsPerSeg + j][lane];
-        seg_sum[seg][lane] = sum;
-        __syncthreads();
-        unsigned run = (d < radix) ? T[d] + S[(size_t)c * radix + d] : 0u;
-        for (int j = 0; j < seg; ++j) run += seg_sum[j][lane];
-        __syncthreads();  // every segment has read S[c][d] and seg_sum
-        if (seg == 0 && d < radix) S[(size_t)c * radix + d] = 0u;
+    for (int j = 0; j < kRowsPerSeg; ++j) sum += tile[seg * kRowsPerSeg + j][lane];
+    seg_sum[seg][lane] = sum;
+    __syncthreads();
+    unsigned run = (d < radix) ? T[d] + S[(size_t)c * radix + d] : 0u;
+    for (int j = 0; j < seg; ++j) run += seg_sum[j][lane];
+    __syncthreads();  // every segment has read S[c][d] and seg_sum
+    if (seg == 0 && d < radix) S[(size_t)c * radix + d] = 0u;
 #pragma unroll
-        for (int j = 0; j < kRowsPerSeg; ++j) {
-            const int r = seg * kRowsPerSeg + j;
-            const unsigned v = tile[r][lane];
-            tile[r][lane] = run;
-            run += v;
-        }
-        __syncthreads();
+    for (int j = 0; j < kRowsPerSeg; ++j) {
+        const int r = seg * kRowsPerSeg + j;
+        const unsigned v = tile[r][lane];
+        tile[r][lane] = run;
+        run += v;
+    }
+    __syncthreads();
 #pragma unroll
-        for (int j = 0; j < kRowsPerSeg; ++j) {
-            const int r = seg + j * kColSegs;
-            if (r < rows && d < radix) counts[(size_t)(t0 + r) * radix + d] = tile[r][lane];
-        }
-        __syncthreads();  // the staged chunk is written out before the next one is loaded
+    for (int j = 0; j < kRowsPerSeg; ++j) {
+        const int r = seg + j * kColSegs;
+        if (r < rows && d < radix) counts[(size_t)(t0 + r) * radix + d] = tile[r][lane];
     }
 }
 
@@ -573,23 +614,26 @@ size_t sort_workspace_bytes(int n) {
            align_up(((size_t)1 << kMaxRadixBits) * sizeof(unsigned) + sizeof(unsigned), 256);
 }
 
-static int col_sums(const unsigned* counts, int tiles, int radix, unsigned* S, cudaStream_t s, const int* n_dev) {
-    k_col_sums<<<dim3(loop_grid(col_chunks(tiles), n_dev, kNumSMs), (radix + kColThreads - 1) / kColThreads),
-                 kColThreads, 0, s>>>(
-        counts, tiles, radix, S, n_dev);
-    SD_LAUNCHED(s);
-    return SD_OK;
-}
-
-// counts[tiles][radix] (tile-major) with their chunk sums in w.S -> exclusive
-// global offsets, in place; leaves w.S zero.
-static int scan_offsets(unsigned* counts, int tiles, int radix, const SortWs& w, cudaStream_t s, const int* n_dev) {
+// counts[tiles][radix] (tile-major) -> exclusive offsets, in place. chunked: the chunk
+// sums are in w.S (summed here when !sums_ready), the offsets are global and w.S is left
+// zero; otherwise they count the digit's own keys and its totals are in w.T.
+static int scan_offsets(unsigned* counts, int tiles, int radix, const SortWs& w, cudaStream_t s, const int* n_dev,
+                        bool chunked, bool sums_ready) {
+    const int slabs = radix / 32;
+    if (!chunked) {
+        k_col_scan<<<slabs, kScanThreads, 0, s>>>(counts, tiles, radix, w.T, n_dev);
+        SD_LAUNCHED(s);
+        return SD_OK;
+    }
     const int chunks = col_chunks(tiles);
-    const int slabs = (radix + 31) / 32;
-    k_col_prefix<<<slabs, kColThreads, 0, s>>>(w.S, chunks, radix, w.T, w.done, n_dev);
+    if (!sums_ready) {
+        k_col_sums<<<dim3(chunks, (radix + kColThreads - 1) / kColThreads), kColThreads, 0, s>>>(counts, tiles, radix,
+                                                                                               w.S);
+        SD_LAUNCHED(s);
+    }
+    k_col_prefix<<<slabs, kColThreads, 0, s>>>(w.S, chunks, radix, w.T, w.done);
     SD_LAUNCHED(s);
-    k_col_apply<<<dim3(loop_grid(chunks, n_dev, kNumSMs), slabs), kColThreads, 0, s>>>(counts, tiles, radix, w.S,
-                                                                                          w.T, n_dev);
+    k_col_apply<<<dim3(chunks, slabs), kColThreads, 0, s>>>(counts, tiles, radix, w.S, w.T);
     SD_LAUNCHED(s);
     return SD_OK;
 }
@@ -640,6 +684,9 @@ int launch_sort_pairs(const uint32_t* keys_in, const int32_t* vals_in, uint32_t*
     const int tiles = (n + kSortTile - 1) / kSortTile;
     const SortWs w = sort_ws_layout(ws, n);
     unsigned* const* cnt = w.cnt;
+    // a count on the device is a merge's changed set, usually few tiles
+    const bool chunked = !n_dev && tiles > kScanTiles;
+    unsigned* const sums = chunked ? w.S : nullptr;
     // a count on the device: grids of about one wave that loop over the tiles in use
     const int count_grid = loop_grid(tiles, n_dev, kNumSMs * 8);
     const int scatter_grid = loop_grid(tiles, n_dev, kNumSMs * 4);
@@ -668,19 +715,20 @@ int launch_sort_pairs(const uint32_t* keys_in, const int32_t* vals_in, uint32_t*
         if (p == 0 && !first_counts_ready) {
             const int g = count_grid;
             switch (bits) {
-                case 8: k_digit_counts<8><<<g, kSortThreads, 0, s>>>(kin, n, shift, counts, w.S, n_dev); break;
-                case 9: k_digit_counts<9><<<g, kSortThreads, 0, s>>>(kin, n, shift, counts, w.S, n_dev); break;
-                default: k_digit_counts<10><<<g, kSortThreads, 0, s>>>(kin, n, shift, counts, w.S, n_dev); break;
+                case 8: k_digit_counts<8><<<g, kSortThreads, 0, s>>>(kin, n, shift, counts, sums, n_dev); break;
+                case 9: k_digit_counts<9><<<g, kSortThreads, 0, s>>>(kin, n, shift, counts, sums, n_dev); break;
+                default: k_digit_counts<10><<<g, kSortThreads, 0, s>>>(kin, n, shift, counts, sums, n_dev); break;
             }
             SD_LAUNCHED(s);
         }
-        // first-pass counts made elsewhere (the gather, launch_sort_first_counts) still
-        // need their chunk sums; the count kernel above and the scatters add theirs
-        if (p == 0 && first_counts_ready && (rc = col_sums(counts, tiles, 1 << bits, w.S, s, n_dev))) return rc;
-        if ((rc = scan_offsets(counts, tiles, 1 << bits, w, s, n_dev))) return rc;
+        // first-pass counts made elsewhere (the gather, launch_sort_first_counts) come
+        // without chunk sums; the count kernel above and the scatters add theirs
+        if ((rc = scan_offsets(counts, tiles, 1 << bits, w, s, n_dev, chunked, p > 0 || !first_counts_ready)))
+            return rc;
+        const unsigned* totals = chunked ? nullptr : w.T;
 #define SD_SCATTER(B, L)                                                                                   \
-    k_digit_scatter<B, L><<<scatter_grid, kSortThreads, 0, s>>>(kin, vin, kout, vout, n, shift, counts, next, w.S, \
-                                                                next_shift, n_dev)
+    k_digit_scatter<B, L><<<scatter_grid, kSortThreads, 0, s>>>(kin, vin, kout, vout, n, shift, counts, totals, next, \
+                                                                sums, next_shift, n_dev)
 #define SD_SCATTER_B(B)        \
     if (n_dev) SD_SCATTER(B, true); \
     else SD_SCATTER(B, false)

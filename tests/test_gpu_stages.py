@@ -76,6 +76,24 @@ def test_sort_permutation_bit_exact(cuda, lib, oracle, n):
     assert np.array_equal(kout.cpu().numpy()[:n].view(np.uint32), np.sort(keys, kind="stable"))
 
 
+# tiles of 2048 keys: one, a run of the column scan less one and just past it, a second
+# round of it, its last tile count and the first that takes the chunked scan
+@pytest.mark.parametrize("bits", [10, 18, 25])
+@pytest.mark.parametrize("tiles,extra", [(1, 0), (32, -5), (33, 1), (512, 0), (513, -2000), (2048, 0), (2048, 1)])
+def test_sort_across_column_scans(cuda, lib, bits, tiles, extra):
+    n = tiles * 2048 + extra
+    gen = cuda.Generator(device="cuda").manual_seed(n + bits)
+    keys = cuda.randint(0, 1 << bits, (n,), generator=gen, device="cuda", dtype=cuda.int32)
+    keys[: n // 3] = keys[: n // 3] >> 4  # uneven digits
+    ko, vo, kt, vt = (cuda.empty(n, dtype=cuda.int32, device="cuda") for _ in range(4))
+    w = ws(cuda, lib.sd_sort_workspace_bytes(n))
+    L.check(lib.sd_sort_pairs(keys.data_ptr(), None, ko.data_ptr(), vo.data_ptr(), kt.data_ptr(), vt.data_ptr(), n,
+                              bits, w.data_ptr(), w.numel(), None), "sort")
+    ref, perm = cuda.sort(keys, stable=True)
+    assert cuda.equal(ko, ref)
+    assert cuda.equal(vo.long(), perm)
+
+
 def test_sort_with_a_dirty_workspace(cuda, lib):
     """A workspace handed to sd_sort_pairs may hold anything: the sort clears the
     sums it accumulates into before using them."""
