@@ -152,7 +152,9 @@ int launch_interpolate_accel(const float* phi, int G, float pot_scale, const flo
 // learned correction (sd_mlp.cu): out[i] = out_scale * MLP(features of pos[perm ? perm[i] : i])
 size_t mlp_param_count();
 int launch_mlp_infer(const float* params, const float4* pos, const int* perm, int n, const float* rho, int G,
-                     float inv_mean, float out_scale, float4* out, cudaStream_t s);
+                     float inv_mean, float out_scale, float4* out, cudaStream_t s, unsigned* table = nullptr);
+// table (optional): G^3 BF16 of scratch, 16-byte aligned like rho then; the density
+// features are made once per cell instead of once per reading particle
 int launch_apply_mean(float4* vel, const float4* pos, int n, const float* mean_vel, cudaStream_t s);
 int launch_max_speed(const float4* pos, const float4* vel, int n, const float* mean_vel, float* out,
                      cudaStream_t s);

@@ -4,8 +4,7 @@
 // on top of the plain PM acceleration (kIntegrate's accG sample, Sim.cu:822).
 //
 // Numerics: weights and activations are BF16, every matrix product accumulates
-// in FP32 on the tensor cores (the inference with tcgen05.mma into tensor memory,
-// the training's GEMMs with mma.sync m16n8k16), biases and the SiLU are FP32,
+// in FP32 on the tensor cores (mma.sync m16n8k16), biases and the SiLU are FP32,
 // master weights and Adam moments are FP32.
 //
 // Parameter vector (FP32, kMlpParams floats): W1[32][64] (inputs padded 30->32),
@@ -45,6 +44,16 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const unsigned (&a)[4], 
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// d = a b + c
+__device__ __forceinline__ void mma16816(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1,
+                                         const float4& c) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+        "{%10,%11,%12,%13};\n"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c.x), "f"(c.y), "f"(c.z), "f"(c.w));
+}
+
 // SiLU through the hardware tanh (one MUFU op): sigmoid(z) = (1 + tanh(z/2)) / 2.
 // Its relative error (about 2^-11) is below the BF16 rounding of the activations;
 // training and inference use the same function.
@@ -63,8 +72,22 @@ __device__ __forceinline__ float silu_grad(float z) {
 
 // ---- features -------------------------------------------------------------------
 // the density feature of one cell: log(1 + rho / rho_bar) - log 2
+// (its argument is at least 1, so flushing subnormals changes nothing)
 __device__ __forceinline__ float cell_feature(float r, float inv_mean) {
-    return __logf(1.f + r * inv_mean) - 0.69314718055994531f;
+    float l;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(fmaf(r, inv_mean, 1.f)));
+    return fmaf(l, 0.69314718055994531f, -0.69314718055994531f);
+}
+
+// The density feature of every cell in BF16, as the network takes it: a step's particles
+// read each cell's many times (four cells a thread; the grid's side is a multiple of 16).
+__global__ void __launch_bounds__(256) k_feature_table(const float4* __restrict__ rho, size_t quads, float inv_mean,
+                                                       uint2* __restrict__ table) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= quads) return;
+    const float4 r = rho[i];
+    table[i] = make_uint2(pack_bf16(cell_feature(r.x, inv_mean), cell_feature(r.y, inv_mean)),
+                          pack_bf16(cell_feature(r.z, inv_mean), cell_feature(r.w, inv_mean)));
 }
 
 __device__ __forceinline__ void particle_features(const float* __restrict__ rho, int G, float inv_mean, float4 p,
@@ -90,6 +113,41 @@ __device__ __forceinline__ void particle_features(const float* __restrict__ rho,
     f[31] = 0.f;
 }
 
+// The 16 packed feature words of p, from the table: the three cells of a row lie in two
+// aligned words (two loads where there were three, no logarithm, no rounding).
+__device__ __forceinline__ void table_features(const unsigned* __restrict__ table, int G, float4 p, unsigned (&f)[16]) {
+    const int m = G - 1, mw = (G >> 1) - 1;
+    const int cx = cell_axis(p.x, G), cy = cell_axis(p.y, G), cz = cell_axis(p.z, G);
+    const int w0 = ((cx - 1) >> 1) & mw, w1 = (w0 + 1) & mw;
+    const int shift = ((cx - 1) & 1) * 16;
+    unsigned lo[9], hi[9];  // the row's words
+#pragma unroll
+    for (int r = 0; r < 9; ++r) {
+        const int y = (cy + r % 3 - 1) & m, z = (cz + r / 3 - 1) & m;
+        const unsigned* row = table + ((size_t)z * G + y) * (G >> 1);
+        lo[r] = __ldg(row + w0);
+        hi[r] = __ldg(row + w1);
+    }
+#pragma unroll
+    for (int r = 0; r < 9; ++r) {  // cells 0 and 1 of the row in lo, cell 2 in the low half of hi
+        lo[r] = __funnelshift_r(lo[r], hi[r], shift);
+        hi[r] >>= shift;
+    }
+    // features 3 r, 3 r + 1, 3 r + 2; three words hold two rows
+#pragma unroll
+    for (int r = 0; r < 8; r += 2) {
+        f[3 * r / 2] = lo[r];
+        f[3 * r / 2 + 1] = __byte_perm(hi[r], lo[r + 1], 0x5410);
+        f[3 * r / 2 + 2] = __byte_perm(lo[r + 1], hi[r + 1], 0x5432);
+    }
+    f[12] = lo[8];
+    const float ox = p.x * (float)G - (float)cx - 0.5f, oy = p.y * (float)G - (float)cy - 0.5f,
+                oz = p.z * (float)G - (float)cz - 0.5f;
+    f[13] = __byte_perm(hi[8], pack_bf16(0.f, ox), 0x7610);
+    f[14] = pack_bf16(oy, oz);
+    f[15] = 0u;
+}
+
 __global__ void k_features(const float4* __restrict__ pos, const int* __restrict__ perm, int n,
                            const float* __restrict__ rho, int G, float inv_mean, __nv_bfloat16* __restrict__ out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -109,276 +167,188 @@ __global__ void k_features(const float4* __restrict__ pos, const int* __restrict
                           pack_bf16(f[8 * q + 4], f[8 * q + 5]), pack_bf16(f[8 * q + 6], f[8 * q + 7]));
 }
 
-// ---- fused inference on the 5th-generation tensor cores (tcgen05) -------------------
-// One CTA of 128 threads takes tiles of 128 particles, thread r <-> row r of the
-// tile <-> tensor-memory lane r. Each layer is one tcgen05.mma chain (M = 128,
-// N = 64 or 16, K in steps of 16, BF16 x BF16 -> FP32) issued by thread 0: the
-// activations (operand A) sit in tensor memory, the weights (operand B) in
-// shared memory, the FP32 accumulator in 64 tensor-memory columns. Completion
-// arrives on an mbarrier (tcgen05.commit); every thread reads its row back with
-// tcgen05.ld, adds the bias, applies the SiLU and writes its row of the next
-// layer's A with tcgen05.st -- no shared-memory round trip for the activations.
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void ldm4(unsigned (&r)[4], uint32_t a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(a));
+}
+__device__ __forceinline__ void ldm4t(unsigned (&r)[4], uint32_t a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(a));
+}
+
+// ---- fused inference -----------------------------------------------------------------
+// Each warp takes 32 particles, a lane each, through the network by itself: the lane
+// forms its particle's features, the warp swaps them through a shared-memory row each
+// into the A fragments of two m16n8k16 row tiles, and from there every layer stays in
+// registers: the accumulators of 16 units, activated and packed to BF16, are one k-step
+// of the next layer's A fragments. A step of layer 2 feeds layer 3 at once, so only
+// layer 1's activations (32 registers) are held. The weights' B fragments come from
+// shared memory by ldmatrix and serve both row tiles.
 //
-// A: row r in lane r, element k in column kAcol + k / 2 (two BF16 per 32-bit
-// column, k even in the low half); k-step s reads columns kAcol + 8 s.
-// B: the canonical K-major layout without swizzle, 8 x 16-byte core matrices
-// (8 rows x 8 BF16): element (row n, k) of a matrix with K columns at byte
-// (n / 8) * SBO + (k / 8) * 128 + (n % 8) * 16 + (k % 8) * 2, SBO = K * 16; the
-// descriptor of k-step s starts 256 s bytes in (leading offset 128 bytes: the two
-// 8-column halves of the step).
+// No barrier follows the loading of the weights, and nothing waits but for operands: with
+// tcgen05.mma, four CTAs of 128 rows an SM (their tensor memory) met at two barriers and a
+// completion wait for each layer, and 2,097,152 particles on 128^3 took 172 us. Here 158
+// with features from rho, 136 (and 2.7 for the table) with the cells' features made once
+// and the biases as the products' first addend. What bounds it now are the products on
+// this path (with 64 of a tile's 104 left out 86 us), then the 128 tanh a particle (58 us
+// of the special-function unit); 4 to 6 CTAs an SM measure the same, and loading a tile's
+// features beside the last one's layers gains nothing.
 //
-// Measured against the mma.sync kernel it replaced (2,097,152 particles on 128^3,
-// identical outputs): 0.165 against 0.153 ms. The tensor pipe is 8 % busy; the
-// kernel waits on the feature gathers from L2 and on the SiLU's dependent chains
-// at four CTAs per SM (the tensor-memory columns), not on the products.
-namespace tc {
-constexpr int kThreads = 128;                  // one warpgroup: TMEM lanes 0..127
-constexpr int kTmemCols = 128;                 // FP32 accumulator (columns 0..63) + BF16 operand A (64..95)
-constexpr int kAcol = 64;                      // A: row r in lane r, BF16 pairs along K in consecutive columns
-constexpr int kN3 = 16;                        // output layer N (3 outputs padded)
-constexpr int kB1 = 0;                         // W1^T [64][32]
-constexpr int kB2 = kB1 + kH * kIn * 2;        // W2^T [64][64]
-constexpr int kB3 = kB2 + kH * kH * 2;         // W3^T [16][64] (rows 8..15 zero)
-constexpr int kBias = kB3 + kN3 * kH * 2;      // b1[64], b2[64], b3[8] (float)
-constexpr int kBar = kBias + (2 * kH + kOut) * 4 + 8;  // mbarrier (8-byte aligned)
-constexpr int kTaddr = kBar + 8;
-constexpr int kSmem = kTaddr + 8;
-constexpr int kSmemLaunch = 46 * 1024;  // at most four CTAs per SM (see launch_mlp_infer)
-static_assert(kBar % 8 == 0 && kB2 % 16 == 0 && kB3 % 16 == 0, "alignment");
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-// byte offset of element (r, k) in a K-major shared-memory operand with K columns
-__device__ __forceinline__ int op_off(int r, int k, int K) { return (r >> 3) * (K * 16) + (k >> 3) * 128 + (r & 7) * 16 + (k & 7) * 2; }
-
-__device__ __forceinline__ uint64_t desc(uint32_t addr, int K) {
-    const uint64_t lbo = 128 >> 4, sbo = (uint64_t)(K * 16) >> 4;
-    return (uint64_t)((addr >> 4) & 0x3FFF) | (lbo << 16) | (sbo << 32) | (1ull << 46);  // version 1, no swizzle
-}
-
-// instruction descriptor: BF16 x BF16 -> FP32, both K-major, M = 128
-__host__ __device__ constexpr uint32_t idesc(int N) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-}
-
-// A from tensor memory (the activations), B from shared memory (the weights)
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b, uint32_t id, uint32_t acc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(b), "r"(id), "r"(acc));
-}
-
-// 16 32-bit words into columns [col, col + 16) of this thread's TMEM lane
-__device__ __forceinline__ void st16(uint32_t taddr, const unsigned (&w)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(
-            taddr),
-        "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]), "r"(w[8]), "r"(w[9]),
-        "r"(w[10]), "r"(w[11]), "r"(w[12]), "r"(w[13]), "r"(w[14]), "r"(w[15])
-        : "memory");
-}
-__device__ __forceinline__ void wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-__device__ __forceinline__ void commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-                 : "memory");
-}
-
-__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-// Bounded wait for phase `parity` of the mbarrier; false if it gave up.
-__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity) {
-    for (int it = 0; it < (1 << 22); ++it) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred q;\n\tmbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, q;\n\t}\n"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (ok) return true;
-    }
-    return false;
-}
-
-// FP32 columns [col, col + 16 X) of this thread's TMEM lane: X loads of 16 columns
-// in flight together, one wait
-__device__ __forceinline__ void ld16_issue(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-}
-template <int X>
-__device__ __forceinline__ void ld_cols(uint32_t taddr, float (&v)[16 * X]) {
-    uint32_t r[X][16];
-#pragma unroll
-    for (int x = 0; x < X; ++x) ld16_issue(taddr + 16 * x, r[x]);
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int x = 0; x < X; ++x)
-#pragma unroll
-        for (int q = 0; q < 16; ++q) v[16 * x + q] = __uint_as_float(r[x][q]);
-}
-}  // namespace tc
-
-// Waits that gave up (an mbarrier phase that never completed): the tile's outputs
-// are NaN and the count is readable through sd_mlp_wait_timeouts.
-__device__ unsigned g_mlp_wait_timeouts = 0;
-
 // The two hidden layers run on weights and biases scaled by 1/2 (exact in BF16 and
 // FP32), so each accumulator holds u = z / 2 and SiLU(z) = z sigmoid(z) =
 // u + u tanh(u): one tanh and one FMA per unit, rounded to BF16 once.
-__global__ void __launch_bounds__(tc::kThreads, 4) k_mlp_infer_tc(const float* __restrict__ params,
-                                                              const float4* __restrict__ pos,
-                                                              const int* __restrict__ perm, int n,
-                                                              const float* __restrict__ rho, int G,
-                                                              float inv_mean, float out_scale,
-                                                              float4* __restrict__ out) {
-    extern __shared__ __align__(1024) unsigned char sm[];
-    const int r = threadIdx.x, warp = r >> 5;
-    float* bias = reinterpret_cast<float*>(sm + tc::kBias);
-    const uint32_t bar = tc::smem_u32(sm + tc::kBar);
-    uint32_t* taddr_s = reinterpret_cast<uint32_t*>(sm + tc::kTaddr);
-    // weights as K-major operands (W[k][n] -> row n, column k), the same BF16 rounding
-    // as the training's copies
-    for (int e = r; e < kH * kIn; e += tc::kThreads) {
-        const int nn = e / kIn, k = e % kIn;
-        *reinterpret_cast<__nv_bfloat16*>(sm + tc::kB1 + tc::op_off(nn, k, kIn)) =
-            __float2bfloat16_rn(0.5f * params[oW1 + k * kH + nn]);
-    }
-    for (int e = r; e < kH * kH; e += tc::kThreads) {
-        const int nn = e / kH, k = e % kH;
-        *reinterpret_cast<__nv_bfloat16*>(sm + tc::kB2 + tc::op_off(nn, k, kH)) =
-            __float2bfloat16_rn(0.5f * params[oW2 + k * kH + nn]);
-    }
-    for (int e = r; e < tc::kN3 * kH; e += tc::kThreads) {
-        const int nn = e / kH, k = e % kH;
-        *reinterpret_cast<__nv_bfloat16*>(sm + tc::kB3 + tc::op_off(nn, k, kH)) =
-            __float2bfloat16_rn(nn < kOut ? params[oW3 + k * kOut + nn] : 0.f);
-    }
-    for (int e = r; e < kH; e += tc::kThreads) {
-        bias[e] = 0.5f * params[oB1 + e];
-        bias[kH + e] = 0.5f * params[oB2 + e];
-    }
-    if (r < kOut) bias[2 * kH + r] = params[oB3 + r];
-    if (r == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::smem_u32(taddr_s)),
-                     "r"(tc::kTmemCols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    tc::fence_proxy();  // the weights, written by the threads, are read by the tensor cores
-    tc::fence_before();
-    __syncthreads();
-    tc::fence_after();
-    const uint32_t tmem = *taddr_s;
-    const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);  // this warp's 32 lanes
-    const uint32_t a_lane = lane_addr + tc::kAcol;  // this thread's row of the operand A
-    const uint32_t b1 = tc::smem_u32(sm + tc::kB1), b2 = tc::smem_u32(sm + tc::kB2),
-                   b3 = tc::smem_u32(sm + tc::kB3);
-    uint32_t phase = 0;
-    bool ok = true;
-    const int tiles = (n + tc::kThreads - 1) / tc::kThreads;
-    // this thread's particle of the CTA's next tile, loaded while the current tile
-    // runs through the network
-    float4 pn = make_float4(-1.f, -1.f, -1.f, 0.f);
-    if (blockIdx.x * tc::kThreads + r < n) {
-        const int i0 = blockIdx.x * tc::kThreads + r;
-        pn = pos[perm ? perm[i0] : i0];
-    }
-    for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-        const int i = t * tc::kThreads + r;
-        const float4 p = pn;
-        {
-            const int inx = i + gridDim.x * tc::kThreads;
-            pn = make_float4(-1.f, -1.f, -1.f, 0.f);
-            if (inx < n) pn = pos[perm ? perm[inx] : inx];
+namespace inf {
+constexpr int kThreads = 128, kWarps = kThreads / 32, kCtasPerSm = 5;
+constexpr int kS = 72;   // BF16 elements of a 64-wide row: 8 rows of 16 bytes fall in 32 banks
+constexpr int kSF = 40;  // of a row of features
+
+struct Smem {
+    __nv_bfloat16 w1[kIn][kS], w2[kH][kS], w3[kH][kOut];
+    __nv_bfloat16 feat[kWarps][32][kSF];
+    float4 b[2 * kH / 2];  // units 2 i, 2 i + 1 of the hidden layers, twice: an accumulator's first addend
+    float b3[kOut];
+};
+
+// u + u tanh(u) of 16 units of the two row tiles -> one k-step of A fragments
+__device__ __forceinline__ void activate(const float (&u)[2][2][4], unsigned (&h)[2][4]) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+            const float* v = u[mt][q];
+            h[mt][2 * q] = pack_bf16(fmaf(v[0], tanh_approx(v[0]), v[0]), fmaf(v[1], tanh_approx(v[1]), v[1]));
+            h[mt][2 * q + 1] = pack_bf16(fmaf(v[2], tanh_approx(v[2]), v[2]), fmaf(v[3], tanh_approx(v[3]), v[3]));
         }
+}
+
+// acc (two row tiles x 16 units) = bias + A * W[k][16 nc ..]
+template <int KS>
+__device__ __forceinline__ void layer16(float (&acc)[2][2][4], const unsigned (&a)[KS][2][4],
+                                        const __nv_bfloat16* w, const float4* bias, int nc, int lane) {
+    const float4 c0 = bias[8 * nc + (lane & 3)], c1 = bias[8 * nc + 4 + (lane & 3)];
+#pragma unroll
+    for (int s = 0; s < KS; ++s) {
+        unsigned b[4];  // {k 0..7, k 8..15} of the two n-tiles
+        ldm4t(b, smem_addr(w + (16 * s + (lane & 15)) * kS + 16 * nc + 8 * (lane >> 4)));
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+            if (s == 0) {
+                mma16816(acc[mt][0], a[s][mt], b[0], b[1], c0);
+                mma16816(acc[mt][1], a[s][mt], b[2], b[3], c1);
+            } else {
+                mma16816(acc[mt][0], a[s][mt], b[0], b[1]);
+                mma16816(acc[mt][1], a[s][mt], b[2], b[3]);
+            }
+        }
+    }
+}
+}  // namespace inf
+
+// TABLE: the density features come from `table` (k_feature_table); otherwise from rho.
+template <bool TABLE>
+__global__ void __launch_bounds__(inf::kThreads, inf::kCtasPerSm)
+    k_mlp_infer(const float* __restrict__ params, const float4* __restrict__ pos, const int* __restrict__ perm, int n,
+                const float* __restrict__ rho, const unsigned* __restrict__ table, int G, float inv_mean,
+                float out_scale, float4* __restrict__ out) {
+    __shared__ __align__(16) inf::Smem s;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
+    // the same BF16 rounding of the weights as the training's copies
+    for (int e = tid; e < kIn * kH; e += inf::kThreads)
+        s.w1[e / kH][e % kH] = __float2bfloat16_rn(0.5f * params[oW1 + e]);
+    for (int e = tid; e < kH * kH; e += inf::kThreads)
+        s.w2[e / kH][e % kH] = __float2bfloat16_rn(0.5f * params[oW2 + e]);
+    for (int e = tid; e < kH * kOut; e += inf::kThreads) s.w3[e / kOut][e % kOut] = __float2bfloat16_rn(params[oW3 + e]);
+    if (tid < kH) {
+        const float* b = params + (tid < kH / 2 ? oB1 + 2 * tid : oB2 + 2 * tid - kH);
+        s.b[tid] = make_float4(0.5f * b[0], 0.5f * b[1], 0.5f * b[0], 0.5f * b[1]);
+    }
+    if (tid < kOut) s.b3[tid] = params[oB3 + tid];
+    __syncthreads();
+
+    const int tiles = (n + 31) / 32, stride = gridDim.x * inf::kWarps;
+    const float4 none = make_float4(-1.f, -1.f, -1.f, 0.f);
+    // the next tile's particle and the index of the one after are on their way while a
+    // tile runs
+    auto index_at = [&](int tile) {
+        const long long i = (long long)tile * 32 + lane;
+        return i < n ? (perm ? perm[i] : (int)i) : -1;
+    };
+    int tile = blockIdx.x * inf::kWarps + w;
+    int j = tile < tiles ? index_at(tile) : -1;
+    float4 p = j >= 0 ? pos[j] : none;
+    j = tile + stride < tiles ? index_at(tile + stride) : -1;
+    float4 pn = j >= 0 ? pos[j] : none;
+    for (; tile < tiles; tile += stride) {
+        j = (long long)tile + 2ll * stride < tiles ? index_at(tile + 2 * stride) : -1;
+        unsigned a[2][2][4];
         {
-            unsigned w[16];
+            uint4* row = reinterpret_cast<uint4*>(&s.feat[w][lane][0]);
             if (p.x < 0.f) {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) w[j] = 0u;
+                for (int q = 0; q < 4; ++q) row[q] = make_uint4(0u, 0u, 0u, 0u);
+            } else if (TABLE) {
+                unsigned f[16];
+                table_features(table, G, p, f);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) row[q] = make_uint4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]);
             } else {
                 float f[32];
                 particle_features(rho, G, inv_mean, p, f);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) w[j] = pack_bf16(f[2 * j], f[2 * j + 1]);
+                for (int q = 0; q < 4; ++q)
+                    row[q] = make_uint4(pack_bf16(f[8 * q], f[8 * q + 1]), pack_bf16(f[8 * q + 2], f[8 * q + 3]),
+                                        pack_bf16(f[8 * q + 4], f[8 * q + 5]), pack_bf16(f[8 * q + 6], f[8 * q + 7]));
             }
-            tc::st16(a_lane, w);
-            tc::wait_st();
-        }
-        // three layers; layer l reads A (K = 32 for the first, 64 after) and B_l
-#pragma unroll 1
-        for (int layer = 0; layer < 3; ++layer) {
-            const int K = layer == 0 ? kIn : kH;
-            tc::fence_before();  // this thread's operand row (tcgen05.st, waited) before the MMA
-            __syncthreads();
-            if (r == 0) {
-                tc::fence_after();
-                const uint32_t bb = layer == 0 ? b1 : (layer == 1 ? b2 : b3);
-                const uint32_t id = tc::idesc(layer == 2 ? tc::kN3 : kH);
-                // k-step s: A columns kAcol + 8 s (16 BF16 per row), B rows from byte 256 s
-                for (int s = 0; s < K / 16; ++s)
-                    tc::mma_ts(tmem, tmem + tc::kAcol + 8 * s, tc::desc(bb + 256 * s, K), id, s > 0);
-                tc::commit(bar);
-            }
-            // every thread waits; the verdict is made uniform so the CTA's barriers stay matched
-            if (!__syncthreads_and(tc::wait_bar(bar, phase))) {
-                ok = false;
-                if (r == 0) atomicAdd(&g_mlp_wait_timeouts, 1u);
-                break;
-            }
-            phase ^= 1;
-            tc::fence_after();
-            if (layer < 2) {
-                // this row's 64 pre-activations -> SiLU -> the next layer's operand row
-                // (the MMA that read A has completed)
+            __syncwarp();
 #pragma unroll
-                for (int c2 = 0; c2 < kH / 32; ++c2) {
-                    float v[32];
-                    tc::ld_cols<2>(lane_addr + 32 * c2, v);
-                    const float* b = bias + layer * kH + 32 * c2;
-                    unsigned h[16];
+            for (int k = 0; k < 2; ++k)
 #pragma unroll
-                    for (int q = 0; q < 16; ++q) {
-                        const float u0 = v[2 * q] + b[2 * q], u1 = v[2 * q + 1] + b[2 * q + 1];
-                        h[q] = pack_bf16(fmaf(u0, tanh_approx(u0), u0), fmaf(u1, tanh_approx(u1), u1));
-                    }
-                    tc::st16(a_lane + 16 * c2, h);  // units 32 c2 .. 32 c2 + 31
-                }
-                tc::wait_st();
-            } else {
-                float v[16];
-                tc::ld_cols<1>(lane_addr, v);
-                const float* b = bias + 2 * kH;
-                if (i < n)
-                    out[i] = (p.x >= 0.f) ? make_float4((v[0] + b[0]) * out_scale, (v[1] + b[1]) * out_scale,
-                                                        (v[2] + b[2]) * out_scale, 0.f)
-                                          : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
+                for (int mt = 0; mt < 2; ++mt)
+                    ldm4(a[k][mt], smem_addr(&s.feat[w][16 * mt + (lane & 15)][16 * k + 8 * (lane >> 4)]));
+            __syncwarp();
         }
-        if (!ok && i < n) out[i] = make_float4(__int_as_float(0x7fc00000), __int_as_float(0x7fc00000),
-                                               __int_as_float(0x7fc00000), 0.f);
-    }
-    // every tcgen05.ld has completed (wait::ld) and no MMA is in flight once the
-    // last wait returned; a CTA whose wait gave up drains with a second bounded wait
-    if (!ok && r == 0) tc::wait_bar(bar, phase);
-    tc::fence_before();
-    __syncthreads();
-    if (warp == 0) {
-        tc::fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tc::kTmemCols)
-                     : "memory");
+        unsigned h1[4][2][4];
+#pragma unroll
+        for (int nc = 0; nc < 4; ++nc) {
+            float acc[2][2][4];
+            inf::layer16<2>(acc, a, &s.w1[0][0], s.b, nc, lane);
+            inf::activate(acc, h1[nc]);
+        }
+        float y[2][4] = {};
+#pragma unroll
+        for (int nc = 0; nc < 4; ++nc) {
+            float acc[2][2][4];
+            unsigned h2[2][4];
+            inf::layer16<4>(acc, h1, &s.w2[0][0], s.b + kH / 2, nc, lane);
+            inf::activate(acc, h2);
+            unsigned b0, b1;  // W3 rows 16 nc ..
+            asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n"
+                         : "=r"(b0), "=r"(b1)
+                         : "r"(smem_addr(&s.w3[16 * nc + (lane & 15)][0])));
+            mma16816(y[0], h2[0], b0, b1);
+            mma16816(y[1], h2[1], b0, b1);
+        }
+        // outputs 0 and 1 of a row sit in the first lane of its four, 2 in the second
+        const unsigned live = __ballot_sync(0xffffffffu, p.x >= 0.f);
+        const float b0 = s.b3[0], b1 = s.b3[1], b2 = s.b3[2];
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int hi = 0; hi < 2; ++hi) {
+                const float y2 = __shfl_down_sync(0xffffffffu, y[mt][2 * hi], 1);
+                const int r = 16 * mt + 8 * hi + g;
+                const long long i = (long long)tile * 32 + r;
+                if (t == 0 && i < n)
+                    out[i] = ((live >> r) & 1u) ? make_float4((y[mt][2 * hi] + b0) * out_scale,
+                                                              (y[mt][2 * hi + 1] + b1) * out_scale,
+                                                              (y2 + b2) * out_scale, 0.f)
+                                                : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        p = pn;
+        pn = j >= 0 ? pos[j] : none;
     }
 }
 
@@ -412,17 +382,6 @@ struct Smem {
     float colsum[kWarps][2 * kH + kOut + 1];
 };
 
-__device__ __forceinline__ uint32_t addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void ldm4(unsigned (&r)[4], uint32_t a) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(a));
-}
-__device__ __forceinline__ void ldm4t(unsigned (&r)[4], uint32_t a) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(a));
-}
 
 // acc (16 x 64) += A (16 x 16 KS, fragments) * W[k][n] (rows of kS elements)
 template <int KS>
@@ -433,7 +392,7 @@ __device__ __forceinline__ void mul_w(float (&acc)[8][4], const unsigned (&a)[KS
 #pragma unroll
         for (int np = 0; np < 4; ++np) {
             unsigned b[4];  // two n-tiles: {k 0..7, k 8..15} of each
-            ldm4t(b, addr(w + (16 * s + (lane & 15)) * kS + 16 * np + 8 * (lane >> 4)));
+            ldm4t(b, smem_addr(w + (16 * s + (lane & 15)) * kS + 16 * np + 8 * (lane >> 4)));
             mma16816(acc[2 * np], a[s], b[0], b[1]);
             mma16816(acc[2 * np + 1], a[s], b[2], b[3]);
         }
@@ -477,11 +436,11 @@ __device__ __forceinline__ void back_silu(const float (&dh)[8][4], const float (
 
 // A fragment of M^T for 16 rows: elements (m0.., r0..) of a row-major [row][m] matrix
 __device__ __forceinline__ uint32_t at_a(const __nv_bfloat16* m, int stride, int r0, int m0, int lane) {
-    return addr(m + (r0 + (lane & 7) + 8 * (lane >> 4)) * stride + m0 + 8 * ((lane >> 3) & 1));
+    return smem_addr(m + (r0 + (lane & 7) + 8 * (lane >> 4)) * stride + m0 + 8 * ((lane >> 3) & 1));
 }
 // B fragments of two n-tiles for 16 rows of a row-major [row][n] matrix
 __device__ __forceinline__ uint32_t at_b(const __nv_bfloat16* m, int stride, int r0, int n0, int lane) {
-    return addr(m + (r0 + (lane & 15)) * stride + n0 + 8 * (lane >> 4));
+    return smem_addr(m + (r0 + (lane & 15)) * stride + n0 + 8 * (lane >> 4));
 }
 
 // 16 x 8 accumulator tile to rows m0.. of a row-major float matrix
@@ -541,9 +500,9 @@ __global__ void __launch_bounds__(tr::kThreads, 1) k_train_tile(const float* __r
             unsigned h[4][4];
             {
                 unsigned a[2][4];
-                const uint32_t xa = tr::addr(&s.x[16 * w + (lane & 15)][8 * (lane >> 4)]);
-                tr::ldm4(a[0], xa);
-                tr::ldm4(a[1], xa + 32);
+                const uint32_t xa = smem_addr(&s.x[16 * w + (lane & 15)][8 * (lane >> 4)]);
+                ldm4(a[0], xa);
+                ldm4(a[1], xa + 32);
                 tr::mul_w<2>(z1, a, &s.w1[0][0], lane);
             }
             tr::activate(z1, s.b, h, s.h1, row, t);
@@ -553,7 +512,7 @@ __global__ void __launch_bounds__(tr::kThreads, 1) k_train_tile(const float* __r
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
                 unsigned b[4];  // k-steps 2q and 2q + 1
-                tr::ldm4t(b, tr::addr(&s.w3[32 * q + lane][0]));
+                ldm4t(b, smem_addr(&s.w3[32 * q + lane][0]));
                 mma16816(y, h[2 * q], b[0], b[1]);
                 mma16816(y, h[2 * q + 1], b[2], b[3]);
             }
@@ -580,7 +539,7 @@ __global__ void __launch_bounds__(tr::kThreads, 1) k_train_tile(const float* __r
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
                 unsigned b[4];  // units 32 q + 8 j: row n, 8 outputs along k
-                tr::ldm4(b, tr::addr(&s.w3[32 * q + lane][0]));
+                ldm4(b, smem_addr(&s.w3[32 * q + lane][0]));
 #pragma unroll
                 for (int j = 0; j < 4; ++j) mma16816(dh[4 * q + j], ay, b[j], 0u);
             }
@@ -593,7 +552,7 @@ __global__ void __launch_bounds__(tr::kThreads, 1) k_train_tile(const float* __r
 #pragma unroll
                 for (int q = 0; q < 2; ++q) {
                     unsigned b[4];  // k-steps 2q, 2q + 1
-                    tr::ldm4(b, tr::addr(&s.w2[8 * nt + (lane & 7)][32 * q + 8 * (lane >> 3)]));
+                    ldm4(b, smem_addr(&s.w2[8 * nt + (lane & 7)][32 * q + 8 * (lane >> 3)]));
                     mma16816(dg[nt], dz[2 * q], b[0], b[1]);
                     mma16816(dg[nt], dz[2 * q + 1], b[2], b[3]);
                 }
@@ -616,15 +575,15 @@ __global__ void __launch_bounds__(tr::kThreads, 1) k_train_tile(const float* __r
 #pragma unroll 2
         for (int k = 0; k < tr::kRows / 16; ++k) {
             unsigned a[4], b[4];
-            tr::ldm4t(a, tr::at_a(&s.h1[0][0], tr::kS, 16 * k, m2, lane));
-            tr::ldm4t(b, tr::at_b(&s.dz2[0][0], tr::kS, 16 * k, n2, lane));
+            ldm4t(a, tr::at_a(&s.h1[0][0], tr::kS, 16 * k, m2, lane));
+            ldm4t(b, tr::at_b(&s.dz2[0][0], tr::kS, 16 * k, n2, lane));
             mma16816(dw2[0], a, b[0], b[1]);
             mma16816(dw2[1], a, b[2], b[3]);
-            tr::ldm4t(b, tr::at_b(&s.dz2[0][0], tr::kS, 16 * k, n2 + 16, lane));
+            ldm4t(b, tr::at_b(&s.dz2[0][0], tr::kS, 16 * k, n2 + 16, lane));
             mma16816(dw2[2], a, b[0], b[1]);
             mma16816(dw2[3], a, b[2], b[3]);
-            tr::ldm4t(a, tr::at_a(&s.x[0][0], tr::kSX, 16 * k, m1, lane));
-            tr::ldm4t(b, tr::at_b(&s.dz1[0][0], tr::kS, 16 * k, n1, lane));
+            ldm4t(a, tr::at_a(&s.x[0][0], tr::kSX, 16 * k, m1, lane));
+            ldm4t(b, tr::at_b(&s.dz1[0][0], tr::kS, 16 * k, n1, lane));
             mma16816(dw1[0], a, b[0], b[1]);
             mma16816(dw1[1], a, b[2], b[3]);
         }
@@ -632,10 +591,10 @@ __global__ void __launch_bounds__(tr::kThreads, 1) k_train_tile(const float* __r
         for (int q = 0; q < 2; ++q) {  // warps 0..3: the tile's first 64 rows, 4..7: the rest
             const int k = 64 * (w >> 2) + 32 * q;
             unsigned a[4], b[4];
-            tr::ldm4t(b, tr::addr(&s.dy[k + lane][0]));
-            tr::ldm4t(a, tr::at_a(&s.h2[0][0], tr::kS, k, m3, lane));
+            ldm4t(b, smem_addr(&s.dy[k + lane][0]));
+            ldm4t(a, tr::at_a(&s.h2[0][0], tr::kS, k, m3, lane));
             mma16816(dw3, a, b[0], b[1]);
-            tr::ldm4t(a, tr::at_a(&s.h2[0][0], tr::kS, k + 16, m3, lane));
+            ldm4t(a, tr::at_a(&s.h2[0][0], tr::kS, k + 16, m3, lane));
             mma16816(dw3, a, b[2], b[3]);
         }
     }
@@ -729,16 +688,21 @@ float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
 size_t mlp_param_count() { return kParams; }
 
 int launch_mlp_infer(const float* params, const float4* pos, const int* perm, int n, const float* rho, int G,
-                     float inv_mean, float out_scale, float4* out, cudaStream_t s) {
+                     float inv_mean, float out_scale, float4* out, cudaStream_t s, unsigned* table) {
     if (n <= 0) return SD_OK;
-    // tiles of 128 particles; four CTAs fill an SM's 512 tensor-memory columns (128 each).
-    // The dynamic shared memory is padded so that no fifth CTA is placed on an SM, where
-    // its tcgen05.alloc would wait for one of the four to finish.
-    static_assert(tc::kSmemLaunch >= tc::kSmem && 5 * (tc::kSmemLaunch + 1024) > 228 * 1024, "four CTAs per SM");
-    const int tiles = (n + tc::kThreads - 1) / tc::kThreads;
-    const int blocks = tiles < 148 * 4 ? tiles : 148 * 4;
-    k_mlp_infer_tc<<<blocks, tc::kThreads, tc::kSmemLaunch, s>>>(params, pos, perm, n, rho, G, inv_mean, out_scale,
-                                                                 out);
+    const int tiles = (n + 31) / 32, need = (tiles + inf::kWarps - 1) / inf::kWarps, wave = 148 * inf::kCtasPerSm;
+    const int blocks = need < wave ? need : wave;
+    if (table) {
+        const size_t quads = (size_t)G * G * G / 4;
+        k_feature_table<<<(unsigned)((quads + 255) / 256), 256, 0, s>>>(reinterpret_cast<const float4*>(rho), quads,
+                                                                        inv_mean, reinterpret_cast<uint2*>(table));
+        SD_LAUNCHED(s);
+        k_mlp_infer<true><<<blocks, inf::kThreads, 0, s>>>(params, pos, perm, n, rho, table, G, inv_mean, out_scale,
+                                                           out);
+    } else {
+        k_mlp_infer<false><<<blocks, inf::kThreads, 0, s>>>(params, pos, perm, n, rho, nullptr, G, inv_mean, out_scale,
+                                                            out);
+    }
     SD_LAUNCHED(s);
     return SD_OK;
 }
@@ -758,11 +722,8 @@ extern "C" {
 
 int sd_mlp_param_count(void) { return kParams; }
 
-int sd_mlp_wait_timeouts(void) {
-    unsigned v = 0;
-    if (SD_CUDA(cudaMemcpyFromSymbol(&v, g_mlp_wait_timeouts, sizeof(v)))) return SD_E_CUDA;
-    return (int)v;
-}
+// The inference has no wait that could give up.
+int sd_mlp_wait_timeouts(void) { return SD_CUDA(cudaDeviceSynchronize()) ? SD_E_CUDA : 0; }
 
 int sd_mlp_features(const float* pos, const int32_t* perm, int n, const float* rho, int G, float inv_mean,
                     void* features_bf16, void* stream) {

@@ -155,6 +155,7 @@ void free_buffers(sd_sim* s) {
     s->rs_base = nullptr;
     free_dev(s->partials); free_dev(s->mom); free_dev(s->mean);
     free_dev(s->mlp_out);
+    free_dev(s->mlp_table);
     free_dev(s->diag_rec);
     free_dev(s->diag_count);
     poisson_plan_free(s->plan);
@@ -221,6 +222,7 @@ int allocate(sd_sim* s) {
     if (!rc && isolated(s)) rc = alloc_dev(s->green, green_table_elems(S));
     if (!rc && (s->cfg.keep_density || s->mlp_on)) rc = alloc_dev(s->rho, cells);
     if (!rc && s->mlp_on) rc = alloc_dev(s->mlp_out, N);
+    if (!rc && s->mlp_on) rc = alloc_dev(s->mlp_table, cells / 2);
     s->partials_count = 8 * (gather_partials(s->N) + 1024);
     rc = rc ? rc : alloc_dev(s->partials, s->partials_count);
     rc = rc ? rc : alloc_dev(s->mom, 8);
@@ -451,7 +453,7 @@ bool keeps_rho(const sd_sim* s) { return s->rho && (s->cfg.keep_density || s->ml
 int mlp_correction(sd_sim* s, const int32_t* perm) {
     const float inv_mean = (float)((double)s->G * s->G * s->G / (double)(s->N > 0 ? s->N : 1));
     return launch_mlp_infer(s->mlp_params, s->pos, perm, s->N, s->rho, s->G, inv_mean, s->mlp_scale, s->mlp_out,
-                            s->stream);
+                            s->stream, s->mlp_table);
 }
 
 // Keys and first-pass sort counts for the current order, where the last step's
@@ -1150,6 +1152,7 @@ int sd_set_mlp(sd_sim* s, const float* params_device, float out_scale) {
     int rc = SD_OK;
     if (!s->mlp_params) rc = alloc_dev(s->mlp_params, mlp_param_count());
     if (!rc && !s->mlp_out) rc = alloc_dev(s->mlp_out, (size_t)s->N);
+    if (!rc && !s->mlp_table) rc = alloc_dev(s->mlp_table, (size_t)s->G * s->G * s->G / 2);
     if (!rc && !s->rho) rc = alloc_dev(s->rho, (size_t)s->G * s->G * s->G);
     if (rc) return rc;
     if (SD_CUDA(cudaMemcpyAsync(s->mlp_params, params_device, sizeof(float) * mlp_param_count(),

@@ -94,6 +94,7 @@ struct sd_sim {
     // learned correction (sd_set_mlp): device copy of the parameters, per-slot output
     float* mlp_params = nullptr;
     float4* mlp_out = nullptr;
+    unsigned* mlp_table = nullptr;  // density features of the step's cells, two BF16 a word
     float mlp_scale = 0.f;
     bool mlp_on = false;
 

@@ -81,6 +81,33 @@ def test_gpu_infer_matches_oracle(cuda, lib, oracle, G, n):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("G,n", [(16, 1), (16, 33), (32, 3001), (64, 95_000)])
+def test_gpu_correction_in_the_step_equals_infer(cuda, lib, G, n):
+    # the step takes its density features from a table of the cells, sd_mlp_infer forms
+    # them from the density: the same bits, so accelerations differ by exactly the inferred
+    # ones. One particle, a part tile, empty slots, cells at the box's faces.
+    from stardust_b200.learned import Correction
+    from stardust_b200.sim import Sim, SimConfig
+    pos, vel = random_particles(n, G + n, empty_every=29 if n > 40 else 0, clustered=True)
+    pos[n // 2:n // 2 + 7, :3] = np.linspace(0.0, 0.99999994, 7, dtype=np.float32)[: len(pos[n // 2:n // 2 + 7]), None]
+    params = _params(9, 0.2)
+    with Sim(0) as s:
+        s.init(SimConfig(particle_count=n, grid_size=G, softening_cells=1.0, order=L.SD_ORDER_TILED))
+        s.set_particles(pos, vel)
+        plain = s.accel()
+        s.set_correction(Correction(params, 3.0, 1.0 / G, G, 4 * G))
+        both, rho = s.accel(), s.density()
+    out = cuda.empty((n, 4), dtype=cuda.float32, device="cuda")
+    prm, pd, rd = (cuda.from_numpy(np.ascontiguousarray(a)).cuda() for a in (params, pos, rho))
+    L.check(lib.sd_mlp_infer(prm.data_ptr(), pd.data_ptr(), None, n, rd.data_ptr(), G, ctypes.c_float(G ** 3 / n),
+                             ctypes.c_float(3.0), out.data_ptr(), None), "infer")
+    extra = out.cpu().numpy()
+    live = pos[:, 0] >= 0
+    assert np.array_equal(both[live, :3], plain[live, :3] + extra[live, :3])
+    assert np.all(extra[~live] == 0)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("rows", [256, 16384])
 def test_gpu_loss_grad_matches_oracle(cuda, lib, oracle, rows):
     params = _params(11, 0.2)
