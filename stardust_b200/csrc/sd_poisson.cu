@@ -1072,11 +1072,12 @@ struct Launcher {
     static size_t smem_bal() {
         return sizeof(float2) * ((size_t)G + DepGeo<G, ISO>::kStore + (G == 512 ? xl::kTw2 : 0));
     }
-    // CTAs that take the extra shares of heavy bundles
-    template <bool ISO>
-    static int extra_ctas() {
-        const int nb = DepPlan<DepGeo<G, ISO>::M>::NB / 4;
-        return nb < 8 ? 8 : (nb > 296 ? 296 : nb);
+    // CTAs that take the extra shares of heavy bundles: one for each that there can be, so
+    // none takes two in a row. (A window of w particles has at most w / split extra shares,
+    // and a particle lies in at most four windows.) Idle ones cost little: 1.5 us for 1,024.
+    static int extra_ctas(const DepositWork& dw) {
+        const long long x = 4ll * dw.n / dw.split;
+        return (int)(x < 8 ? 8 : (x > 1184 ? 1184 : x));
     }
 
     template <bool ISO, bool WIDE>
@@ -1086,7 +1087,7 @@ struct Launcher {
         k_deposit_plan<DepGeo<G, ISO>::M, WIDE, ISO><<<P::NC, 256, 0, s>>>(
             row_start, dw.ints, dw.split, pos, dw.n, reinterpret_cast<unsigned long long*>(dw.acc));
         SD_LAUNCHED(s);
-        k_pass_a_deposit_bal<G, ISO, WIDE><<<extra_ctas<ISO>() + P::NB, kDepositThreads, smem_bal<ISO>(), s>>>(
+        k_pass_a_deposit_bal<G, ISO, WIDE><<<extra_ctas(dw) + P::NB, kDepositThreads, smem_bal<ISO>(), s>>>(
             pos, perm, row_start, keep, spec, p.tw, dw);
         SD_LAUNCHED(s);
         return SD_OK;
@@ -1238,13 +1239,15 @@ size_t deposit_work_ints(int G) {
 int* deposit_stray_flag(int* ints, int G) { return ints + deposit_work_ints(G) - 1; }
 
 int deposit_split(int n, int G, int mult) {
-    // by default ten times a window's mean particle count (a window spans 25 rows for a
-    // bundle's 16) where the grid has at least 1024 bundles, five times below that, and at
-    // least 2048: 4M particles on 256^3 (two galaxies) deposit in 0.153 ms with 10x, 0.155
-    // with 5x, 0.163 with 3x; 262,144 on 64^3 (one disk, 256 bundles) in 0.048 ms with 10x,
-    // 0.040 with 5x, 0.042 with 3x
+    // By default three times a window's mean particle count up to 256 bundles, which are
+    // resident all at once, so the time is the heaviest share's; six times at 1024, ten times
+    // above, where shares cost more than they balance (each adds its rows with global
+    // atomics); at least 2048. 262,144 particles of a disk on 64^3: 31 us with 5x, 19.5 with
+    // 3x, 19.4 with 2x; 1,000,003 on an isolated 128^3 74 us with 10x, 67 with 6x, 64 with
+    // 4x, but 2,000,000 of a ball 62, 64 and 69; 4M on 256^3 (two galaxies) 154 with 10x and
+    // 6x, 160 with 4x.
     const long long nb = (long long)G * G / 16;
-    if (mult <= 0) mult = nb >= 1024 ? 10 : 5;
+    if (mult <= 0) mult = nb <= 256 ? 3 : (nb <= 1024 ? 6 : 10);
     const long long t = (long long)mult * (long long)n / (nb > 0 ? nb : 1);
     return (int)(t < 2048 ? 2048 : (t > (1 << 30) ? (1 << 30) : t));
 }
