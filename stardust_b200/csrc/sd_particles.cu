@@ -68,6 +68,11 @@ __global__ void k_clear_u64(unsigned long long* __restrict__ a, size_t n) {
     if (i < n) a[i] = 0ull;
 }
 
+template <bool BIG>
+struct OffsetOf { using type = unsigned; };
+template <>
+struct OffsetOf<true> { using type = size_t; };
+
 // CIC-interpolated central-difference gradient of phi at p: the reference's
 // kGridAccel values (Sim.cu:604-610) sampled with sampleAcc's weights and FMA
 // order (Sim.cu:614-629). The 8 corners' 48 potential reads touch 32 distinct
@@ -75,40 +80,45 @@ __global__ void k_clear_u64(unsigned long long* __restrict__ a, size_t n) {
 //   A[oy][oz][d]  rows (iy+oy, iz+oz), x = ix-1+d, d < 4
 //   Y[e][oz][ox]  rows (iy-1+3e, iz+oz), x = ix+ox
 //   Z[e][oy][ox]  rows (iy+oy, iz-1+3e), x = ix+ox
-__device__ __forceinline__ float3 gather_accel(const float* __restrict__ phi, int G, float h, float4 p,
-                                               float* phi_at = nullptr) {
-    int ix, iy, iz;
-    float fx, fy, fz;
-    cic_axis(p.x, G, ix, fx);
-    cic_axis(p.y, G, iy, fy);
-    cic_axis(p.z, G, iz, fz);
-    const int m = G - 1;
-    const size_t G2 = (size_t)G * G;
-    int xs[4];
-#pragma unroll
-    for (int d = 0; d < 4; ++d) xs[d] = (ix - 1 + d) & m;
-    size_t ys[4], zs[4];
+// Off: byte offsets in 32 bits where the potential has at most 2^30 cells (64-bit index
+// sums took two instructions each: 0.096 -> 0.089 ms at 4M particles on 256^3, 0.391 ->
+// 0.369 at 16M on 512^3). WRAP: periodic; otherwise every index is inside the box (ix, iy,
+// iz in [1, G - 3]). Rows lie R cells apart.
+template <class Off, bool WRAP>
+__device__ __forceinline__ float3 gather_accel(const float* __restrict__ phi, int G, int R, float h, int ix, int iy,
+                                               int iz, float fx, float fy, float fz, float* phi_at) {
+    const unsigned m = G - 1;
+    const Off R4 = (Off)4 * R, RR4 = R4 * R;
+    Off xs[4], ys[4], zs[4];
 #pragma unroll
     for (int d = 0; d < 4; ++d) {
-        ys[d] = (size_t)((iy - 1 + d) & m) * G;
-        zs[d] = (size_t)((iz - 1 + d) & m) * G2;
+        const unsigned x = ix - 1 + d, y = iy - 1 + d, z = iz - 1 + d;
+        xs[d] = (Off)(WRAP ? x & m : x) * 4u;
+        ys[d] = (Off)(WRAP ? y & m : y) * R4;
+        zs[d] = (Off)(WRAP ? z & m : z) * RR4;
     }
+    const char* base = reinterpret_cast<const char*>(phi);
+    auto at = [&](Off off) { return __ldg(reinterpret_cast<const float*>(base + off)); };
     float A[2][2][4], Y[2][2][2], Z[2][2][2];
 #pragma unroll
     for (int oy = 0; oy < 2; ++oy)
 #pragma unroll
-        for (int oz = 0; oz < 2; ++oz)
+        for (int oz = 0; oz < 2; ++oz) {
+            const Off row = zs[1 + oz] + ys[1 + oy];
 #pragma unroll
-            for (int d = 0; d < 4; ++d) A[oy][oz][d] = __ldg(phi + zs[1 + oz] + ys[1 + oy] + xs[d]);
+            for (int d = 0; d < 4; ++d) A[oy][oz][d] = at(row + xs[d]);
+        }
 #pragma unroll
     for (int e = 0; e < 2; ++e)
 #pragma unroll
-        for (int o = 0; o < 2; ++o)
+        for (int o = 0; o < 2; ++o) {
+            const Off ry = zs[1 + o] + ys[3 * e], rz = zs[3 * e] + ys[1 + o];
 #pragma unroll
             for (int ox = 0; ox < 2; ++ox) {
-                Y[e][o][ox] = __ldg(phi + zs[1 + o] + ys[3 * e] + xs[1 + ox]);
-                Z[e][o][ox] = __ldg(phi + zs[3 * e] + ys[1 + o] + xs[1 + ox]);
+                Y[e][o][ox] = at(ry + xs[1 + ox]);
+                Z[e][o][ox] = at(rz + xs[1 + ox]);
             }
+        }
     float3 a = make_float3(0.f, 0.f, 0.f);
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
@@ -138,16 +148,11 @@ __device__ __forceinline__ float3 gather_accel(const float* __restrict__ phi, in
 
 // Isolated boundary (kGridAccel/sampleAcc with clamped indices, Sim.cu:589-629):
 // the potential lives in the low G^3 corner of an S^3 box (rows S apart); every
-// corner cell and its gradient neighbours are clamped to [0, G). The 8 corners'
-// 48 reads are not merged (edge clamping makes them differ); this path is not
-// the benchmark's.
-__device__ __forceinline__ float3 gather_accel_iso(const float* __restrict__ phi, int G, int S, float h, float4 p,
-                                                   float* phi_at = nullptr) {
-    int ix, iy, iz;
-    float fx, fy, fz;
-    cic_axis(p.x, G, ix, fx);
-    cic_axis(p.y, G, iy, fy);
-    cic_axis(p.z, G, iz, fz);
+// corner cell and its gradient neighbours are clamped to [0, G). Near a face the
+// clamping makes the 8 corners' 48 reads differ, so they are not merged; inside they
+// are the periodic box's 32 (1,000,003 particles on 128^3: 36 -> 28 us).
+__device__ __forceinline__ float3 gather_accel_iso(const float* __restrict__ phi, int G, int S, float h, int ix, int iy,
+                                                   int iz, float fx, float fy, float fz, float* phi_at) {
     auto at = [&](int x, int y, int z) { return __ldg(phi + ((size_t)z * S + y) * S + x); };
     float3 a = make_float3(0.f, 0.f, 0.f);
     float f = 0.f;
@@ -172,11 +177,21 @@ __device__ __forceinline__ float3 gather_accel_iso(const float* __restrict__ phi
     return a;
 }
 
-// Acceleration at p: periodic grid (S == 0) or the isolated box of side S.
-template <bool ISO>
+// Acceleration at p: periodic grid or the isolated box of side S; BIG: above 2^30 cells.
+template <bool ISO, bool BIG>
 __device__ __forceinline__ float3 accel_at(const float* __restrict__ phi, int G, int S, float h, float4 p,
                                            float* phi_at = nullptr) {
-    return ISO ? gather_accel_iso(phi, G, S, h, p, phi_at) : gather_accel(phi, G, h, p, phi_at);
+    int ix, iy, iz;
+    float fx, fy, fz;
+    cic_axis(p.x, G, ix, fx);
+    cic_axis(p.y, G, iy, fy);
+    cic_axis(p.z, G, iz, fz);
+    using Off = typename OffsetOf<BIG>::type;
+    if (!ISO) return gather_accel<Off, true>(phi, G, G, h, ix, iy, iz, fx, fy, fz, phi_at);
+    const unsigned inner = G - 3;  // 1 <= i <= G - 3 on every axis
+    if ((unsigned)(ix - 1) < inner && (unsigned)(iy - 1) < inner && (unsigned)(iz - 1) < inner)
+        return gather_accel<Off, false>(phi, G, S, h, ix, iy, iz, fx, fy, fz, phi_at);
+    return gather_accel_iso(phi, G, S, h, ix, iy, iz, fx, fy, fz, phi_at);
 }
 
 // FP64 block sums of K values into partials[blockIdx.x*K + j], fixed tree order.
@@ -246,17 +261,20 @@ __device__ __forceinline__ float3 sample_field(const float4* __restrict__ f, int
 // kKeysChanged the change bits (chg_words). Each instantiation holds only its own
 // bookkeeping: the gather runs at its register limit, and code that a launch
 // never executes still costs it.
-template <bool DIAG, bool ISO, bool PRESS, int KEYS>
+//
+// BIG: a potential of more than 2^30 cells (stage calls on a grid above 1024^3).
+template <bool DIAG, bool ISO, bool PRESS, int KEYS, bool BIG = false>
 __global__ void __launch_bounds__(kGatherThreads, 3) k_gather_kick_drift(
     const float* __restrict__ phi, int G, float h, const float4* pos_in, const float4* vel_in,
     const int* __restrict__ perm, float4* pos_out, float4* vel_out, uint32_t* __restrict__ keys_out, int order, int n,
     float dt_kick, float dt_drift, float c2, const float* __restrict__ mean_vel, double* __restrict__ partials,
     const float4* __restrict__ extra, int S, unsigned* __restrict__ tile_counts, int count_bits,
     const float4* __restrict__ press, unsigned* __restrict__ chg_words) {
-    // Per-thread FP64 sums (momentum, count; with DIAG |v|^2 and phi), each in the
-    // thread's own shared-memory slot: held in registers they crowd out the stencil's
-    // loads at the kernel's register limit. The summation order is the same.
-    __shared__ double acc[6][kGatherThreads];
+    // Per-thread FP64 sums: momentum and, with DIAG, |v|^2 and phi, each in the thread's own
+    // shared-memory slot: held in registers they crowd out the stencil's loads at the
+    // kernel's register limit. The count is an integer. The summation order is the same.
+    __shared__ double acc[5][kGatherThreads];
+    int live = 0;
     // Software pipeline over the grid-stride loop: the records (pos, vel) of this
     // thread's next kAhead particles are in flight into its own shared-memory slots
     // (cp.async, one copy group per particle), and the permutation index of the
@@ -267,7 +285,7 @@ __global__ void __launch_bounds__(kGatherThreads, 3) k_gather_kick_drift(
     __shared__ float4 rec[kAhead + 1][2][kGatherThreads];
     const int me = threadIdx.x;
 #pragma unroll
-    for (int q = 0; q < 6; ++q) acc[q][me] = 0.0;
+    for (int q = 0; q < 5; ++q) acc[q][me] = 0.0;
     const unsigned cmask = (1u << count_bits) - 1u;
     const float mx = mean_vel ? mean_vel[0] : 0.f, my = mean_vel ? mean_vel[1] : 0.f,
                 mz = mean_vel ? mean_vel[2] : 0.f;
@@ -318,7 +336,7 @@ __global__ void __launch_bounds__(kGatherThreads, 3) k_gather_kick_drift(
                 v.z = __fsub_rn(v.z, mz);
             }
             float phi_p = 0.f;
-            float3 a = accel_at<ISO>(phi, G, S, h, p, DIAG ? &phi_p : nullptr);
+            float3 a = accel_at<ISO, BIG>(phi, G, S, h, p, DIAG ? &phi_p : nullptr);
             if (extra) {  // learned correction, indexed like the outputs
                 const float4 e = extra[i];
                 a.x = __fadd_rn(a.x, e.x);
@@ -376,10 +394,10 @@ __global__ void __launch_bounds__(kGatherThreads, 3) k_gather_kick_drift(
             acc[0][me] += v.x;
             acc[1][me] += v.y;
             acc[2][me] += v.z;
-            acc[3][me] += 1.0;
+            ++live;
             if (DIAG) {
-                acc[4][me] += (double)v.x * v.x + (double)v.y * v.y + (double)v.z * v.z;
-                acc[5][me] += (double)phi_p;
+                acc[3][me] += (double)v.x * v.x + (double)v.y * v.y + (double)v.z * v.z;
+                acc[4][me] += (double)phi_p;
             }
         } while (0);
         // The change bit of output i for the next step's merge sort: one word per
@@ -400,10 +418,10 @@ __global__ void __launch_bounds__(kGatherThreads, 3) k_gather_kick_drift(
     }
     if (partials) {
         if (DIAG) {
-            double v6[6] = {acc[0][me], acc[1][me], acc[2][me], acc[3][me], acc[4][me], acc[5][me]};
+            double v6[6] = {acc[0][me], acc[1][me], acc[2][me], (double)live, acc[3][me], acc[4][me]};
             block_sum<6>(v6, partials);
         } else {
-            double v4[4] = {acc[0][me], acc[1][me], acc[2][me], acc[3][me]};
+            double v4[4] = {acc[0][me], acc[1][me], acc[2][me], (double)live};
             block_sum<4>(v4, partials);
         }
     }
@@ -473,7 +491,9 @@ __global__ void __launch_bounds__(256) k_interpolate_accel(const float* __restri
         acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         return;
     }
-    float3 a = S ? gather_accel_iso(phi, G, S, h, p) : gather_accel(phi, G, h, p);
+    const float3 g = S ? accel_at<true, false>(phi, G, S, h, p)
+                       : (G > 1024 ? accel_at<false, true>(phi, G, 0, h, p) : accel_at<false, false>(phi, G, 0, h, p));
+    float3 a = g;
     if (extra) {
         const float4 e = extra[i];
         a.x = __fadd_rn(a.x, e.x);
@@ -771,7 +791,12 @@ int launch_gather_kick_drift(const float* phi, int G, float pot_scale, const flo
 #define SD_GATHER_P(D, I)                \
     if (press) { SD_GATHER_K(D, I, true); } \
     else { SD_GATHER_K(D, I, false); }
-    if (iso_S) {
+    if (!iso_S && G > 1024) {  // the simulation's grids end at 512: a stage call, plain
+        if (dg || press || keys_mode != kKeysPlain) return fail(SD_E_UNSUPPORTED, "gather: grid %d above 1024", G);
+        k_gather_kick_drift<false, false, false, kKeysPlain, true><<<blocks, kGatherThreads, 0, s>>>(
+            phi, G, h, pos_in, vel_in, perm, pos_out, vel_out, keys_out, order, n, dt_kick, dt_drift, c2, mean_vel,
+            partials, extra, iso_S, tile_counts, count_bits, press, chg_words);
+    } else if (iso_S) {
         if (dg) { SD_GATHER_P(true, true); }
         else { SD_GATHER_P(false, true); }
     } else {

@@ -51,6 +51,21 @@ def test_isolated_potential_and_accel_match_fp64(cuda, oracle, G):
     assert rel_rms(a, a64) < 5e-5
 
 
+@pytest.mark.parametrize("G", [16, 32])
+def test_isolated_accel_at_every_edge_cell(cuda, oracle, G):
+    # coordinates in the first and last four cells and their halves, in every combination:
+    # where clamping changes a stencil and where the merged one takes over. FP32 bound as above.
+    e = np.concatenate([(np.arange(8) + 0.25) / (2 * G), 1 - (np.arange(8) + 0.25) / (2 * G), [0.5]])
+    x = np.stack(np.meshgrid(e, e, e, indexing="ij"), -1).reshape(-1, 3)
+    n = len(x)
+    pos = np.zeros((n, 4), np.float32)
+    pos[:, :3] = x
+    with iso_sim(n, G) as s:
+        s.set_particles(pos, np.zeros_like(pos))
+        a = s.accel()[:, :3]
+    assert rel_rms(a, oracle.pm_accel_iso_f64(pos, G, 1.0 / n, 1.5)) < 5e-5
+
+
 @pytest.mark.parametrize("G", [16, 128, 256])
 def test_isolated_transform_sizes(cuda, oracle, G):
     # the smallest and the largest transform boxes, 2 G a side: the parts of the lines
