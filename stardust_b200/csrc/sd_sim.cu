@@ -495,12 +495,38 @@ int do_sort(sd_sim* s, int32_t* perm_out_dev) {
 }
 
 // Field for the current positions: deposit + Poisson -> phi (computeAccel, Sim.cu:3605-3633).
+// On a 512^3 grid the particles are sorted by tiled row for it, so that pass A deposits
+// them itself: the int64 grid, 1 GB to read and clear again, costs more than the sort
+// (2,097,152 particles: atomics and pass A 0.64 ms, keys, sort and fused deposit 0.46).
+// Smaller grids come out even or worse.
 int do_field(sd_sim* s, bool keep) {
-    int rc = launch_deposit_fixed(s->pos, s->N, s->G, s->acc, s->stream, isolated(s) ? 0 : 1);
-    if (rc) return rc;
+    int rc = SD_OK;
+    const bool fused = !isolated(s) && s->G == 512;
+    DepositWork dw;
+    int* rows = nullptr;
+    if (fused) {
+        const bool have = s->keys_valid && s->cfg.order == SD_ORDER_TILED;
+        // the other set's velocities are free between steps
+        uint32_t* keys = have ? s->keys : reinterpret_cast<uint32_t*>(s->vel2);
+        if (!have && (rc = launch_cell_keys(s->pos, s->N, s->G, SD_ORDER_TILED, keys, s->stream))) return rc;
+        rc = launch_sort_pairs(keys, nullptr, s->keys2, s->vals, s->keys3, s->vals2, s->N,
+                               key_bits_for(s->G, SD_ORDER_TILED), s->sort_ws, s->sort_ws_bytes, s->stream, true);
+        if (rc) return rc;
+        s->counts_valid = false;  // the step's first-pass counts were in the workspace
+        // a merge of the next step needs the row table of the last one
+        rows = s->rs_base ? s->rs.c_rows : s->row_start;
+        if ((rc = launch_row_bounds(s->keys2, s->N, row_last(s->G, SD_ORDER_TILED), -1, rows, s->stream))) return rc;
+        dw.acc = s->acc;
+        dw.ints = s->dep_ints;
+        dw.split = deposit_split(s->N, s->G);
+        dw.n = s->N;
+    } else if ((rc = launch_deposit_fixed(s->pos, s->N, s->G, s->acc, s->stream, isolated(s) ? 0 : 1))) {
+        return rc;
+    }
     PoissonIso io;
-    rc = launch_poisson_ex(s->plan, s->acc, nullptr, nullptr, nullptr, nullptr, keep ? s->rho : nullptr, s->spec,
-                           s->phi, s->stream, nullptr, iso_opts(s, io));
+    rc = launch_poisson_ex(s->plan, fused ? nullptr : s->acc, nullptr, fused ? s->pos : nullptr,
+                           fused ? s->vals : nullptr, rows, keep ? s->rho : nullptr, s->spec, s->phi, s->stream, nullptr,
+                           iso_opts(s, io), &dw);
     if (rc) return rc;
     if (keep) s->rho_valid = true;
     return SD_OK;

@@ -263,6 +263,36 @@ def test_fused_deposit_equals_atomic_deposit(cuda, boundary, order, G, n, cluste
         assert np.array_equal(a.view(np.int32), b.view(np.int32))
 
 
+@pytest.mark.parametrize("order,full_sort", [(L.SD_ORDER_TILED, -1), (L.SD_ORDER_TILED, 1), (L.SD_ORDER_ROWMAJOR, -1),
+                                             (L.SD_ORDER_MORTON, 0)])
+def test_field_on_512_between_steps(cuda, order, full_sort):
+    """On 512^3 the field of the current positions sorts them for the fused deposit, in
+    buffers that the steps use too: density as the atomic deposit's, bit for bit, and the
+    steps around it as if it had not been asked for (merges, counts and keys included)."""
+    G, n = 512, 150_001
+    pos, vel = random_particles(n, 77, empty_every=53, clustered=True)
+    vel[:, 3] = np.arange(n, dtype=np.float32)
+    got = []
+    for ask in (True, False):
+        with make_sim(cuda, n, G, gravity=5.0, softening_cells=1.0, order=order, full_sort=full_sort) as s:
+            s.set_particles(pos, vel)
+            if ask:
+                a0, rho = s.accel(), s.density()
+                assert np.array_equal(s.accel(), a0)
+            s.steps(1e-3, 3)
+            if ask:
+                s.accel()
+            s.steps(1e-3, 2)
+            s.step(1e-3)
+            got.append(s.get_particles())
+    assert np.array_equal(got[0][0].view(np.int32), got[1][0].view(np.int32))
+    assert np.array_equal(got[0][1].view(np.int32), got[1][1].view(np.int32))
+    w = cuda.empty(int(L.lib().sd_deposit_workspace_bytes(G)), dtype=cuda.uint8, device="cuda")
+    pd, ref = cuda.from_numpy(pos).cuda(), cuda.empty((G, G, G), dtype=cuda.float32, device="cuda")
+    L.check(L.lib().sd_deposit(pd.data_ptr(), n, G, ref.data_ptr(), w.data_ptr(), w.numel(), None), "deposit")
+    assert np.array_equal(rho, ref.cpu().numpy())
+
+
 def test_tiled_graph_replay_matches_eager(cuda):
     G, n = 64, 150_000
     pos, vel = random_particles(n, 12, clustered=True)
