@@ -327,6 +327,7 @@ __global__ void __launch_bounds__(kPassAThreads<G>, G == 512 ? 3 : 0)
 //   arrive[NB]   CTAs of a shared bundle done so far (zero between uses)
 //   cta_sum[NC], cta_pre[NC + 1]   per-block totals and their exclusive prefix
 //   plan_done    blocks of the plan kernel done (zero between uses)
+//   ticket       next work item of the deposit's CTAs, past their first ones
 //   use          nonzero: this use deposits from the fixed-point grid (see stray)
 //   stray        nonzero: a particle sits where its row's windows do not reach (set where
 //                keys are made, launch_cell_keys; cleared by the next plan)
@@ -335,7 +336,7 @@ struct DepPlan {
     static constexpr int NB = G * G / 16;
     static constexpr int NC = (NB + 255) / 256;
     static constexpr int kItems = 0, kXpre = NB, kArrive = 2 * NB, kCtaSum = 3 * NB, kCtaPre = 3 * NB + NC,
-                         kDone = 3 * NB + 2 * NC + 1, kUse = kDone + 1, kStray = kUse + 1, kInts = kStray + 1;
+                         kDone = 3 * NB + 2 * NC + 1, kTicket = kDone + 1, kUse = kTicket + 1, kStray = kUse + 1, kInts = kStray + 1;
 };
 
 // Where the particles of a bundle's window sit among the sorted ones, as kRanges
@@ -479,6 +480,7 @@ __global__ void __launch_bounds__(256) k_deposit_plan(const int* __restrict__ rs
     if (threadIdx.x == 0) {
         w[P::kCtaPre + P::NC] = all;
         w[P::kDone] = 0;
+        w[P::kTicket] = 0;
         if (kMayStray) {  // every block has read the flag
             w[P::kUse] = stray;
             w[P::kStray] = 0;
@@ -504,12 +506,17 @@ struct DepGeo {
     static constexpr int kStore = G == 512 ? (kWarp > kSums ? kWarp : kSums) : (kLines > kSums ? kLines : kSums);
 };
 
+template <int G>
+constexpr bool kDepositLoop = G == 512;
+template <int G>
+constexpr int kDepositPerSm = G >= 128 ? 3 : 2;
+
 template <int G, bool ISO, bool WIDE, bool SHARED>
 __device__ __forceinline__ void deposit_bundle(int b, int slice, int items, const float4* __restrict__ pos,
                                                const int* __restrict__ perm, const int* __restrict__ row_start,
                                                float* __restrict__ rho_keep, float2* __restrict__ spec,
-                                               const DepositWork& w, unsigned* __restrict__ arrive, bool reuse,
-                                               bool from_grid) {
+                                               const DepositWork& w, unsigned* __restrict__ arrive,
+                                               int* __restrict__ ticket, int* s_next, bool reuse, bool from_grid) {
     using T = Geo<G>;
     using D = DepGeo<G, ISO>;
     constexpr int M = D::M, NR = kRanges<WIDE>;
@@ -551,6 +558,8 @@ __device__ __forceinline__ void deposit_bundle(int b, int slice, int items, cons
         if (j == 0) r_off[0] = 0;
     }
     __syncthreads();
+    // the CTA's next work item, read after later barriers
+    if (kDepositLoop<G> && threadIdx.x == 0) *s_next = atomicAdd(ticket, 1) + (int)gridDim.x;
     const int total = from_grid ? 0 : r_off[NR];  // from_grid: the sums are in the fixed-point grid
     const int f_lo = SHARED ? (int)((long long)total * slice / items) : 0;
     const int f_hi = SHARED ? (int)((long long)total * (slice + 1) / items) : total;
@@ -784,33 +793,34 @@ __device__ __forceinline__ void deposit_bundle(int b, int slice, int items, cons
     }
 }
 
-// Grid: X CTAs that take the extra shares of heavy bundles (first, so they start
-// early), then one CTA per bundle for its first share. 40 registers at G = 512
-// keep three 70 KB CTAs per SM; smaller grids need more for their FFT stages.
+// Work items: the extra shares of heavy bundles (first, so they start early), then one
+// item per bundle for its first share. At G = 512 as many CTAs as are resident take them by
+// ticket: a CTA's twiddles (8 KB with their tables) are loaded once and its next item is
+// known while it works (16M particles 0.471 -> 0.445 ms, 2M 0.394 -> 0.360). Smaller grids
+// take a CTA per item: the loop's registers are spilled there (4M on 256^3 0.153 against
+// 0.181 ms, 2M on 128^3 0.062 against 0.074). 40 registers from 128^3 up keep three CTAs
+// per SM; smaller grids need more for their FFT stages.
 template <int G, bool ISO, bool WIDE>
-__global__ void __launch_bounds__(kDepositThreads, G >= 128 ? 3 : 2)
+__global__ void __launch_bounds__(kDepositThreads, kDepositPerSm<G>)
     k_pass_a_deposit_bal(const float4* __restrict__ pos, const int* __restrict__ perm,
                          const int* __restrict__ row_start, float* __restrict__ rho_keep, float2* __restrict__ spec,
                          const float2* __restrict__ tw_g, DepositWork w) {
     using P = DepPlan<DepGeo<G, ISO>::M>;
     extern __shared__ float2 sm[];
+    __shared__ int s_next;
     const int* items = w.ints + P::kItems;
     const int* xpre = w.ints + P::kXpre;
     const int* cta_pre = w.ints + P::kCtaPre;
     unsigned* arrive = reinterpret_cast<unsigned*>(w.ints + P::kArrive);
-    const int X = (int)gridDim.x - P::NB;
     const bool from_grid = WIDE != ISO && w.ints[P::kUse] != 0;
-    const bool first = (int)blockIdx.x >= X;  // a bundle's first share, then done
-    const int extras = first ? 0 : cta_pre[P::NC];
-    if (!first && (int)blockIdx.x >= extras) return;  // no extra share for this CTA
+    const int extras = cta_pre[P::NC];
+    if ((int)blockIdx.x >= extras + P::NB) return;  // fewer extra shares than there can be
     for (int i = threadIdx.x; i < G; i += kDepositThreads) sm[i] = tw_g[i];  // ordered by a later barrier
     if constexpr (G == 512) xl::fill_twiddles(sm + G + DepGeo<G, ISO>::kStore, tw_g);  // the twiddle tables, after the sums
-    for (int e = first ? 0 : (int)blockIdx.x; first || e < extras; e += X) {
-        int b, slice;
-        if (first) {
-            b = (int)blockIdx.x - X;
-            slice = 0;
-        } else {
+    bool reuse = false;
+    for (int e = blockIdx.x; e < extras + P::NB; e = s_next, reuse = true) {
+        int b = e - extras, slice = 0;
+        if (e < extras) {
             // the bundle of extra share e: the last b whose extras start at or before e
             int lo = 0, hi = P::NB - 1;
             while (lo < hi) {
@@ -828,11 +838,11 @@ __global__ void __launch_bounds__(kDepositThreads, G >= 128 ? 3 : 2)
         const int nb = items[b];
         if (G >= 512 && nb == 1 && !from_grid)
             deposit_bundle<G, ISO, WIDE, false>(b, 0, 1, pos, perm, row_start, rho_keep, spec, w, arrive,
-                                                !first && e != (int)blockIdx.x, false);
+                                                w.ints + P::kTicket, &s_next, reuse, false);
         else
             deposit_bundle<G, ISO, WIDE, true>(b, slice, nb, pos, perm, row_start, rho_keep, spec, w, arrive,
-                                               !first && e != (int)blockIdx.x, from_grid);
-        if (first) break;
+                                               w.ints + P::kTicket, &s_next, reuse, from_grid);
+        if (!kDepositLoop<G>) break;
     }
 }
 
@@ -1081,14 +1091,6 @@ struct Launcher {
     static size_t smem_bal() {
         return sizeof(float2) * ((size_t)G + DepGeo<G, ISO>::kStore + (G == 512 ? xl::kTw2 : 0));
     }
-    // CTAs that take the extra shares of heavy bundles: one for each that there can be, so
-    // none takes two in a row. (A window of w particles has at most w / split extra shares,
-    // and a particle lies in at most four windows.) Idle ones cost little: 1.5 us for 1,024.
-    static int extra_ctas(const DepositWork& dw) {
-        const long long x = 4ll * dw.n / dw.split;
-        return (int)(x < 8 ? 8 : (x > 1184 ? 1184 : x));
-    }
-
     template <bool ISO, bool WIDE>
     static int deposit(const PoissonPlan& p, const float4* pos, const int* perm, const int* row_start, float* keep,
                        float2* spec, const DepositWork& dw, cudaStream_t s) {
@@ -1096,8 +1098,13 @@ struct Launcher {
         k_deposit_plan<DepGeo<G, ISO>::M, WIDE, ISO><<<P::NC, 256, 0, s>>>(
             row_start, dw.ints, dw.split, pos, dw.n, reinterpret_cast<unsigned long long*>(dw.acc));
         SD_LAUNCHED(s);
-        k_pass_a_deposit_bal<G, ISO, WIDE><<<extra_ctas(dw) + P::NB, kDepositThreads, smem_bal<ISO>(), s>>>(
-            pos, perm, row_start, keep, spec, p.tw, dw);
+        // a CTA for each extra share that there can be, so none waits for another (a window of
+        // w particles has at most w / split extra shares, and a particle lies in at most four
+        // windows); idle ones cost little, 1.5 us for 1,024. Never more than are taken by ticket.
+        const long long extra = 4ll * dw.n / dw.split, wave = 148 * kDepositPerSm<G>;
+        const long long ctas = P::NB + (extra < 8 ? 8 : extra);
+        k_pass_a_deposit_bal<G, ISO, WIDE><<<(unsigned)(kDepositLoop<G> && ctas > wave ? wave : ctas), kDepositThreads,
+                                             smem_bal<ISO>(), s>>>(pos, perm, row_start, keep, spec, p.tw, dw);
         SD_LAUNCHED(s);
         return SD_OK;
     }
