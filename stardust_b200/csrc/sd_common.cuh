@@ -14,6 +14,11 @@
 
 namespace sd {
 
+// First statement of every kernel that launch() (sd_internal.h) starts: waits until the
+// kernels before it in the stream are done and their writes can be seen. None of them
+// lets the next one start early, so all of their blocks have left by then.
+__device__ __forceinline__ void wait_previous() { cudaGridDependencySynchronize(); }
+
 // CIC base cell and fraction along one axis: g = p*G - 1/2 (kScatter, Sim.cu:509-511).
 __device__ __forceinline__ void cic_axis(float p, int G, int& i, float& f) {
     const float g = __fmaf_rn(p, (float)G, -0.5f);

@@ -83,6 +83,7 @@ __device__ __forceinline__ float cell_feature(float r, float inv_mean) {
 // read each cell's many times (four cells a thread; the grid's side is a multiple of 16).
 __global__ void __launch_bounds__(256) k_feature_table(const float4* __restrict__ rho, size_t quads, float inv_mean,
                                                        uint2* __restrict__ table) {
+    wait_previous();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= quads) return;
     const float4 r = rho[i];
@@ -150,6 +151,7 @@ __device__ __forceinline__ void table_features(const unsigned* __restrict__ tabl
 
 __global__ void k_features(const float4* __restrict__ pos, const int* __restrict__ perm, int n,
                            const float* __restrict__ rho, int G, float inv_mean, __nv_bfloat16* __restrict__ out) {
+    wait_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 p = pos[perm ? perm[i] : i];
@@ -253,6 +255,7 @@ __global__ void __launch_bounds__(inf::kThreads, inf::kCtasPerSm)
     k_mlp_infer(const float* __restrict__ params, const float4* __restrict__ pos, const int* __restrict__ perm, int n,
                 const float* __restrict__ rho, const unsigned* __restrict__ table, int G, float inv_mean,
                 float out_scale, float4* __restrict__ out) {
+    wait_previous();
     __shared__ __align__(16) inf::Smem s;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
     // the same BF16 rounding of the weights as the training's copies
@@ -458,6 +461,7 @@ __global__ void __launch_bounds__(tr::kThreads, 1) k_train_tile(const float* __r
                                                                 const __nv_bfloat16* __restrict__ X,
                                                                 const float* __restrict__ tgt, int rows,
                                                                 float* __restrict__ part) {
+    wait_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     tr::Smem& s = *reinterpret_cast<tr::Smem*>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
@@ -652,6 +656,7 @@ __global__ void __launch_bounds__(tr::kThreads, 1) k_train_tile(const float* __r
 // them each; *sse from the entry after the gradient.
 __global__ void __launch_bounds__(256) k_train_reduce(const float* __restrict__ part, int parts,
                                                       float* __restrict__ grad, float* __restrict__ sse) {
+    wait_previous();
     __shared__ float red[4][64];
     const int c = threadIdx.x & 63, q = threadIdx.x >> 6, i = blockIdx.x * 64 + c;
     const int per = (parts + 3) / 4, p0 = q * per, p1 = min(parts, p0 + per);
@@ -673,6 +678,7 @@ __global__ void k_adam(
 float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
                        const float* __restrict__ grad, int n, float lr, float b1, float b2, float eps, float c1,
                        float c2) {
+    wait_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float g = grad[i];
@@ -694,13 +700,13 @@ int launch_mlp_infer(const float* params, const float4* pos, const int* perm, in
     const int blocks = need < wave ? need : wave;
     if (table) {
         const size_t quads = (size_t)G * G * G / 4;
-        k_feature_table<<<(unsigned)((quads + 255) / 256), 256, 0, s>>>(reinterpret_cast<const float4*>(rho), quads,
+        launch(k_feature_table, (unsigned)((quads + 255) / 256), 256, 0, s, reinterpret_cast<const float4*>(rho), quads,
                                                                         inv_mean, reinterpret_cast<uint2*>(table));
         SD_LAUNCHED(s);
-        k_mlp_infer<true><<<blocks, inf::kThreads, 0, s>>>(params, pos, perm, n, rho, table, G, inv_mean, out_scale,
+        launch(k_mlp_infer<true>, blocks, inf::kThreads, 0, s, params, pos, perm, n, rho, table, G, inv_mean, out_scale,
                                                            out);
     } else {
-        k_mlp_infer<false><<<blocks, inf::kThreads, 0, s>>>(params, pos, perm, n, rho, nullptr, G, inv_mean, out_scale,
+        launch(k_mlp_infer<false>, blocks, inf::kThreads, 0, s, params, pos, perm, n, rho, nullptr, G, inv_mean, out_scale,
                                                             out);
     }
     SD_LAUNCHED(s);
@@ -731,7 +737,7 @@ int sd_mlp_features(const float* pos, const int32_t* perm, int n, const float* r
         return fail(SD_E_ARG, "mlp_features: bad arguments");
     if (n == 0) return SD_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    k_features<<<(n + 255) / 256, 256, 0, st>>>(reinterpret_cast<const float4*>(pos), perm, n, rho, G, inv_mean,
+    launch(k_features, (n + 255) / 256, 256, 0, st, reinterpret_cast<const float4*>(pos), perm, n, rho, G, inv_mean,
                                                  reinterpret_cast<__nv_bfloat16*>(features_bf16));
     SD_LAUNCHED(st);
     return SD_OK;
@@ -764,10 +770,10 @@ int sd_mlp_loss_grad(const float* params, const void* features_bf16, const float
     // the shared-memory limit is per device, so it is set on each call (a host-side look-up)
     if (SD_CUDA(cudaFuncSetAttribute(k_train_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(tr::Smem))))
         return SD_E_CUDA;
-    k_train_tile<<<ctas, tr::kThreads, sizeof(tr::Smem), st>>>(
+    launch(k_train_tile, ctas, tr::kThreads, sizeof(tr::Smem), st,
         params, reinterpret_cast<const __nv_bfloat16*>(features_bf16), targets, rows, part);
     SD_LAUNCHED(st);
-    k_train_reduce<<<(kParams + 1 + 63) / 64, 256, 0, st>>>(part, ctas, grad, sse);
+    launch(k_train_reduce, (kParams + 1 + 63) / 64, 256, 0, st, part, ctas, grad, sse);
     SD_LAUNCHED(st);
     return SD_OK;
 }
@@ -777,7 +783,7 @@ int sd_mlp_adam(float* params, float* m, float* v, const float* grad, int step, 
     if (!params || !m || !v || !grad || step < 1) return fail(SD_E_ARG, "mlp_adam: bad arguments");
     cudaStream_t st = (cudaStream_t)stream;
     const float c1 = 1.f / (1.f - powf(beta1, (float)step)), c2 = 1.f / (1.f - powf(beta2, (float)step));
-    k_adam<<<(kParams + 255) / 256, 256, 0, st>>>(params, m, v, grad, kParams, lr, beta1, beta2, eps, c1, c2);
+    launch(k_adam, (kParams + 255) / 256, 256, 0, st, params, m, v, grad, kParams, lr, beta1, beta2, eps, c1, c2);
     SD_LAUNCHED(st);
     return SD_OK;
 }

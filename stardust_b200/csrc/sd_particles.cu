@@ -51,12 +51,14 @@ constexpr int kAhead = 1;
 
 __global__ void __launch_bounds__(256) k_deposit_fixed(const float4* __restrict__ pos, int n, int G,
                                                        unsigned long long* __restrict__ acc, int periodic) {
+    wait_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     deposit_particle(pos[i], G, acc, periodic);
 }
 
 __global__ void k_fixed_to_float(long long* __restrict__ acc, size_t cells, float* __restrict__ rho, int clear) {
+    wait_previous();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= cells) return;
     rho[i] = fixed_to_float(acc[i]);
@@ -64,6 +66,7 @@ __global__ void k_fixed_to_float(long long* __restrict__ acc, size_t cells, floa
 }
 
 __global__ void k_clear_u64(unsigned long long* __restrict__ a, size_t n) {
+    wait_previous();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) a[i] = 0ull;
 }
@@ -270,6 +273,7 @@ __global__ void __launch_bounds__(kGatherThreads, 3) k_gather_kick_drift(
     float dt_kick, float dt_drift, float c2, const float* __restrict__ mean_vel, double* __restrict__ partials,
     const float4* __restrict__ extra, int S, unsigned* __restrict__ tile_counts, int count_bits,
     const float4* __restrict__ press, unsigned* __restrict__ chg_words) {
+    wait_previous();
     // Per-thread FP64 sums: momentum and, with DIAG, |v|^2 and phi, each in the thread's own
     // shared-memory slot: held in registers they crowd out the stencil's loads at the
     // kernel's register limit. The count is an integer. The summation order is the same.
@@ -438,6 +442,7 @@ __global__ void __launch_bounds__(256) k_finalize_mean(const double* __restrict_
                                                        double* __restrict__ mom_out, float* __restrict__ mean_out,
                                                        double* __restrict__ rec, unsigned long long* __restrict__ rec_n,
                                                        int cap, double mass, double pot_scale) {
+    wait_previous();
     __shared__ double red[K][256];
     double s[K];
 #pragma unroll
@@ -484,6 +489,7 @@ __global__ void __launch_bounds__(256) k_finalize_mean(const double* __restrict_
 __global__ void __launch_bounds__(256) k_interpolate_accel(const float* __restrict__ phi, int G, float h,
                                                            const float4* __restrict__ pos, float4* __restrict__ acc,
                                                            int n, const float4* __restrict__ extra, int S) {
+    wait_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 p = pos[i];
@@ -505,6 +511,7 @@ __global__ void __launch_bounds__(256) k_interpolate_accel(const float* __restri
 
 __global__ void k_apply_mean(float4* __restrict__ vel, const float4* __restrict__ pos, int n,
                              const float* __restrict__ mean_vel) {
+    wait_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n || pos[i].x < 0.f) return;
     float4 v = vel[i];
@@ -521,6 +528,7 @@ constexpr int kSpeedCtasPerSm = 8;
 __global__ void __launch_bounds__(256) k_max_speed(const float4* __restrict__ pos, const float4* __restrict__ vel,
                                                    int n, const float* __restrict__ mean_vel,
                                                    float* __restrict__ out) {
+    wait_previous();
     const float mx = mean_vel ? mean_vel[0] : 0.f, my = mean_vel ? mean_vel[1] : 0.f,
                 mz = mean_vel ? mean_vel[2] : 0.f;
     float s = 0.f;
@@ -567,6 +575,7 @@ __global__ void __launch_bounds__(kGatherThreads) k_energy(const float* __restri
                                                            const float4* __restrict__ vel, int n,
                                                            const float* __restrict__ mean_vel,
                                                            double* __restrict__ partials, int S) {
+    wait_previous();
     double ke = 0.0, pe = 0.0, px = 0.0, py = 0.0, pz = 0.0, c = 0.0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float4 p = pos[i];
@@ -620,6 +629,7 @@ __global__ void __launch_bounds__(kGatherThreads) k_energy(const float* __restri
 
 __global__ void __launch_bounds__(256) k_finalize8(const double* __restrict__ partials, int blocks,
                                                    double* __restrict__ out) {
+    wait_previous();
     __shared__ double red[8][256];
     double s[8];
 #pragma unroll
@@ -642,6 +652,7 @@ __global__ void __launch_bounds__(256) k_finalize8(const double* __restrict__ pa
 // op 0: sum, 1: max. Grid-stride, 8 partial doubles per block slot (only [0] used).
 __global__ void __launch_bounds__(256) k_reduce_grid(const float* __restrict__ a, size_t n, int op,
                                                      double* __restrict__ partials) {
+    wait_previous();
     double acc = (op == 1) ? -INFINITY : 0.0;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const double v = (op == 2) ? (a[i] > 1e-6f ? 1.0 : 0.0) : (double)a[i];
@@ -659,6 +670,7 @@ __global__ void __launch_bounds__(256) k_reduce_grid(const float* __restrict__ a
 }
 
 __global__ void k_reduce_final(const double* __restrict__ partials, int blocks, int op, double* __restrict__ out) {
+    wait_previous();
     if (threadIdx.x != 0) return;
     double acc = (op == 1) ? -INFINITY : 0.0;
     for (int b = 0; b < blocks; ++b) acc = (op == 1) ? fmax(acc, partials[b]) : acc + partials[b];
@@ -668,6 +680,7 @@ __global__ void k_reduce_final(const double* __restrict__ partials, int blocks, 
 // Per-block sums of x, y and the count of live particles (pos.x >= 0), then one
 // thread adds the block sums in block order: the result does not depend on timing.
 __global__ void __launch_bounds__(256) k_centroid(const float4* __restrict__ pos, int n, double* __restrict__ partials) {
+    wait_previous();
     double sx = 0.0, sy = 0.0, c = 0.0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float4 p = pos[i];
@@ -690,6 +703,7 @@ __global__ void __launch_bounds__(256) k_centroid(const float4* __restrict__ pos
 }
 
 __global__ void k_centroid_final(const double* __restrict__ partials, int blocks, double* __restrict__ out) {
+    wait_previous();
     if (threadIdx.x >= 3) return;
     double acc = 0.0;
     for (int b = 0; b < blocks; ++b) acc += partials[3 * b + threadIdx.x];
@@ -697,6 +711,7 @@ __global__ void k_centroid_final(const double* __restrict__ partials, int blocks
 }
 
 __global__ void k_hide_range(float4* __restrict__ pos, float4* __restrict__ vel, int from, int to) {
+    wait_previous();
     const int i = from + blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= to) return;
     pos[i] = make_float4(-1.f, -1.f, -1.f, 0.f);
@@ -709,21 +724,21 @@ size_t deposit_workspace_bytes(int G) { return align_up(sizeof(long long) * (siz
 
 int launch_deposit_fixed(const float4* pos, int n, int G, long long* acc, cudaStream_t s, int periodic) {
     if (n <= 0) return SD_OK;
-    k_deposit_fixed<<<(n + 255) / 256, 256, 0, s>>>(pos, n, G, reinterpret_cast<unsigned long long*>(acc),
+    launch(k_deposit_fixed, (n + 255) / 256, 256, 0, s, pos, n, G, reinterpret_cast<unsigned long long*>(acc),
                                                      periodic);
     SD_LAUNCHED(s);
     return SD_OK;
 }
 
 int launch_clear_u64(long long* a, size_t n, cudaStream_t s) {
-    k_clear_u64<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(reinterpret_cast<unsigned long long*>(a), n);
+    launch(k_clear_u64, (unsigned)((n + 255) / 256), 256, 0, s, reinterpret_cast<unsigned long long*>(a), n);
     SD_LAUNCHED(s);
     return SD_OK;
 }
 
 int launch_fixed_to_float(const long long* acc, int G, float* rho, int clear, cudaStream_t s) {
     const size_t cells = (size_t)G * G * G;
-    k_fixed_to_float<<<(unsigned)((cells + 255) / 256), 256, 0, s>>>(const_cast<long long*>(acc), cells, rho, clear);
+    launch(k_fixed_to_float, (unsigned)((cells + 255) / 256), 256, 0, s, const_cast<long long*>(acc), cells, rho, clear);
     SD_LAUNCHED(s);
     return SD_OK;
 }
@@ -781,7 +796,7 @@ int launch_gather_kick_drift(const float* phi, int G, float pot_scale, const flo
         return fail(SD_E_ARG, "gather: change bits need keys, no tile counts and the periodic box");
     const int keys_mode = chg_words ? kKeysChanged : (tile_counts ? kKeysCounts : kKeysPlain);
 #define SD_GATHER(D, I, P, K)                                                                              \
-    k_gather_kick_drift<D, I, P, K><<<blocks, kGatherThreads, 0, s>>>(                                         \
+    launch(k_gather_kick_drift<D, I, P, K>, blocks, kGatherThreads, 0, s,                                          \
         phi, G, h, pos_in, vel_in, perm, pos_out, vel_out, keys_out, order, n, dt_kick, dt_drift, c2, mean_vel, \
         partials, extra, iso_S, tile_counts, count_bits, press, chg_words)
 #define SD_GATHER_K(D, I, P)                                          \
@@ -793,7 +808,7 @@ int launch_gather_kick_drift(const float* phi, int G, float pot_scale, const flo
     else { SD_GATHER_K(D, I, false); }
     if (!iso_S && G > 1024) {  // the simulation's grids end at 512: a stage call, plain
         if (dg || press || keys_mode != kKeysPlain) return fail(SD_E_UNSUPPORTED, "gather: grid %d above 1024", G);
-        k_gather_kick_drift<false, false, false, kKeysPlain, true><<<blocks, kGatherThreads, 0, s>>>(
+        launch(k_gather_kick_drift<false, false, false, kKeysPlain, true>, blocks, kGatherThreads, 0, s,
             phi, G, h, pos_in, vel_in, perm, pos_out, vel_out, keys_out, order, n, dt_kick, dt_drift, c2, mean_vel,
             partials, extra, iso_S, tile_counts, count_bits, press, chg_words);
     } else if (iso_S) {
@@ -808,11 +823,11 @@ int launch_gather_kick_drift(const float* phi, int G, float pot_scale, const flo
 #undef SD_GATHER
     SD_LAUNCHED(s);
     if (dg) {
-        k_finalize_mean<6><<<1, 256, 0, s>>>(partials, blocks, mom_out, mean_out, diag->rec, diag->count, diag->cap,
+        launch(k_finalize_mean<6>, 1, 256, 0, s, partials, blocks, mom_out, mean_out, diag->rec, diag->count, diag->cap,
                                             diag->mass, (double)pot_scale);
         SD_LAUNCHED(s);
     } else if (partials && (mom_out || mean_out)) {
-        k_finalize_mean<4><<<1, 256, 0, s>>>(partials, blocks, mom_out, mean_out, nullptr, nullptr, 1, 0.0, 0.0);
+        launch(k_finalize_mean<4>, 1, 256, 0, s, partials, blocks, mom_out, mean_out, nullptr, nullptr, 1, 0.0, 0.0);
         SD_LAUNCHED(s);
     }
     return SD_OK;
@@ -822,14 +837,14 @@ int launch_interpolate_accel(const float* phi, int G, float pot_scale, const flo
                              cudaStream_t s, const float4* extra, int iso_S) {
     if (n <= 0) return SD_OK;
     const float h = (0.5f * (float)G) * pot_scale;
-    k_interpolate_accel<<<(n + 255) / 256, 256, 0, s>>>(phi, G, h, pos, acc, n, extra, iso_S);
+    launch(k_interpolate_accel, (n + 255) / 256, 256, 0, s, phi, G, h, pos, acc, n, extra, iso_S);
     SD_LAUNCHED(s);
     return SD_OK;
 }
 
 int launch_apply_mean(float4* vel, const float4* pos, int n, const float* mean_vel, cudaStream_t s) {
     if (n <= 0) return SD_OK;
-    k_apply_mean<<<(n + 255) / 256, 256, 0, s>>>(vel, pos, n, mean_vel);
+    launch(k_apply_mean, (n + 255) / 256, 256, 0, s, vel, pos, n, mean_vel);
     SD_LAUNCHED(s);
     return SD_OK;
 }
@@ -839,7 +854,7 @@ int launch_max_speed(const float4* pos, const float4* vel, int n, const float* m
     if (SD_CUDA(cudaMemsetAsync(out, 0, sizeof(float), s)) != SD_OK) return SD_E_CUDA;
     if (n <= 0) return SD_OK;
     const int need = (n + 511) / 512, wave = 148 * kSpeedCtasPerSm;
-    k_max_speed<<<need < wave ? need : wave, 256, 0, s>>>(pos, vel, n, mean_vel, out);
+    launch(k_max_speed, need < wave ? need : wave, 256, 0, s, pos, vel, n, mean_vel, out);
     SD_LAUNCHED(s);
     return SD_OK;
 }
@@ -848,34 +863,34 @@ int launch_energy(const float* phi, int G, const float4* pos, const float4* vel,
                   double* partials, double* out8, cudaStream_t s, int iso_S) {
     if (n <= 0) return SD_OK;
     const int blocks = (int)gather_partials(n);  // partials hold 8 doubles per block
-    k_energy<<<blocks, kGatherThreads, 0, s>>>(phi, G, pos, vel, n, mean_vel, partials, iso_S);
+    launch(k_energy, blocks, kGatherThreads, 0, s, phi, G, pos, vel, n, mean_vel, partials, iso_S);
     SD_LAUNCHED(s);
-    k_finalize8<<<1, 256, 0, s>>>(partials, blocks, out8);
+    launch(k_finalize8, 1, 256, 0, s, partials, blocks, out8);
     SD_LAUNCHED(s);
     return SD_OK;
 }
 
 int launch_reduce_grid(const float* a, size_t cells, int op, double* partials, double* out, cudaStream_t s) {
     const int blocks = 296;
-    k_reduce_grid<<<blocks, 256, 0, s>>>(a, cells, op, partials);
+    launch(k_reduce_grid, blocks, 256, 0, s, a, cells, op, partials);
     SD_LAUNCHED(s);
-    k_reduce_final<<<1, 32, 0, s>>>(partials, blocks, op, out);
+    launch(k_reduce_final, 1, 32, 0, s, partials, blocks, op, out);
     SD_LAUNCHED(s);
     return SD_OK;
 }
 
 int launch_centroid(const float4* pos, int n, double* partials, double* out3, cudaStream_t s) {
     const int blocks = 296;
-    k_centroid<<<blocks, 256, 0, s>>>(pos, n, partials);
+    launch(k_centroid, blocks, 256, 0, s, pos, n, partials);
     SD_LAUNCHED(s);
-    k_centroid_final<<<1, 32, 0, s>>>(partials, blocks, out3);
+    launch(k_centroid_final, 1, 32, 0, s, partials, blocks, out3);
     SD_LAUNCHED(s);
     return SD_OK;
 }
 
 int launch_hide_range(float4* pos, float4* vel, int from, int to, cudaStream_t s) {
     if (to <= from) return SD_OK;
-    k_hide_range<<<(to - from + 255) / 256, 256, 0, s>>>(pos, vel, from, to);
+    launch(k_hide_range, (to - from + 255) / 256, 256, 0, s, pos, vel, from, to);
     SD_LAUNCHED(s);
     return SD_OK;
 }

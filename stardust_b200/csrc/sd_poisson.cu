@@ -186,6 +186,7 @@ template <int G, int SRC>
 __global__ void __launch_bounds__(kPassAThreads<G>, G == 512 ? 3 : 0)
     k_pass_a(const float* __restrict__ rho, long long* __restrict__ acc, float* __restrict__ rho_keep,
              float2* __restrict__ spec, const float2* __restrict__ tw_g, int src_g) {
+    wait_previous();
     using T = Geo<G>;
     constexpr int H = T::H, NBX = T::NBX;
     constexpr int ITEMS = 16 * (H / 2);  // (line, pair of positions)
@@ -440,6 +441,7 @@ template <int G, bool WIDE, bool ISO>
 __global__ void __launch_bounds__(256) k_deposit_plan(const int* __restrict__ rs, int* __restrict__ w, int split,
                                                       const float4* __restrict__ pos, int n,
                                                       unsigned long long* __restrict__ acc) {
+    wait_previous();
     using P = DepPlan<G>;
     const int b = blockIdx.x * 256 + threadIdx.x;
     int extra = 0;
@@ -805,6 +807,7 @@ __global__ void __launch_bounds__(kDepositThreads, kDepositPerSm<G>)
     k_pass_a_deposit_bal(const float4* __restrict__ pos, const int* __restrict__ perm,
                          const int* __restrict__ row_start, float* __restrict__ rho_keep, float2* __restrict__ spec,
                          const float2* __restrict__ tw_g, DepositWork w) {
+    wait_previous();
     using P = DepPlan<DepGeo<G, ISO>::M>;
     extern __shared__ float2 sm[];
     __shared__ int s_next;
@@ -901,6 +904,7 @@ __device__ __forceinline__ void store_lines(const float2* s, float2* __restrict_
 template <int G, bool INV, bool HALF>
 __global__ void __launch_bounds__(kFftThreads, G == 512 && HALF && !INV ? 3 : 0)
     k_pass_y(float2* __restrict__ spec, const float2* __restrict__ tw_g) {
+    wait_previous();
     extern __shared__ float2 sm[];
     float2* tw = sm;
     float2* s = sm + G;
@@ -923,6 +927,7 @@ template <int G, int MODE, bool HALF>
 __global__ void __launch_bounds__(kFftThreads) k_pass_c(float2* __restrict__ spec, const float2* __restrict__ tw_g,
                                                         const float* __restrict__ gexp_g, float scale,
                                                         const float* __restrict__ table, float table_scale) {
+    wait_previous();
     using T = Geo<G>;
     constexpr int H = T::H;
     extern __shared__ float2 sm[];
@@ -1016,6 +1021,7 @@ __global__ void k_green_kernel(float* __restrict__ g, int S, float soft) {
 template <int G, bool HALF>
 __global__ void __launch_bounds__(kFftThreads, 5) k_pass_e(const float2* __restrict__ spec, float* __restrict__ phi,
                                                         const float2* __restrict__ tw_g) {
+    wait_previous();
     using T = Geo<G>;
     constexpr int H = T::H, NBX = T::NBX;
     constexpr int ITEMS = NBX * 32;
@@ -1095,7 +1101,7 @@ struct Launcher {
     static int deposit(const PoissonPlan& p, const float4* pos, const int* perm, const int* row_start, float* keep,
                        float2* spec, const DepositWork& dw, cudaStream_t s) {
         using P = DepPlan<DepGeo<G, ISO>::M>;
-        k_deposit_plan<DepGeo<G, ISO>::M, WIDE, ISO><<<P::NC, 256, 0, s>>>(
+        launch(k_deposit_plan<DepGeo<G, ISO>::M, WIDE, ISO>, P::NC, 256, 0, s,
             row_start, dw.ints, dw.split, pos, dw.n, reinterpret_cast<unsigned long long*>(dw.acc));
         SD_LAUNCHED(s);
         // a CTA for each extra share that there can be, so none waits for another (a window of
@@ -1103,8 +1109,8 @@ struct Launcher {
         // windows); idle ones cost little, 1.5 us for 1,024. Never more than are taken by ticket.
         const long long extra = 4ll * dw.n / dw.split, wave = 148 * kDepositPerSm<G>;
         const long long ctas = P::NB + (extra < 8 ? 8 : extra);
-        k_pass_a_deposit_bal<G, ISO, WIDE><<<(unsigned)(kDepositLoop<G> && ctas > wave ? wave : ctas), kDepositThreads,
-                                             smem_bal<ISO>(), s>>>(pos, perm, row_start, keep, spec, p.tw, dw);
+        launch(k_pass_a_deposit_bal<G, ISO, WIDE>, (unsigned)(kDepositLoop<G> && ctas > wave ? wave : ctas), kDepositThreads,
+                                             smem_bal<ISO>(), s, pos, perm, row_start, keep, spec, p.tw, dw);
         SD_LAUNCHED(s);
         return SD_OK;
     }
@@ -1167,45 +1173,45 @@ struct Launcher {
             if (rc) return rc;
         } else {
             if (acc)
-                k_pass_a<G, 1><<<grid_rows, kPassAThreads<G>, smem_a(), s>>>(nullptr, const_cast<long long*>(acc), keep,
+                launch(k_pass_a<G, 1>, grid_rows, kPassAThreads<G>, smem_a(), s, nullptr, const_cast<long long*>(acc), keep,
                                                                          spec, p.tw, src_g);
             else
-                k_pass_a<G, 0><<<grid_rows, kPassAThreads<G>, smem_a(), s>>>(rho, nullptr, keep, spec, p.tw, src_g);
+                launch(k_pass_a<G, 0>, grid_rows, kPassAThreads<G>, smem_a(), s, rho, nullptr, keep, spec, p.tw, src_g);
             SD_LAUNCHED(s);
         }
         if (ev) cudaEventRecord(ev[0], s);
         if constexpr (kIsoBox) {
             if (half) {
-                k_pass_y<G, false, true><<<grid_y, kFftThreads, smem_bd(), s>>>(spec, p.tw);
+                launch(k_pass_y<G, false, true>, grid_y, kFftThreads, smem_bd(), s, spec, p.tw);
                 SD_LAUNCHED(s);
                 if (ev) cudaEventRecord(ev[1], s);
-                k_pass_c<G, 2, true><<<grid_z, kFftThreads, smem_ct(), s>>>(spec, p.tw, p.gexp, p.scale, iso->table,
+                launch(k_pass_c<G, 2, true>, grid_z, kFftThreads, smem_ct(), s, spec, p.tw, p.gexp, p.scale, iso->table,
                                                                            iso->table_scale);
                 SD_LAUNCHED(s);
                 if (ev) cudaEventRecord(ev[2], s);
-                k_pass_y<G, true, true><<<grid_y, kFftThreads, smem_bd(), s>>>(spec, p.tw);
+                launch(k_pass_y<G, true, true>, grid_y, kFftThreads, smem_bd(), s, spec, p.tw);
                 SD_LAUNCHED(s);
                 if (ev) cudaEventRecord(ev[3], s);
-                k_pass_e<G, true><<<grid_rows, kFftThreads, smem_ae(), s>>>(spec, phi, p.tw);
+                launch(k_pass_e<G, true>, grid_rows, kFftThreads, smem_ae(), s, spec, phi, p.tw);
                 SD_LAUNCHED(s);
                 return SD_OK;
             }
         }
-        k_pass_y<G, false, false><<<grid_y, kFftThreads, smem_bd(), s>>>(spec, p.tw);
+        launch(k_pass_y<G, false, false>, grid_y, kFftThreads, smem_bd(), s, spec, p.tw);
         SD_LAUNCHED(s);
         if (ev) cudaEventRecord(ev[1], s);
         if (iso && iso->forward_only) {
-            k_pass_c<G, 1, false><<<grid_z, kFftThreads, smem_c(), s>>>(spec, p.tw, p.gexp, p.scale, nullptr, 0.f);
+            launch(k_pass_c<G, 1, false>, grid_z, kFftThreads, smem_c(), s, spec, p.tw, p.gexp, p.scale, nullptr, 0.f);
             SD_LAUNCHED(s);
             return SD_OK;
         }
-        k_pass_c<G, 0, false><<<grid_z, kFftThreads, smem_c(), s>>>(spec, p.tw, p.gexp, p.scale, nullptr, 0.f);
+        launch(k_pass_c<G, 0, false>, grid_z, kFftThreads, smem_c(), s, spec, p.tw, p.gexp, p.scale, nullptr, 0.f);
         SD_LAUNCHED(s);
         if (ev) cudaEventRecord(ev[2], s);
-        k_pass_y<G, true, false><<<grid_y, kFftThreads, smem_bd(), s>>>(spec, p.tw);
+        launch(k_pass_y<G, true, false>, grid_y, kFftThreads, smem_bd(), s, spec, p.tw);
         SD_LAUNCHED(s);
         if (ev) cudaEventRecord(ev[3], s);
-        k_pass_e<G, false><<<grid_rows, kFftThreads, smem_ae(), s>>>(spec, phi, p.tw);
+        launch(k_pass_e<G, false>, grid_rows, kFftThreads, smem_ae(), s, spec, phi, p.tw);
         SD_LAUNCHED(s);
         return SD_OK;
     }

@@ -98,6 +98,7 @@ __device__ __forceinline__ void load_words8(const unsigned* __restrict__ p, unsi
 // padded to whole chunks, and the padding stays zero).
 __global__ void __launch_bounds__(kChgThreads) k_chg_count(const unsigned* __restrict__ words,
                                                            unsigned* __restrict__ chunk_cnt) {
+    wait_previous();
     __shared__ unsigned red[kChgThreads / 32];
     unsigned w[8];
     load_words8(words + (size_t)blockIdx.x * kChunkWords + threadIdx.x * kChgWordsPer, w);
@@ -116,6 +117,7 @@ __global__ void __launch_bounds__(kChgThreads) k_chg_compact(const unsigned* __r
                                                              const uint32_t* __restrict__ keys,
                                                              unsigned* __restrict__ word_pre, uint32_t* __restrict__ ck,
                                                              int32_t* __restrict__ ci, int* __restrict__ n_changed) {
+    wait_previous();
     __shared__ unsigned red[kChgThreads / 32];
     unsigned before = 0u;  // changed positions in the chunks before this one
     for (int c0 = 0; c0 < (int)blockIdx.x; c0 += 8 * kChgThreads) {  // eight loads in flight per thread
@@ -183,6 +185,7 @@ __global__ void k_merge_changed(const uint32_t* __restrict__ ck, const int32_t* 
                                 const int* __restrict__ n_changed, const uint32_t* __restrict__ keys, int shift,
                                 const int* __restrict__ row_start_old, const unsigned* __restrict__ words,
                                 const unsigned* __restrict__ word_pre, int32_t* __restrict__ vals_out) {
+    wait_previous();
     const int nc = *n_changed;
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nc; r += gridDim.x * blockDim.x) {
         const uint32_t k = ck[r];
@@ -220,6 +223,7 @@ __global__ void k_merge_changed(const uint32_t* __restrict__ ck, const int32_t* 
 __global__ void k_rows(const uint32_t* __restrict__ ck, const int* __restrict__ n_changed, int rows, int shift,
                        const unsigned* __restrict__ words, const unsigned* __restrict__ word_pre,
                        int* __restrict__ c_rows, int* __restrict__ row_start) {
+    wait_previous();
     const int nc = *n_changed;
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r <= rows; r += gridDim.x * blockDim.x) {
         const uint32_t low = row_low(r, shift);
@@ -267,6 +271,7 @@ __global__ void __launch_bounds__(kMergeThreads) k_merge_unchanged(const uint32_
                                                                    const uint32_t* __restrict__ ck,
                                                                    const int32_t* __restrict__ ci, int n,
                                                                    int32_t* __restrict__ vals_out) {
+    wait_previous();
     const int lane = threadIdx.x & 31;
     const size_t wb = (size_t)blockIdx.x * kMergeWords + (threadIdx.x >> 5) * kMergeWordsPerWarp;
     const int base = (int)(wb * 32);
@@ -358,9 +363,9 @@ int launch_resort(const ResortBufs& r, const uint32_t* keys, int n, int G, int o
     if (n <= 0) return SD_OK;
     const int chunks = (int)(padded_words(n) / kChunkWords);
     const int rows = row_last(G, order), shift = row_shift(G, order);
-    k_chg_count<<<chunks, kChgThreads, 0, s>>>(r.words, r.chunk_cnt);
+    launch(k_chg_count, chunks, kChgThreads, 0, s, r.words, r.chunk_cnt);
     SD_LAUNCHED(s);
-    k_chg_compact<<<chunks, kChgThreads, 0, s>>>(r.words, r.chunk_cnt, keys, r.word_pre, r.ck_in, r.ci_in,
+    launch(k_chg_compact, chunks, kChgThreads, 0, s, r.words, r.chunk_cnt, keys, r.word_pre, r.ck_in, r.ci_in,
                                                  r.n_changed);
     SD_LAUNCHED(s);
     // C by key, stable: the radix sort with the count on the device
@@ -368,15 +373,15 @@ int launch_resort(const ResortBufs& r, const uint32_t* keys, int n, int G, int o
                                sort_ws_bytes, s, true, false, r.n_changed);
     if (rc) return rc;
     auto changed = shift < 0 ? k_merge_changed<false> : k_merge_changed<true>;
-    changed<<<148 * 4, 256, 0, s>>>(r.ck_out, r.ci_out, r.n_changed, keys, shift, row_start, r.words, r.word_pre,
+    launch(changed, 148 * 4, 256, 0, s, r.ck_out, r.ci_out, r.n_changed, keys, shift, row_start, r.words, r.word_pre,
                                     vals_out);
     SD_LAUNCHED(s);
-    k_rows<<<(rows + 1 + 255) / 256, 256, 0, s>>>(r.ck_out, r.n_changed, rows, shift, r.words, r.word_pre, r.c_rows,
+    launch(k_rows, (rows + 1 + 255) / 256, 256, 0, s, r.ck_out, r.n_changed, rows, shift, r.words, r.word_pre, r.c_rows,
                                                    row_start);
     SD_LAUNCHED(s);
     const int warps = (n + 255) / 256;
     auto unchanged = shift < 0 ? k_merge_unchanged<false> : k_merge_unchanged<true>;
-    unchanged<<<(warps + kMergeThreads / 32 - 1) / (kMergeThreads / 32), kMergeThreads, 0, s>>>(
+    launch(unchanged, (warps + kMergeThreads / 32 - 1) / (kMergeThreads / 32), kMergeThreads, 0, s,
         keys, r.words, r.word_pre, r.c_rows, shift, r.ck_out, r.ci_out, n, vals_out);
     SD_LAUNCHED(s);
     return SD_OK;

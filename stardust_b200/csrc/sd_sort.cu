@@ -54,6 +54,7 @@ constexpr int kColSegs = kColThreads / 32;  // 8 segments of a column per CTA
 __global__ void __launch_bounds__(256) k_cell_keys(const float4* __restrict__ pos, int n, int G, int order,
                                                    uint32_t* __restrict__ keys, int* __restrict__ stray,
                                                    int periodic) {
+    wait_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 p = pos[i];
@@ -87,6 +88,7 @@ __global__ void __launch_bounds__(kSortThreads) k_digit_counts(const uint32_t* _
                                                                unsigned* __restrict__ counts,
                                                                unsigned* __restrict__ chunk_sums,
                                                                const int* __restrict__ n_dev) {
+    wait_previous();
     constexpr int kRadix = 1 << BITS;
     constexpr unsigned mask = kRadix - 1;
     __shared__ unsigned hist[kRadix];
@@ -289,6 +291,7 @@ __global__ void __launch_bounds__(kSortThreads) k_digit_scatter(const uint32_t* 
                                                                 unsigned* __restrict__ next_counts,
                                                                 unsigned* __restrict__ next_sums, int next_shift,
                                                                 const int* __restrict__ n_dev) {
+    wait_previous();
     __shared__ ScatterSmem<BITS> sm;
     if (!LOOP) {
         scatter_tile<BITS>(sm, blockIdx.x, keys_in, vals_in, keys_out, vals_out, n, shift, offsets, totals,
@@ -317,6 +320,7 @@ constexpr int kScanRows = 16;
 constexpr int kScanTiles = 2048;  // above (4M keys) the chunked scan's many CTAs are faster
 __global__ void __launch_bounds__(kScanThreads) k_col_scan(unsigned* __restrict__ counts, int tiles, int radix,
                                                            unsigned* __restrict__ T, const int* __restrict__ n_dev) {
+    wait_previous();
     __shared__ unsigned pre[32][33];
     __shared__ unsigned total[32];
     if (n_dev) tiles = (*n_dev + kSortTile - 1) / kSortTile;
@@ -366,6 +370,7 @@ __global__ void __launch_bounds__(kScanThreads) k_col_scan(unsigned* __restrict_
 //                and clears S, ready for the adds of the next counts
 __global__ void __launch_bounds__(kColThreads) k_col_sums(const unsigned* __restrict__ counts, int tiles, int radix,
                                                           unsigned* __restrict__ S) {
+    wait_previous();
     const int d = blockIdx.y * kColThreads + threadIdx.x;
     if (d >= radix) return;
     const int c = blockIdx.x, t0 = c * kColChunk, t1 = min(tiles, t0 + kColChunk);
@@ -379,6 +384,7 @@ __global__ void __launch_bounds__(kColThreads) k_col_sums(const unsigned* __rest
 // contiguous run of chunks; two sweeps (sum, rewrite) around a scan of the runs.
 __global__ void __launch_bounds__(kColThreads) k_col_prefix(unsigned* __restrict__ S, int chunks, int radix,
                                                             unsigned* __restrict__ T, unsigned* __restrict__ done) {
+    wait_previous();
     __shared__ unsigned seg_sum[kColSegs][32];
     __shared__ unsigned scan_tmp[kWarps];
     __shared__ bool last;
@@ -443,6 +449,7 @@ __global__ void __launch_bounds__(kColThreads) k_col_prefix(unsigned* __restrict
 __global__ void __launch_bounds__(kColThreads) k_col_apply(unsigned* __restrict__ counts, int tiles, int radix,
                                                            unsigned* __restrict__ S,
                                                            const unsigned* __restrict__ T) {
+    wait_previous();
     __shared__ unsigned tile[kColChunk][33];
     __shared__ unsigned seg_sum[kColSegs][32];
     const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
@@ -482,6 +489,7 @@ __global__ void __launch_bounds__(kColThreads) k_col_apply(unsigned* __restrict_
 __global__ void __launch_bounds__(256) k_reorder(const float4* __restrict__ pos_in, const float4* __restrict__ vel_in,
                                                  const int32_t* __restrict__ perm, float4* __restrict__ pos_out,
                                                  float4* __restrict__ vel_out, int n) {
+    wait_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int j = perm[i];
@@ -491,6 +499,7 @@ __global__ void __launch_bounds__(256) k_reorder(const float4* __restrict__ pos_
 
 __global__ void k_copy_keys(const uint32_t* __restrict__ kin, const int32_t* __restrict__ vin,
                             uint32_t* __restrict__ kout, int32_t* __restrict__ vout, int n) {
+    wait_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     kout[i] = kin[i];
@@ -511,6 +520,7 @@ __global__ void k_copy_keys(const uint32_t* __restrict__ kin, const int32_t* __r
 constexpr int kRowShortRun = 8;
 __global__ void __launch_bounds__(256) k_row_marks(const uint32_t* __restrict__ keys, int n, int rows, int shift,
                                                    int* __restrict__ row_start) {
+    wait_previous();
     __shared__ int q_lo[256], q_hi[256], q_val[256];
     __shared__ int q_count;
     if (threadIdx.x == 0) q_count = 0;
@@ -537,6 +547,7 @@ __global__ void __launch_bounds__(256) k_row_marks(const uint32_t* __restrict__ 
 // One thread per row: a lower-bound search over the keys.
 __global__ void k_row_bounds(const uint32_t* __restrict__ keys, int n, int rows, int shift,
                              int* __restrict__ row_start) {
+    wait_previous();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r > rows) return;
     const uint32_t low = row_low(r, shift);
@@ -557,9 +568,9 @@ __global__ void k_row_bounds(const uint32_t* __restrict__ keys, int n, int rows,
 
 int launch_row_bounds(const uint32_t* keys, int n, int rows, int shift, int* row_start, cudaStream_t s) {
     if (n <= (1 << 20))
-        k_row_marks<<<(n + 1 + 255) / 256, 256, 0, s>>>(keys, n, rows, shift, row_start);
+        launch(k_row_marks, (n + 1 + 255) / 256, 256, 0, s, keys, n, rows, shift, row_start);
     else
-        k_row_bounds<<<(rows + 1 + 255) / 256, 256, 0, s>>>(keys, n, rows, shift, row_start);
+        launch(k_row_bounds, (rows + 1 + 255) / 256, 256, 0, s, keys, n, rows, shift, row_start);
     SD_LAUNCHED(s);
     return SD_OK;
 }
@@ -567,7 +578,7 @@ int launch_row_bounds(const uint32_t* keys, int n, int rows, int shift, int* row
 int launch_cell_keys(const float4* pos, int n, int G, int order, uint32_t* keys, cudaStream_t s, int* stray,
                      int periodic) {
     if (n <= 0) return SD_OK;
-    k_cell_keys<<<(n + 255) / 256, 256, 0, s>>>(pos, n, G, order, keys, stray, periodic);
+    launch(k_cell_keys, (n + 255) / 256, 256, 0, s, pos, n, G, order, keys, stray, periodic);
     SD_LAUNCHED(s);
     return SD_OK;
 }
@@ -621,19 +632,19 @@ static int scan_offsets(unsigned* counts, int tiles, int radix, const SortWs& w,
                         bool chunked, bool sums_ready) {
     const int slabs = radix / 32;
     if (!chunked) {
-        k_col_scan<<<slabs, kScanThreads, 0, s>>>(counts, tiles, radix, w.T, n_dev);
+        launch(k_col_scan, slabs, kScanThreads, 0, s, counts, tiles, radix, w.T, n_dev);
         SD_LAUNCHED(s);
         return SD_OK;
     }
     const int chunks = col_chunks(tiles);
     if (!sums_ready) {
-        k_col_sums<<<dim3(chunks, (radix + kColThreads - 1) / kColThreads), kColThreads, 0, s>>>(counts, tiles, radix,
+        launch(k_col_sums, dim3(chunks, (radix + kColThreads - 1) / kColThreads), kColThreads, 0, s, counts, tiles, radix,
                                                                                                w.S);
         SD_LAUNCHED(s);
     }
-    k_col_prefix<<<slabs, kColThreads, 0, s>>>(w.S, chunks, radix, w.T, w.done);
+    launch(k_col_prefix, slabs, kColThreads, 0, s, w.S, chunks, radix, w.T, w.done);
     SD_LAUNCHED(s);
-    k_col_apply<<<dim3(chunks, slabs), kColThreads, 0, s>>>(counts, tiles, radix, w.S, w.T);
+    launch(k_col_apply, dim3(chunks, slabs), kColThreads, 0, s, counts, tiles, radix, w.S, w.T);
     SD_LAUNCHED(s);
     return SD_OK;
 }
@@ -655,9 +666,9 @@ int launch_sort_first_counts(const uint32_t* keys, int n, int key_bits, void* ws
     const int tiles = (n + kSortTile - 1) / kSortTile;
     const SortWs w = sort_ws_layout(ws, n);
     switch (bits) {
-        case 8: k_digit_counts<8><<<tiles, kSortThreads, 0, s>>>(keys, n, 0, w.cnt[0], nullptr, nullptr); break;
-        case 9: k_digit_counts<9><<<tiles, kSortThreads, 0, s>>>(keys, n, 0, w.cnt[0], nullptr, nullptr); break;
-        default: k_digit_counts<10><<<tiles, kSortThreads, 0, s>>>(keys, n, 0, w.cnt[0], nullptr, nullptr); break;
+        case 8: launch(k_digit_counts<8>, tiles, kSortThreads, 0, s, keys, n, 0, w.cnt[0], nullptr, nullptr); break;
+        case 9: launch(k_digit_counts<9>, tiles, kSortThreads, 0, s, keys, n, 0, w.cnt[0], nullptr, nullptr); break;
+        default: launch(k_digit_counts<10>, tiles, kSortThreads, 0, s, keys, n, 0, w.cnt[0], nullptr, nullptr); break;
     }
     SD_LAUNCHED(s);
     return SD_OK;
@@ -676,7 +687,7 @@ int launch_sort_pairs(const uint32_t* keys_in, const int32_t* vals_in, uint32_t*
     // fewest passes of at most kMaxRadixBits bits
     const int passes = (key_bits + kMaxRadixBits - 1) / kMaxRadixBits;
     if (passes == 0) {
-        k_copy_keys<<<(n + 255) / 256, 256, 0, s>>>(keys_in, vals_in, keys_out, vals_out, n);
+        launch(k_copy_keys, (n + 255) / 256, 256, 0, s, keys_in, vals_in, keys_out, vals_out, n);
         SD_LAUNCHED(s);
         return SD_OK;
     }
@@ -715,9 +726,9 @@ int launch_sort_pairs(const uint32_t* keys_in, const int32_t* vals_in, uint32_t*
         if (p == 0 && !first_counts_ready) {
             const int g = count_grid;
             switch (bits) {
-                case 8: k_digit_counts<8><<<g, kSortThreads, 0, s>>>(kin, n, shift, counts, sums, n_dev); break;
-                case 9: k_digit_counts<9><<<g, kSortThreads, 0, s>>>(kin, n, shift, counts, sums, n_dev); break;
-                default: k_digit_counts<10><<<g, kSortThreads, 0, s>>>(kin, n, shift, counts, sums, n_dev); break;
+                case 8: launch(k_digit_counts<8>, g, kSortThreads, 0, s, kin, n, shift, counts, sums, n_dev); break;
+                case 9: launch(k_digit_counts<9>, g, kSortThreads, 0, s, kin, n, shift, counts, sums, n_dev); break;
+                default: launch(k_digit_counts<10>, g, kSortThreads, 0, s, kin, n, shift, counts, sums, n_dev); break;
             }
             SD_LAUNCHED(s);
         }
@@ -727,7 +738,7 @@ int launch_sort_pairs(const uint32_t* keys_in, const int32_t* vals_in, uint32_t*
             return rc;
         const unsigned* totals = chunked ? nullptr : w.T;
 #define SD_SCATTER(B, L)                                                                                   \
-    k_digit_scatter<B, L><<<scatter_grid, kSortThreads, 0, s>>>(kin, vin, kout, vout, n, shift, counts, totals, next, \
+    launch(k_digit_scatter<B, L>, scatter_grid, kSortThreads, 0, s, kin, vin, kout, vout, n, shift, counts, totals, next, \
                                                                 sums, next_shift, n_dev)
 #define SD_SCATTER_B(B)        \
     if (n_dev) SD_SCATTER(B, true); \
@@ -749,7 +760,7 @@ int launch_sort_pairs(const uint32_t* keys_in, const int32_t* vals_in, uint32_t*
 int launch_reorder(const float4* pos_in, const float4* vel_in, const int32_t* perm, float4* pos_out,
                    float4* vel_out, int n, cudaStream_t s) {
     if (n <= 0) return SD_OK;
-    k_reorder<<<(n + 255) / 256, 256, 0, s>>>(pos_in, vel_in, perm, pos_out, vel_out, n);
+    launch(k_reorder, (n + 255) / 256, 256, 0, s, pos_in, vel_in, perm, pos_out, vel_out, n);
     SD_LAUNCHED(s);
     return SD_OK;
 }
