@@ -30,42 +30,79 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ float2 conjf2(float2 a) { return make_float2(a.x, -a.y); }
-// multiply by -i (forward) or +i (inverse)
+// a - i b (forward) or a + i b (inverse)
 template <bool INV>
-__device__ __forceinline__ float2 mul_mi(float2 a) {
-    return INV ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
+__device__ __forceinline__ float2 add_mi(float2 a, float2 b) {
+    return INV ? make_float2(a.x - b.y, a.y + b.x) : make_float2(a.x + b.y, a.y - b.x);
 }
 
-// W_32^k = exp(-2 pi i k / 32), k < 16 (mathematical constants; the inverse uses
-// conjugates). W_16^k = W_32^(2k).
+// a + b, a - b and a + c b. PAIR: both halves in one instruction, each rounded as a
+// scalar's.
+template <bool PAIR>
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    if (!PAIR) return cadd(a, b);
+    float2 r;
+    asm("{ .reg .b64 x, y;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.f32x2 x, x, y;\n mov.b64 {%0, %1}, x; }"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+template <bool PAIR>
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+    if (!PAIR) return csub(a, b);
+    float2 r;
+    asm("{ .reg .b64 x, y;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n sub.rn.f32x2 x, x, y;\n mov.b64 {%0, %1}, x; }"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+template <bool PAIR>
+__device__ __forceinline__ float2 fma2(float c, float2 b, float2 a) {
+    if (!PAIR) return make_float2(fmaf(c, b.x, a.x), fmaf(c, b.y, a.y));
+    float2 r;
+    asm("{ .reg .b64 x, y, z;\n mov.b64 x, {%2, %2};\n mov.b64 y, {%3, %4};\n mov.b64 z, {%5, %6};\n"
+        " fma.rn.f32x2 x, x, y, z;\n mov.b64 {%0, %1}, x; }"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(c), "f"(b.x), "f"(b.y), "f"(a.x), "f"(a.y));
+    return r;
+}
+
+// exp(-2 pi i k / 32), 0 < k < 16, k != 8, as c (1 + i t) where the cosine is the larger
+// part and as c (t + i) where the sine is (swap). Two fused operations then form
+// u = b (1 + i t), and four more a + c u and a - c u, one rounding each: a butterfly is
+// 6 instead of 8 instructions. (The inverse's: t changes sign, and c with swap.)
+struct Turn {
+    float t, c;
+    bool swap;
+};
 namespace w32 {
-constexpr float c1 = 0.98078528040323044913f, s1 = 0.19509032201612826785f;
-constexpr float c2 = 0.92387953251128675613f, s2 = 0.38268343236508977173f;
-constexpr float c3 = 0.83146961230254523708f, s3 = 0.55557023301960222474f;
-constexpr float r = 0.70710678118654752440f;
-__device__ __forceinline__ float2 get(int k) {  // k is a compile-time constant after unrolling
+constexpr double c1 = 0.98078528040323044913, s1 = 0.19509032201612826785;
+constexpr double c2 = 0.92387953251128675613, s2 = 0.38268343236508977173;
+constexpr double c3 = 0.83146961230254523708, s3 = 0.55557023301960222474;
+constexpr double r = 0.70710678118654752440;
+__device__ __forceinline__ Turn get(int k) {  // k is a compile-time constant after unrolling
+    constexpr float t1 = (float)(s1 / c1), t2 = (float)(s2 / c2), t3 = (float)(s3 / c3);
+    constexpr float f1 = (float)c1, f2 = (float)c2, f3 = (float)c3, fr = (float)r;
     switch (k) {
-        case 0: return make_float2(1.f, 0.f);
-        case 1: return make_float2(c1, -s1);
-        case 2: return make_float2(c2, -s2);
-        case 3: return make_float2(c3, -s3);
-        case 4: return make_float2(r, -r);
-        case 5: return make_float2(s3, -c3);
-        case 6: return make_float2(s2, -c2);
-        case 7: return make_float2(s1, -c1);
-        case 8: return make_float2(0.f, -1.f);
-        case 9: return make_float2(-s1, -c1);
-        case 10: return make_float2(-s2, -c2);
-        case 11: return make_float2(-s3, -c3);
-        case 12: return make_float2(-r, -r);
-        case 13: return make_float2(-c3, -s3);
-        case 14: return make_float2(-c2, -s2);
-        default: return make_float2(-c1, -s1);
+        case 1: return {-t1, f1, false};
+        case 2: return {-t2, f2, false};
+        case 3: return {-t3, f3, false};
+        case 4: return {-1.f, fr, false};
+        case 5: return {-t3, -f3, true};
+        case 6: return {-t2, -f2, true};
+        case 7: return {-t1, -f1, true};
+        case 9: return {t1, -f1, true};
+        case 10: return {t2, -f2, true};
+        case 11: return {t3, -f3, true};
+        case 12: return {1.f, -fr, false};
+        case 13: return {t3, -f3, false};
+        case 14: return {t2, -f2, false};
+        default: return {t1, -f1, false};
     }
 }
 }  // namespace w32
 
-template <int R, bool INV>
+template <int R, bool INV, bool PAIR = false>
 __device__ __forceinline__ void dft(float2* v) {
     if constexpr (R == 16 || R == 32) {
         // radix-2 split: DFTs of the even and odd inputs, combined with W_R^k
@@ -76,47 +113,51 @@ __device__ __forceinline__ void dft(float2* v) {
             e[i] = v[2 * i];
             o[i] = v[2 * i + 1];
         }
-        dft<H, INV>(e);
-        dft<H, INV>(o);
+        dft<H, INV, PAIR>(e);
+        dft<H, INV, PAIR>(o);
+        v[0] = add2<PAIR>(e[0], o[0]);
+        v[H] = sub2<PAIR>(e[0], o[0]);
 #pragma unroll
-        for (int k = 0; k < H; ++k) {
-            float2 w = w32::get(k * (32 / R));
-            if (INV) w.y = -w.y;
-            const float2 t = (k == 0) ? o[k] : cmul(o[k], w);
-            v[k] = cadd(e[k], t);
-            v[k + H] = csub(e[k], t);
+        for (int k = 1; k < H; ++k) {
+            if (k == H / 2) {
+                v[k] = add_mi<INV>(e[k], o[k]);
+                v[k + H] = add_mi<!INV>(e[k], o[k]);
+                continue;
+            }
+            const Turn w = w32::get(k * (32 / R));
+            const float t = INV ? -w.t : w.t, c = INV && w.swap ? -w.c : w.c;
+            const float2 u = w.swap ? make_float2(fmaf(t, o[k].x, -o[k].y), fmaf(t, o[k].y, o[k].x))
+                                    : make_float2(fmaf(-t, o[k].y, o[k].x), fmaf(t, o[k].x, o[k].y));
+            v[k] = fma2<PAIR>(c, u, e[k]);
+            v[k + H] = fma2<PAIR>(-c, u, e[k]);
         }
     } else if constexpr (R == 2) {
         const float2 a = v[0], b = v[1];
-        v[0] = cadd(a, b);
-        v[1] = csub(a, b);
+        v[0] = add2<PAIR>(a, b);
+        v[1] = sub2<PAIR>(a, b);
     } else if constexpr (R == 4) {
-        const float2 t0 = cadd(v[0], v[2]), t1 = csub(v[0], v[2]);
-        const float2 t2 = cadd(v[1], v[3]), t3 = mul_mi<INV>(csub(v[1], v[3]));
-        v[0] = cadd(t0, t2);
-        v[2] = csub(t0, t2);
-        v[1] = cadd(t1, t3);
-        v[3] = csub(t1, t3);
+        const float2 t0 = add2<PAIR>(v[0], v[2]), t1 = sub2<PAIR>(v[0], v[2]);
+        const float2 t2 = add2<PAIR>(v[1], v[3]), t3 = sub2<PAIR>(v[1], v[3]);
+        v[0] = add2<PAIR>(t0, t2);
+        v[2] = sub2<PAIR>(t0, t2);
+        v[1] = add_mi<INV>(t1, t3);
+        v[3] = add_mi<!INV>(t1, t3);
     } else {  // R == 8: two 4-point DFTs of the even and odd inputs
         float2 e[4] = {v[0], v[2], v[4], v[6]};
         float2 o[4] = {v[1], v[3], v[5], v[7]};
-        dft<4, INV>(e);
-        dft<4, INV>(o);
+        dft<4, INV, PAIR>(e);
+        dft<4, INV, PAIR>(o);
         constexpr float c = 0.70710678118654752440f;
-        // W8^1 = c(1 -/+ i), W8^2 = -/+ i, W8^3 = c(-1 -/+ i)
-        const float2 o1 = INV ? make_float2(c * (o[1].x - o[1].y), c * (o[1].x + o[1].y))
-                              : make_float2(c * (o[1].x + o[1].y), c * (o[1].y - o[1].x));
-        const float2 o2 = mul_mi<INV>(o[2]);
-        const float2 o3 = INV ? make_float2(-c * (o[3].x + o[3].y), c * (o[3].x - o[3].y))
-                              : make_float2(c * (o[3].y - o[3].x), -c * (o[3].x + o[3].y));
-        v[0] = cadd(e[0], o[0]);
-        v[4] = csub(e[0], o[0]);
-        v[1] = cadd(e[1], o1);
-        v[5] = csub(e[1], o1);
-        v[2] = cadd(e[2], o2);
-        v[6] = csub(e[2], o2);
-        v[3] = cadd(e[3], o3);
-        v[7] = csub(e[3], o3);
+        // W8^1 = c(1 -/+ i), W8^2 = -/+ i, W8^3 = -c(1 +/- i)
+        const float2 o1 = add_mi<INV>(o[1], o[1]), o3 = add_mi<!INV>(o[3], o[3]);
+        v[0] = add2<PAIR>(e[0], o[0]);
+        v[4] = sub2<PAIR>(e[0], o[0]);
+        v[1] = fma2<PAIR>(c, o1, e[1]);
+        v[5] = fma2<PAIR>(-c, o1, e[1]);
+        v[2] = add_mi<INV>(e[2], o[2]);
+        v[6] = add_mi<!INV>(e[2], o[2]);
+        v[3] = fma2<PAIR>(-c, o3, e[3]);
+        v[7] = fma2<PAIR>(c, o3, e[3]);
     }
 }
 
@@ -159,7 +200,8 @@ struct PlainLoad {
 // Stages from sub-transform length Ns on, stopping before the stage at STOP; the
 // stage at Ns = 1 reads through `load`. HALF: positions N/2 and up of the input are
 // zero and are not read (they are the upper half of the first stage's radix).
-template <int N, int Ns, int NT, int TWS, bool INV, int STOP = N, class Load = PlainLoad, bool HALF = false>
+template <int N, int Ns, int NT, int TWS, bool INV, int STOP = N, class Load = PlainLoad, bool HALF = false,
+          bool PAIR = false>
 __device__ __forceinline__ void stages16(float2* s, const float2* tw, Load load = Load()) {
     if constexpr (Ns < N && Ns < STOP) {
         constexpr int R = radix_of<N / Ns, N, NT>::value;
@@ -194,14 +236,14 @@ __device__ __forceinline__ void stages16(float2* s, const float2* tw, Load load 
             const int u = threadIdx.x + p * NT;
             if (TOT % NT == 0 || u < TOT) {
                 const int l = u & 15, j = u >> 4, k = j % Ns;
-                dft<R, INV>(v[p]);
+                dft<R, INV, PAIR>(v[p]);
                 const int base = (j / Ns) * Ns * R + k;
 #pragma unroll
                 for (int r = 0; r < R; ++r) s[(base + r * Ns) * 16 + l] = v[p][r];
             }
         }
         __syncthreads();
-        stages16<N, Ns * R, NT, TWS, INV, STOP>(s, tw);
+        stages16<N, Ns * R, NT, TWS, INV, STOP, PlainLoad, false, PAIR>(s, tw);
     }
 }
 
@@ -216,7 +258,7 @@ __device__ __forceinline__ void lines16(float2* s, const float2* tw) {
 // The forward's last stage (radix R, sub-length Ns = N / R) leaves, in each
 // thread's registers, the outputs at positions j + r Ns -- exactly the inputs of
 // an inverse first stage of the same radix. So that stage, the multiply
-// mul(line, position, value) and the inverse's first stage run in registers with
+// mul(line, position, position >= N / 2, value) and the inverse's first stage run in registers with
 // no shared-memory round trip or barrier between them; the inverse then goes on
 // from sub-length R. The caller synchronises before the call; it ends with a
 // barrier. HALF: the input's upper half is zero (N takes at least two stages).
@@ -228,7 +270,7 @@ __device__ __forceinline__ void convolve16(float2* s, const float2* tw, Mul mul)
     constexpr int TOT = 16 * NB;
     constexpr int PER = (TOT + NT - 1) / NT;
     static_assert(!HALF || NsL > 1, "a half-zero input is pruned in a first stage of its own");
-    stages16<N, 1, NT, TWS, false, NsL, PlainLoad, HALF>(s, tw);
+    stages16<N, 1, NT, TWS, false, NsL, PlainLoad, HALF, true>(s, tw);
     float2 v[PER][R];
 #pragma unroll
     for (int p = 0; p < PER; ++p) {
@@ -249,16 +291,16 @@ __device__ __forceinline__ void convolve16(float2* s, const float2* tw, Mul mul)
         const int u = threadIdx.x + p * NT;
         if (TOT % NT == 0 || u < TOT) {
             const int l = u & 15, j = u >> 4;
-            dft<R, false>(v[p]);
+            dft<R, false, true>(v[p]);
 #pragma unroll
-            for (int r = 0; r < R; ++r) v[p][r] = mul(l, j + r * NsL, v[p][r]);
-            dft<R, true>(v[p]);
+            for (int r = 0; r < R; ++r) v[p][r] = mul(l, j + r * NsL, r >= R / 2, v[p][r]);
+            dft<R, true, true>(v[p]);
 #pragma unroll
             for (int r = 0; r < R; ++r) s[(j * R + r) * 16 + l] = v[p][r];
         }
     }
     __syncthreads();
-    stages16<N, R, NT, TWS, true>(s, tw);
+    stages16<N, R, NT, TWS, true, N, PlainLoad, false, true>(s, tw);
 }
 
 // lines16, with the last stage writing its outputs row-major (line l at

@@ -923,10 +923,15 @@ __global__ void __launch_bounds__(kFftThreads, G == 512 && HALF && !INV ? 3 : 0)
 //         (columns past kx = H hold zeros) times table_scale, then inverse (isolated
 //         boundary, kMulSpec, Sim.cu:578-584). A CTA's values are 4 contiguous runs.
 // HALF: the lines' upper half is zero on input and not needed on output (see k_pass_y).
+// Two transforms on one trip through memory, so the instructions count (68 % of the issue
+// slots at 512, shared memory 63 %), and the butterflies are in pairs here: 512^3 281 ->
+// 244 us (4.4 TB/s), 256^3 35.2 -> 31.6, isolated 256^3 28.6 -> 25.9. (In passes B, D and E, which
+// wait for memory and shared memory, pairs gain nothing: D at 512 209 -> 224 us.) 80
+// registers keep three CTAs of 512 on an SM; a table takes their shared memory.
 template <int G, int MODE, bool HALF>
-__global__ void __launch_bounds__(kFftThreads) k_pass_c(float2* __restrict__ spec, const float2* __restrict__ tw_g,
-                                                        const float* __restrict__ gexp_g, float scale,
-                                                        const float* __restrict__ table, float table_scale) {
+__global__ void __launch_bounds__(kFftThreads, G == 512 && MODE == 0 ? 3 : 0)
+    k_pass_c(float2* __restrict__ spec, const float2* __restrict__ tw_g, const float* __restrict__ gexp_g, float scale,
+             const float* __restrict__ table, float table_scale) {
     wait_previous();
     using T = Geo<G>;
     constexpr int H = T::H;
@@ -939,13 +944,13 @@ __global__ void __launch_bounds__(kFftThreads) k_pass_c(float2* __restrict__ spe
     if (MODE == 0)
         for (int i = threadIdx.x; i <= H; i += kFftThreads) gexp[i] = gexp_g[i];
     __shared__ float line_g[16];
-    __shared__ int line_k2[16];
+    __shared__ float line_k2[16];
     if (MODE == 0 && threadIdx.x < 16) {
         const int l = threadIdx.x;
         const int kx = bx * 4 + (l & 3), ky = by * 4 + (l >> 2);
         const int kyf = (ky <= G / 2) ? ky : ky - G;
         line_g[l] = (kx <= H) ? -scale * (gexp_g[kx] * gexp_g[abs(kyf)]) : 0.f;  // the global table: no barrier yet
-        line_k2[l] = kx * kx + kyf * kyf;
+        line_k2[l] = (float)(kx * kx + kyf * kyf);
     }
     // MODE 2: the table's values of these 16 lines, 4 runs of H + 1 groups of 4 bins, come
     // into shared memory with the lines. Fetched at the multiply, each thread's 16 or 32
@@ -970,16 +975,19 @@ __global__ void __launch_bounds__(kFftThreads) k_pass_c(float2* __restrict__ spe
     }
     // forward, Green's function, inverse; the multiply happens in registers between
     // the forward's last stage and the inverse's first
-    auto green = [&](int l, int kz, float2 x) {
-        const int kzf = (kz <= G / 2) ? kz : kz - G;
+    auto green = [&](int l, int kz, bool upper, float2 x) {
+        const int kzf = upper ? G - kz : kz;  // |frequency|
         float m;
         if (MODE == 0) {
             // Green's function: -scale/k^2 * exp(-k^2 s^2/2), k = 0 -> 0 (Sim.cu:536-556), with
             // the per-line factors of (kx, ky) hoisted; padding columns kx > H are zeroed.
-            const int k2 = line_k2[l] + kzf * kzf;
-            m = (k2 != 0) ? __fdividef(line_g[l] * gexp[abs(kzf)], (float)k2) : 0.f;
+            // k^2 <= 3 * 256^2 is exact in a float.
+            const float k2 = fmaf((float)kzf, (float)kzf, line_k2[l]);
+            float inv;
+            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(k2));
+            m = (kz != 0 || k2 != 0.f) ? line_g[l] * gexp[kzf] * inv : 0.f;
         } else {
-            m = line_t[(l >> 2) * kRun + 4 * abs(kzf) + (l & 3)] * table_scale;
+            m = line_t[(l >> 2) * kRun + 4 * kzf + (l & 3)] * table_scale;
         }
         return make_float2(x.x * m, x.y * m);
     };
