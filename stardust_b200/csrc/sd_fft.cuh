@@ -1,11 +1,11 @@
 // sd_fft.cuh -- shared-memory Stockham FFT over 16 interleaved lines (sm_100a).
 //
 // A CTA holds 16 lines of N complex values in shared memory, interleaved:
-// element i of line l sits at s[i*16 + l]. All 16 lines are transformed at once.
-// Threads are mapped line-fastest (item u -> line u & 15, butterfly u >> 4), so
-// every load and store of every stage touches two runs of 16 consecutive
-// float2 per warp: the two-wavefront minimum for 8-byte accesses, with no
-// padding and no bank conflicts.
+// element i of line l sits at s[at(i, l)], in row i, of 16 float2. All 16 lines are
+// transformed at once. Threads are mapped line-fastest (item u -> line u & 15, butterfly
+// u >> 4), so every load and store of every stage touches two rows of 16 consecutive
+// float2 per warp: the two-wavefront minimum for 8-byte accesses, with no padding and no
+// bank conflicts.
 //
 // Stages are mixed radix (32 or 16 where every thread still gets a butterfly,
 // else 8, then 4 or 2 for the remainder) in the self-sorting
@@ -23,6 +23,16 @@
 
 namespace sd {
 namespace fft {
+
+// Element `pos` of line l. TURN: the lines of a row are turned by 4 (pos mod 4). Passes B and
+// D copy whole bricks in which 8 lanes take 16 bytes of four rows each: a 4-way bank
+// conflict where rows are not turned (512^3 207 and 209 us, turned 201 and 207; 256^3
+// 27.3 and 24.2). The others' copies have none (C) or small ones, and only pay for the turn
+// (isolated C 25.9 -> 27.2, E at 256 33.2 -> 34.1).
+template <bool TURN = false>
+__device__ __forceinline__ int at(int pos, int l) {
+    return pos * 16 + (TURN ? l ^ ((pos & 3) << 2) : l);
+}
 
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
     return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -194,14 +204,14 @@ constexpr int last_stage_ns(int N, int NT) {
 // caller's functor that forms it from what s holds (a pre-processing step fused
 // into the first stage's loads, saving a shared-memory round trip and a barrier).
 struct PlainLoad {
-    __device__ __forceinline__ float2 operator()(const float2* s, int l, int pos) const { return s[pos * 16 + l]; }
+    __device__ __forceinline__ float2 operator()(const float2* s, int l, int pos) const { return s[at(pos, l)]; }
 };
 
 // Stages from sub-transform length Ns on, stopping before the stage at STOP; the
 // stage at Ns = 1 reads through `load`. HALF: positions N/2 and up of the input are
 // zero and are not read (they are the upper half of the first stage's radix).
 template <int N, int Ns, int NT, int TWS, bool INV, int STOP = N, class Load = PlainLoad, bool HALF = false,
-          bool PAIR = false>
+          bool PAIR = false, bool TURN = false>
 __device__ __forceinline__ void stages16(float2* s, const float2* tw, Load load = Load()) {
     if constexpr (Ns < N && Ns < STOP) {
         constexpr int R = radix_of<N / Ns, N, NT>::value;
@@ -220,7 +230,7 @@ __device__ __forceinline__ void stages16(float2* s, const float2* tw, Load load 
                         v[p][r] = make_float2(0.f, 0.f);
                         continue;
                     }
-                    float2 x = (Ns == 1) ? load(s, l, j + r * NB) : s[(j + r * NB) * 16 + l];
+                    float2 x = (Ns == 1 && !TURN) ? load(s, l, j + r * NB) : s[at<TURN>(j + r * NB, l)];
                     if (Ns > 1 && r > 0) {
                         float2 w = tw[(k * r * (N / (Ns * R))) * TWS];
                         if (INV) w.y = -w.y;
@@ -239,19 +249,19 @@ __device__ __forceinline__ void stages16(float2* s, const float2* tw, Load load 
                 dft<R, INV, PAIR>(v[p]);
                 const int base = (j / Ns) * Ns * R + k;
 #pragma unroll
-                for (int r = 0; r < R; ++r) s[(base + r * Ns) * 16 + l] = v[p][r];
+                for (int r = 0; r < R; ++r) s[at<TURN>(base + r * Ns, l)] = v[p][r];
             }
         }
         __syncthreads();
-        stages16<N, Ns * R, NT, TWS, INV, STOP, PlainLoad, false, PAIR>(s, tw);
+        stages16<N, Ns * R, NT, TWS, INV, STOP, PlainLoad, false, PAIR, TURN>(s, tw);
     }
 }
 
 // Transform the 16 interleaved lines of length N in s. The caller synchronises
 // before the call; the routine ends with a barrier. HALF: the input's upper half is zero.
-template <int N, int NT, int TWS, bool INV, bool HALF = false>
+template <int N, int NT, int TWS, bool INV, bool HALF = false, bool TURN = false>
 __device__ __forceinline__ void lines16(float2* s, const float2* tw) {
-    stages16<N, 1, NT, TWS, INV, N, PlainLoad, HALF>(s, tw);
+    stages16<N, 1, NT, TWS, INV, N, PlainLoad, HALF, false, TURN>(s, tw);
 }
 
 // Forward transform, a pointwise multiply, inverse transform of the 16 lines.
@@ -279,7 +289,7 @@ __device__ __forceinline__ void convolve16(float2* s, const float2* tw, Mul mul)
             const int l = u & 15, j = u >> 4;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                float2 x = s[(j + r * NB) * 16 + l];
+                float2 x = s[at(j + r * NB, l)];
                 if (NsL > 1 && r > 0) x = cmul(x, tw[(j * r) * TWS]);
                 v[p][r] = x;
             }
@@ -296,7 +306,7 @@ __device__ __forceinline__ void convolve16(float2* s, const float2* tw, Mul mul)
             for (int r = 0; r < R; ++r) v[p][r] = mul(l, j + r * NsL, r >= R / 2, v[p][r]);
             dft<R, true, true>(v[p]);
 #pragma unroll
-            for (int r = 0; r < R; ++r) s[(j * R + r) * 16 + l] = v[p][r];
+            for (int r = 0; r < R; ++r) s[at(j * R + r, l)] = v[p][r];
         }
     }
     __syncthreads();
@@ -322,7 +332,7 @@ __device__ __forceinline__ void lines16_rows(float2* s, const float2* tw, Load l
             const int l = u & 15, j = u >> 4;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                float2 x = (NsL == 1) ? load(s, l, j + r * NB) : s[(j + r * NB) * 16 + l];
+                float2 x = (NsL == 1) ? load(s, l, j + r * NB) : s[at(j + r * NB, l)];
                 if (NsL > 1 && r > 0) {
                     float2 w = tw[(j * r) * TWS];
                     if (INV) w.y = -w.y;

@@ -863,7 +863,7 @@ __device__ __forceinline__ void load_lines(float2* s, const float2* __restrict__
         int dst;
         if (DIR == 1) {  // b = by
             src = T::brick(b0, b, b1) + e;
-            dst = (b * 4 + ((e >> 2) & 3)) * 16 + (e >> 4) * 4 + (e & 3);
+            dst = fft::at<true>(b * 4 + ((e >> 2) & 3), (e >> 4) * 4 + (e & 3));
         } else {  // b = bz: the brick lands contiguously
             src = T::brick(b0, b1, b) + e;
             dst = b * 64 + e;
@@ -885,7 +885,7 @@ __device__ __forceinline__ void store_lines(const float2* s, float2* __restrict_
         int src;
         if (DIR == 1) {
             dst = T::brick(bx, b, b1) + e;
-            src = (b * 4 + ((e >> 2) & 3)) * 16 + (e >> 4) * 4 + (e & 3);
+            src = fft::at<true>(b * 4 + ((e >> 2) & 3), (e >> 4) * 4 + (e & 3));
         } else {
             dst = T::brick(bx, b1, b) + e;
             src = b * 64 + e;
@@ -898,11 +898,11 @@ __device__ __forceinline__ void store_lines(const float2* s, float2* __restrict_
 // HALF (isolated boundary): the density fills the low corner of the box and the
 // potential is read only there, so the forward transform's inputs past half the box
 // are zero (never written, not read) and the inverse's outputs past it are not
-// stored; the grid covers the lower half of the z slabs. At 512 the pruned forward
-// transform takes 85 registers left alone, two CTAs an SM; bounded to three 112 -> 102 us
-// (the other instances have three by themselves).
+// stored; the grid covers the lower half of the z slabs. At 512 the
+// transforms take 85 to 96 registers left alone, two CTAs an SM (240 us); bounded to
+// three 201 (B) and 208 (D), 5.3 TB/s, the pruned one 102.
 template <int G, bool INV, bool HALF>
-__global__ void __launch_bounds__(kFftThreads, G == 512 && HALF && !INV ? 3 : 0)
+__global__ void __launch_bounds__(kFftThreads, G == 512 ? 3 : 0)
     k_pass_y(float2* __restrict__ spec, const float2* __restrict__ tw_g) {
     wait_previous();
     extern __shared__ float2 sm[];
@@ -912,7 +912,7 @@ __global__ void __launch_bounds__(kFftThreads, G == 512 && HALF && !INV ? 3 : 0)
     const int bx = blockIdx.x, bz = blockIdx.y ^ (INV ? 0 : Geo<G>::NBZ / (HALF ? 2 : 1) - 1);
     for (int i = threadIdx.x; i < G; i += kFftThreads) tw[i] = tw_g[i];
     load_lines<G, 1, HALF && !INV>(s, spec, bx, bz);
-    fft::lines16<G, kFftThreads, 1, INV, HALF && !INV>(s, tw);
+    fft::lines16<G, kFftThreads, 1, INV, HALF && !INV, true>(s, tw);
     store_lines<G, 1, HALF && INV>(s, spec, bx, bz);
 }
 
