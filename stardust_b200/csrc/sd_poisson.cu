@@ -466,6 +466,19 @@ __global__ void __launch_bounds__(256) k_deposit_plan(const int* __restrict__ rs
     int sum;
     const int excl = block_excl_scan256(extra, &sum);
     if (b < P::NB) w[P::kXpre + b] = excl;
+    if constexpr (P::NC == 1) {
+        // up to 64^3 one block has it all: 2.4 us, 4.2 with the exchange below
+        if (threadIdx.x == 0) {
+            w[P::kCtaPre] = 0;
+            w[P::kCtaPre + 1] = sum;
+            w[P::kTicket] = 0;
+            if (kMayStray) {  // every thread has read the flag
+                w[P::kUse] = stray;
+                w[P::kStray] = 0;
+            }
+        }
+        return;
+    }
     if (threadIdx.x == 0) w[P::kCtaSum + blockIdx.x] = sum;
     __shared__ bool last;
     __threadfence();
