@@ -424,7 +424,7 @@ def run_ensemble(rank, world, steps: int = 100, warmup: int = 3, dt: float = 1e-
             "scenes": len(members), "particles": int(n_total),
             "grids": {str(g): sum(1 for m in members if m["grid"] == g) for g in (32, 64, 128)},
             "graph_launches_per_step": 1, "kernels_per_graph_rank0": kernels,
-            "autotune": {"seconds": tune_s, "tiled_deposit_scenes": tiled, "atomic_deposit_scenes": len(tuning) - tiled,
+            "autotune": {"seconds": tune_s, "tiled_deposit_scenes": tiled, "rowmajor_deposit_scenes": len(tuning) - tiled,
                          "deposit_share_particles": sorted({tt["deposit_split"] for tt in tuning if tt["order"] == "tiled"}),
                          "gather_caps": sorted({tt["gather_blocks"] for tt in tuning})},
             "partition": f"LPT over {world} rank(s)"}
@@ -569,7 +569,7 @@ def main(argv=None) -> int:
     if world == 1 and not args.no_configs:
         # the other single-scene configurations (the headline's workload is cosmic_web_512)
         out["configs"] = {w: time_workload(w) for w in ("disk_64", "two_galaxy_256") if w != args.workload}
-        # the reference's own particle order (row-major cell keys, the atomic deposit) and
+        # the reference's own particle order (row-major cell keys) and
         # the 30-bit Morton order on the headline workload
         out["orders"] = {o: time_workload(args.workload, order=k, steps=10) for k, o in ((0, "rowmajor"), (1, "morton"))}
     if not args.no_ensemble:

@@ -9,8 +9,8 @@
 // step. Two graphs are kept, one per parity of the ping-pong particle buffers.
 //
 // The autotuner times, for every scene, each combination of
-//   deposit path  : fused tiled (pass A deposits from the row table) or
-//                   int64 atomics (row-major sort, separate deposit kernel)
+//   deposit path  : the tiled order (narrow windows of the row table) or the
+//                   row-major one (wide windows, longer keys)
 //   deposit share : for the fused path, the window particles one CTA takes before
 //                   a heavy bundle is split among several (3, 10 or 30 times the
 //                   mean window)
