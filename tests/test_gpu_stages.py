@@ -77,9 +77,13 @@ def test_sort_permutation_bit_exact(cuda, lib, oracle, n):
 
 
 # tiles of 2048 keys: one, a run of the column scan less one and just past it, a second
-# round of it, its last tile count and the first that takes the chunked scan
+# round of it, each side of where three digits are counted anew, the last tile count of it
+# and the first that takes the chunked scan
 @pytest.mark.parametrize("bits", [10, 18, 25])
-@pytest.mark.parametrize("tiles,extra", [(1, 0), (32, -5), (33, 1), (512, 0), (513, -2000), (2048, 0), (2048, 1)])
+@pytest.mark.parametrize(
+    "tiles,extra",
+    [(1, 0), (32, -5), (33, 1), (512, 0), (513, -2000), (767, 0), (768, -1), (2048, 0), (2048, 1)],
+)
 def test_sort_across_column_scans(cuda, lib, bits, tiles, extra):
     n = tiles * 2048 + extra
     gen = cuda.Generator(device="cuda").manual_seed(n + bits)
