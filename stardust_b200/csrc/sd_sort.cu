@@ -10,7 +10,9 @@
 //      k_digit_counts counts each tile in shared memory and writes one coalesced
 //      row; every later pass gets its counts from the scatter before it, which
 //      knows where each key lands and adds one count per (tile, digit) run of a
-//      warp into a zeroed buffer, so the keys are not read an extra time;
+//      warp into a zeroed buffer, so the keys are not read an extra time (keys of three
+//      digits, which gives hardly any runs, are counted for every pass from
+//      kRecountTiles tiles on);
 //   2. a column scan over tiles gives, for every (tile, digit), the global output
 //      offset: all keys of smaller digits plus the same digit's keys in earlier
 //      tiles, which is what makes the result stable across tiles. Up to
