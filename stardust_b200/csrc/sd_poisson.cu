@@ -578,11 +578,15 @@ __device__ __forceinline__ void deposit_bundle(int b, int slice, int items, cons
     const int total = from_grid ? 0 : r_off[NR];  // from_grid: the sums are in the fixed-point grid
     const int f_lo = SHARED ? (int)((long long)total * slice / items) : 0;
     const int f_hi = SHARED ? (int)((long long)total * (slice + 1) / items) : total;
-    // A weight q <= 2^32 is added as (q >> 16) into the high word and (q & 0xffff)
-    // into the low word: with fewer than 2^16 particles in this share neither 32-bit
-    // sum can overflow, so plain adds keep the 64-bit total exact. Larger shares
-    // add the low 32 bits and carry into the high word instead.
-    const bool split16 = f_hi - f_lo < 65536;
+    // A weight q <= 2^32 is added as (q >> kSplit) into the high word and the bits below into
+    // the low word: with fewer than 2^kSplit particles in this share neither 32-bit sum can
+    // overflow, so plain adds keep the 64-bit total exact. Larger shares add the low 32 bits
+    // and carry into the high word instead. Periodic corners are eight cells, so a particle
+    // adds to a cell once and the sums stay at or below 2^16 (2^16 - 1). Clamped corners
+    // coincide, up to eight in one cell and 2^32 together: the low sums stay at or below
+    // 8 (2^14 - 1)^2 < 2^31, the high ones at or below 2^18 (2^14 - 1).
+    constexpr int kSplit = ISO ? 14 : 16;
+    const bool split = f_hi - f_lo < (1 << kSplit);
     const int lane = threadIdx.x & 31;
     constexpr int kBatch = 4;
     // lane f = base + q * NT + lane
@@ -651,9 +655,9 @@ __device__ __forceinline__ void deposit_bundle(int b, int slice, int items, cons
                     const unsigned long long qv =
                         (unsigned long long)__float2ll_rn(__fmul_rn(__fmul_rn(wx[ox], wy[oy]), wz[oz]));
                     const int c = row + (ox ? x1 : x0);
-                    if (split16) {
-                        atomicAdd(acc_hi + c, (unsigned)(qv >> 16));
-                        atomicAdd(acc_lo + c, (unsigned)(qv & 0xffffu));
+                    if (split) {
+                        atomicAdd(acc_hi + c, (unsigned)(qv >> kSplit));
+                        atomicAdd(acc_lo + c, (unsigned)qv & ((1u << kSplit) - 1u));
                     } else {
                         // atomicAdd returns the previous low word, so every wrap is seen by
                         // exactly one add
@@ -667,7 +671,7 @@ __device__ __forceinline__ void deposit_bundle(int b, int slice, int items, cons
         }
     }
     __syncthreads();
-    int sh = split16 ? 16 : 32;  // value of a cell: (hi << sh) + lo
+    int sh = split ? kSplit : 32;  // value of a cell: (hi << sh) + lo
     if (SHARED && (items > 1 || from_grid)) {
         // a shared bundle: every CTA adds its rows into the fixed-point grid; the last
         // to arrive reads the complete sums back (and leaves the grid zero)
