@@ -758,6 +758,9 @@ int reconfigure(sd_sim* s, const sd_config* c) {
             if (s->active > s->N) s->active = s->N;
             s->rho_valid = false;
             invalidate_keys(s);  // the sort covers a shorter range
+            // the workspace is laid out by the range: counts that the last gather left would
+            // lie in the second count buffer, which a sort takes as zero
+            if (SD_CUDA(cudaMemsetAsync(s->sort_ws, 0, s->sort_ws_bytes, s->stream))) return sim_error(s, SD_E_CUDA);
             // change bits of slots past the new range must not reach a merge
             if (s->rs_base &&
                 SD_CUDA(cudaMemsetAsync(s->rs.words, 0, sizeof(unsigned) * resort_words(s->capacity), s->stream)))

@@ -592,3 +592,29 @@ def test_merge_sort_across_sort_interval_changes(cuda):
     for (p0, v0), (p1, v1) in zip(outs[0], outs[1]):
         assert np.array_equal(p0.view(np.int32), p1.view(np.int32))
         assert np.array_equal(v0.view(np.int32), v1.view(np.int32))
+
+
+# two digit passes (row-major and tiled 64^3), three (row-major 128^3), the chunked scan (10M)
+@pytest.mark.parametrize("order,G,n,share", [(L.SD_ORDER_ROWMAJOR, 64, 40_000, 0.75), (L.SD_ORDER_ROWMAJOR, 64, 40_000, 0.4),
+                                             (L.SD_ORDER_ROWMAJOR, 128, 300_000, 0.4), (L.SD_ORDER_MORTON, 64, 50_000, 0.1),
+                                             (L.SD_ORDER_TILED, 64, 100_000, 0.2), (L.SD_ORDER_TILED, 256, 10_500_000, 0.45)])
+def test_steps_after_narrowing_the_range(cuda, order, G, n, share):
+    """A request for fewer particles narrows the range and lays the sort's workspace out anew,
+    over counts that the last step's gather left: the steps after it equal a fresh handle's."""
+    m = int(n * share)
+    pos, vel = random_particles(n, 5, empty_every=97, clustered=True)
+    kw = dict(gravity=5.0, softening_cells=1.0, order=order, full_sort=1)
+    with make_sim(cuda, n, G, **kw) as s:
+        s.set_particles(pos, vel)
+        s.steps(1e-3, 3)
+        p, v = s.get_particles()
+        s.reconfigure(SimConfig(particle_count=m, grid_size=G, **kw))
+        assert s.particle_count() == m and s.particle_capacity() == n
+        s.steps(1e-3, 3)
+        got = s.get_particles()
+    with make_sim(cuda, m, G, **kw) as t:
+        t.set_particles(p[:m], v[:m])
+        t.steps(1e-3, 3)
+        want = t.get_particles()
+    assert np.array_equal(got[0].view(np.int32), want[0].view(np.int32))
+    assert np.array_equal(got[1].view(np.int32), want[1].view(np.int32))
