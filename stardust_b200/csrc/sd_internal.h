@@ -82,7 +82,7 @@ struct PoissonIso {
 // particles of the rows whose stencils reach its 16 rows (25 base rows in the tiled
 // order, 36 cell rows in the row-major order, `wide`; row_start then points at the
 // row table's entry 1, the first row); a bundle whose
-// window holds more than `split` particles is shared by several CTAs, which add
+// window holds more than `split` particles is shared by CTAs of `piece` each, which add
 // their exact int64 partial rows into `acc` (the fixed-point grid, zero between
 // uses) and the last of them to finish transforms the rows. `ints` is scratch of
 // deposit_work_ints(G) ints, zeroed once when allocated and left zero by every use.
@@ -90,14 +90,16 @@ struct DepositWork {
     long long* acc = nullptr;
     int* ints = nullptr;
     int split = 0;
+    int piece = 0;  // at most split
     bool wide = false;
     int n = 0;  // particles
 };
 size_t deposit_work_ints(int G);
 int* deposit_stray_flag(int* ints, int G);
-// the particles per CTA above which a window is split: mult times a window's mean count
-// (mult 0: by the grid's side)
-int deposit_split(int n, int G, int mult = 0);
+// the particles above which a window is split, and of each share: mult times a window's mean count
+int deposit_split(int n, int G, int mult);
+// split and piece by the grid's side
+void deposit_shares(DepositWork& w, int n, int G);
 int launch_poisson_ex(const PoissonPlan& p, const long long* acc, const float* rho, const float4* pos,
                       const int* perm, const int* row_start, float* keep, float2* spec, float* phi, cudaStream_t s,
                       cudaEvent_t* ev = nullptr, const PoissonIso* iso = nullptr, const DepositWork* dw = nullptr);

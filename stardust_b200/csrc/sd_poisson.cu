@@ -426,7 +426,7 @@ __device__ __forceinline__ int block_excl_scan256(int v, int* total) {
     return excl;
 }
 
-// How many CTAs share each bundle: ceil(window particles / split), at least 1,
+// How many CTAs share each bundle: ceil(window particles / piece) above split, else 1,
 // and where each bundle's extra CTAs start. The last block to finish turns the
 // block totals into their prefix.
 //
@@ -439,7 +439,7 @@ __device__ __forceinline__ int block_excl_scan256(int v, int* total) {
 // after a load; its speed does not matter, its not costing the others a launch does.
 template <int G, bool WIDE, bool ISO>
 __global__ void __launch_bounds__(256) k_deposit_plan(const int* __restrict__ rs, int* __restrict__ w, int split,
-                                                      const float4* __restrict__ pos, int n,
+                                                      int piece, const float4* __restrict__ pos, int n,
                                                       unsigned long long* __restrict__ acc) {
     wait_previous();
     using P = DepPlan<G>;
@@ -459,7 +459,7 @@ __global__ void __launch_bounds__(256) k_deposit_plan(const int* __restrict__ rs
             window_range<G, WIDE, ISO>(b, r, rs, lo, hi);
             total += hi - lo;
         }
-        const int items = total > split ? (int)(((long long)total + split - 1) / split) : 1;
+        const int items = total > split ? (int)(((long long)total + piece - 1) / piece) : 1;
         w[P::kItems + b] = items;
         extra = items - 1;
     }
@@ -523,6 +523,7 @@ struct DepGeo {
 
 template <int G>
 constexpr bool kDepositLoop = G == 512;
+constexpr int kIsoShare = (1 << 14) - 1;  // most particles of an isolated share (deposit_bundle)
 template <int G>
 constexpr int kDepositPerSm = G >= 128 ? 3 : 2;
 
@@ -584,9 +585,12 @@ __device__ __forceinline__ void deposit_bundle(int b, int slice, int items, cons
     // and carry into the high word instead. Periodic corners are eight cells, so a particle
     // adds to a cell once and the sums stay at or below 2^16 (2^16 - 1). Clamped corners
     // coincide, up to eight in one cell and 2^32 together: the low sums stay at or below
-    // 8 (2^14 - 1)^2 < 2^31, the high ones at or below 2^18 (2^14 - 1).
+    // 8 (2^14 - 1)^2 < 2^31, the high ones at or below 2^18 (2^14 - 1), and windows are split so
+    // that no isolated share is larger (a step of 1,000,000 on 16^3 345 us
+    // with the carry, 127 without).
     constexpr int kSplit = ISO ? 14 : 16;
-    const bool split = f_hi - f_lo < (1 << kSplit);
+    static_assert(!ISO || kIsoShare < (1 << kSplit), "an isolated share never carries");
+    const bool split = ISO || f_hi - f_lo < (1 << kSplit);
     const int lane = threadIdx.x & 31;
     constexpr int kBatch = 4;
     // lane f = base + q * NT + lane
@@ -1126,13 +1130,16 @@ struct Launcher {
     static int deposit(const PoissonPlan& p, const float4* pos, const int* perm, const int* row_start, float* keep,
                        float2* spec, const DepositWork& dw, cudaStream_t s) {
         using P = DepPlan<DepGeo<G, ISO>::M>;
-        launch(k_deposit_plan<DepGeo<G, ISO>::M, WIDE, ISO>, P::NC, 256, 0, s,
-            row_start, dw.ints, dw.split, pos, dw.n, reinterpret_cast<unsigned long long*>(dw.acc));
+        // an isolated share is one that the plain sums hold (kIsoShare)
+        const int split = ISO && dw.split > kIsoShare ? kIsoShare : dw.split;
+        const int piece = dw.piece > split ? split : dw.piece;
+        launch(k_deposit_plan<DepGeo<G, ISO>::M, WIDE, ISO>, P::NC, 256, 0, s, row_start, dw.ints, split, piece, pos, dw.n,
+               reinterpret_cast<unsigned long long*>(dw.acc));
         SD_LAUNCHED(s);
         // a CTA for each extra share that there can be, so none waits for another (a window of
-        // w particles has at most w / split extra shares, and a particle lies in at most four
+        // w particles has at most w / piece extra shares, and a particle lies in at most four
         // windows); idle ones cost little, 1.5 us for 1,024. Never more than are taken by ticket.
-        const long long extra = 4ll * dw.n / dw.split, wave = 148 * kDepositPerSm<G>;
+        const long long extra = 4ll * dw.n / piece, wave = 148 * kDepositPerSm<G>;
         const long long ctas = P::NB + (extra < 8 ? 8 : extra);
         launch(k_pass_a_deposit_bal<G, ISO, WIDE>, (unsigned)(kDepositLoop<G> && ctas > wave ? wave : ctas), kDepositThreads,
                                              smem_bal<ISO>(), s, pos, perm, row_start, keep, spec, p.tw, dw);
@@ -1185,7 +1192,7 @@ struct Launcher {
         const int hy = half ? T::NBY / 2 : T::NBY, hz = half ? T::NBZ / 2 : T::NBZ;
         const dim3 grid_rows(hy, hz), grid_y(T::NBX, hz), grid_z(T::NBX, T::NBY);
         if (pos) {
-            if (!dw || !dw->acc || !dw->ints || dw->split <= 0) return fail(SD_E_ARG, "fused deposit: no work plan");
+            if (!dw || !dw->acc || !dw->ints || dw->split <= 0 || dw->piece <= 0) return fail(SD_E_ARG, "fused deposit: no work plan");
             int rc = SD_OK;
             if constexpr (kIsoBox) {
                 if (half)
@@ -1286,17 +1293,33 @@ size_t deposit_work_ints(int G) {
 int* deposit_stray_flag(int* ints, int G) { return ints + deposit_work_ints(G) - 1; }
 
 int deposit_split(int n, int G, int mult) {
-    // By default three times a window's mean particle count up to 256 bundles, which are
-    // resident all at once, so the time is the heaviest share's; six times at 1024, ten times
-    // above, where shares cost more than they balance (each adds its rows with global
-    // atomics); at least 2048. 262,144 particles of a disk on 64^3: 31 us with 5x, 19.5 with
-    // 3x, 19.4 with 2x; 1,000,003 on an isolated 128^3 74 us with 10x, 67 with 6x, 64 with
-    // 4x, but 2,000,000 of a ball 62, 64 and 69; 4M on 256^3 (two galaxies) 154 with 10x and
-    // 6x, 160 with 4x.
     const long long nb = (long long)G * G / 16;
-    if (mult <= 0) mult = nb <= 256 ? 3 : (nb <= 1024 ? 6 : 10);
     const long long t = (long long)mult * (long long)n / (nb > 0 ? nb : 1);
     return (int)(t < 2048 ? 2048 : (t > (1 << 30) ? (1 << 30) : t));
+}
+
+void deposit_shares(DepositWork& w, int n, int G) {
+    // Three times a window's mean particle count at 256 bundles, which are resident all at
+    // once, so the time is the heaviest share's; six times at 1024, ten times above, where
+    // shares cost more than they balance (each adds its rows with global atomics); at least
+    // 2048. 262,144 particles of a disk on 64^3: 31 us with 5x, 19.5 with 3x, 19.4 with 2x;
+    // 1,000,003 on an isolated 128^3 74 us with 10x, 67 with 6x, 64 with 4x, but 2,000,000 of
+    // a ball 62, 64 and 69; 4M on 256^3 (two galaxies) 154 with 10x and 6x, 160 with 4x.
+    const int nb = G * G / 16;
+    w.split = w.piece = deposit_split(n, G, nb <= 256 ? 3 : (nb <= 1024 ? 6 : 10));
+    if (nb > 64) return;
+    // The 16 or 64 bundles of 16^3 and 32^3 leave most of the chip idle, and a CTA that adds
+    // thousands of particles to a few cells alone takes longer than global atomics from the
+    // whole chip would. So a window is split into shares that fill the chip once between them,
+    // where it holds enough to pay for their atomics: more than an even spread gives up to
+    // some 50,000 particles on 16^3 and 170,000 on 32^3, less above. A step on 16^3 in
+    // row-major and tiled order, with the rule above and now: 100,000 spread evenly 57 and 39
+    // us, 41 and 31; on the edge of an isolated box 130 and 167, 47 and 45 (101 and 88 with
+    // global atomics). 1,000,000 on 32^3: 128 and 82 us, 97 and 68; 20,000 there 38 and 28,
+    // the same.
+    const int most = n / 48 > 6144 ? n / 48 : 6144;
+    w.split = n / 24 < 2048 ? 2048 : (n / 24 > most ? most : n / 24);
+    w.piece = n / 128 > 512 ? n / 128 : 512;
 }
 
 size_t poisson_spectrum_elems(int G) { return (size_t)G * G * (size_t)(G / 2 + 4); }

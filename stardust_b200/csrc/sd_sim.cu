@@ -518,7 +518,7 @@ int do_field(sd_sim* s, bool keep) {
         if ((rc = launch_row_bounds(s->keys2, s->N, row_last(s->G, SD_ORDER_TILED), -1, rows, s->stream))) return rc;
         dw.acc = s->acc;
         dw.ints = s->dep_ints;
-        dw.split = deposit_split(s->N, s->G);
+        deposit_shares(dw, s->N, s->G);
         dw.n = s->N;
     } else if ((rc = launch_deposit_fixed(s->pos, s->N, s->G, s->acc, s->stream, isolated(s) ? 0 : 1))) {
         return rc;
@@ -597,7 +597,10 @@ int do_step(sd_sim* s, float dt, bool sort, bool timed) {
     DepositWork dw;
     dw.acc = s->acc;
     dw.ints = s->dep_ints;
-    dw.split = s->dep_split > 0 ? s->dep_split : deposit_split(s->N, s->G, s->dep_mult);
+    if (s->dep_split > 0 || s->dep_mult > 0)
+        dw.split = dw.piece = s->dep_split > 0 ? s->dep_split : deposit_split(s->N, s->G, s->dep_mult);
+    else
+        deposit_shares(dw, s->N, s->G);
     dw.wide = wide;
     dw.n = s->N;
     if ((rc = launch_poisson_ex(s->plan, fused ? nullptr : s->acc, nullptr, fused ? s->pos : nullptr, perm,

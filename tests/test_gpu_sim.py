@@ -618,3 +618,27 @@ def test_steps_after_narrowing_the_range(cuda, order, G, n, share):
         want = t.get_particles()
     assert np.array_equal(got[0].view(np.int32), want[0].view(np.int32))
     assert np.array_equal(got[1].view(np.int32), want[1].view(np.int32))
+
+
+# windows of 2,048 and 2,049 particles (the rule's lower end on 16^3 and 32^3), one cell
+# shared by many CTAs, even spreads on both sides of the rule's upper end
+@pytest.mark.parametrize("boundary", [L.SD_BOUNDARY_PERIODIC, L.SD_BOUNDARY_ISOLATED])
+@pytest.mark.parametrize("G,n,pile", [(16, 30_000, 2_048), (16, 30_000, 2_049), (16, 60_000, 60_000), (16, 60_001, 0),
+                                      (32, 150_001, 0), (32, 400_000, 1_000), (32, 49_152, 40_000)])
+def test_deposit_shares_of_small_grids(cuda, boundary, G, n, pile):
+    """However the bundles of a small grid are shared among CTAs, the density is the Morton
+    order's (int64 atomics) bit for bit; `pile` particles sit in one cell."""
+    pos, vel = random_particles(n, G + pile, empty_every=61)
+    live = np.nonzero(pos[:, 0] >= 0)[0][:pile]
+    pos[live, :3] = (np.random.default_rng(1).uniform(0.05, 0.95, (len(live), 3)) + G // 2) / G
+    if pile:
+        rest = np.setdiff1d(np.nonzero(pos[:, 0] >= 0)[0], live)
+        pos[rest, 1:3] *= 0.25  # away from the pile's bundle
+    rho = {}
+    for order in (L.SD_ORDER_MORTON, L.SD_ORDER_ROWMAJOR, L.SD_ORDER_TILED):
+        with make_sim(cuda, n, G, gravity=1.0, softening_cells=1.0, order=order, boundary=boundary) as s:
+            s.set_particles(pos, vel)
+            s.step(1e-6)
+            rho[order] = s.density()
+    for order in (L.SD_ORDER_ROWMAJOR, L.SD_ORDER_TILED):
+        assert np.array_equal(rho[order].view(np.int32), rho[L.SD_ORDER_MORTON].view(np.int32))
