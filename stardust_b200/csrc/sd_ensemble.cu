@@ -109,7 +109,9 @@ void restore_counters(sd_sim* s, const HostCounters& c) {
 }
 
 // Everything a step needs that must not be inside the graph: leapfrog opening
-// kicks, and keys and first-pass sort counts of unsorted buffers.
+// kicks, and keys and first-pass sort counts where the last step's are not there any
+// more (particles loaded, a field on 512^3 that sorted for itself). Before every replay:
+// a scene may have been used on its own since the last one.
 int prepare_scenes(sd_ensemble* e, float dt) {
     for (auto& sl : e->scenes) {
         sd_sim* s = sl.sim;
@@ -411,11 +413,9 @@ int sd_ensemble_steps(sd_ensemble* e, float dt, int nsteps) {
     if (nsteps < 0) return fail(SD_E_ARG, "ensemble_steps: negative count");
     if (e->scenes.empty() || nsteps == 0) return SD_OK;
     DeviceGuard g(e->device);
+    if (int rc = prepare_scenes(e, dt)) return rc;
     // the graphs are stale when dt changed or a scene was stepped or changed on its own
     if (e->graph[0] && !graphs_current(e, dt)) drop_graphs(e);
-    if (!e->graph[0]) {
-        if (int rc = prepare_scenes(e, dt)) return rc;
-    }
     // work issued on the scenes' own streams so far (particle uploads, opening
     // kicks, keys) precedes the replays
     for (auto& sl : e->scenes) {

@@ -147,3 +147,50 @@ def test_ensemble_one_graph_launch_per_step(cuda):
         ens.synchronize()
         assert Sim.kernel_launches() - before == 5 * k
         assert all(ens.scene(i).step_count() == 7 for i in range(len(members)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("order", [L.SD_ORDER_TILED, L.SD_ORDER_ROWMAJOR])
+@pytest.mark.parametrize("ask", ["accel", "density", "load"])
+def test_ensemble_scenes_used_between_replays(cuda, order, ask):
+    """A replayed step sorts by keys and counts that the step before it left. Forces and
+    densities of a 512^3 scene sort in the same workspace, and loading particles makes the
+    keys stale: the next replays start from what the scene holds then."""
+    from stardust_b200.ensemble import Ensemble, member_config
+    from stardust_b200.scenes import disk_galaxy
+    from stardust_b200.sim import Sim
+
+    dt, scenes = 1e-3, [(60_000, 512, 11), (20_000, 32, 12)]
+    new = [disk_galaxy(n, seed + 7) for n, _, seed in scenes]
+
+    def config(n, G):
+        c = member_config({"n": n, "grid": G}, keep_density=1)
+        c.order = order
+        return c
+
+    with Ensemble(0) as ens:
+        for n, G, seed in scenes:
+            ens.add(config(n, G), *disk_galaxy(n, seed))
+        ens.steps(dt, 2)
+        for i in range(len(scenes)):
+            if ask == "load":
+                ens.scene(i).set_particles(*new[i])
+            elif ask == "accel":
+                ens.scene(i).accel()
+            else:
+                ens.scene(i).set_particles(*ens.scene(i).get_particles())
+                ens.scene(i).density()
+        ens.steps(dt, 2)
+        ens.synchronize()
+        got = [ens.scene(i).get_particles() for i in range(len(scenes))]
+    for (n, G, seed), (p, v), fresh in zip(scenes, got, new):
+        with Sim(0) as s:
+            s.init(config(n, G))
+            s.set_particles(*(fresh if ask == "load" else disk_galaxy(n, seed)))
+            for k in range(2 if ask == "load" else 4):
+                if k == 2 and ask == "density":
+                    s.set_particles(*s.get_particles())
+                s.step(dt)
+            sp, sv = s.get_particles()
+        assert np.array_equal(p.view(np.int32), sp.view(np.int32))
+        assert np.array_equal(v.view(np.int32), sv.view(np.int32))
