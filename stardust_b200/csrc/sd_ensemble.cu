@@ -35,10 +35,10 @@ namespace {
 constexpr int kSmCount = 148;
 // Deposit share of an untuned scene, times a window's mean particle count (0: as for a
 // simulation alone). Many scenes fill the GPU, and splitting heavy windows then costs more
-// work than its balance gives. Five steps of scenes of 16,384 to 1,048,576 particles with
-// the solo share, 10x and 30x: 64 scenes 8.76, 8.49 and 8.34 ms, 32 scenes 4.07, 3.93 and
-// 3.85, 16 scenes 2.09, 2.04 and 2.05, 8 scenes 1.19, 1.19 and 1.32; 12 of 8,192 to 65,536
-// 0.47, 0.48 and 0.55.
+// work than its balance gives. A step with the solo share, 10x and 30x, in us: scenes of
+// 16,384 to 1,048,576 particles, 64: 1735, 1691 and 1649; 30: 811, 788 and 764; 16: 412, 403
+// and 392; 8: 225, 222 and 229. Of 8,192 to 65,536, 64: 583, 576 and 576; 30: 203, 200 and
+// 197; 16: 107, 105 and 105; 12: 86, 85 and 85; 4: 53, 54 and 58. 30 of 8,192: 142, 141, 141.
 int scene_share(size_t scenes) { return scenes >= 24 ? 30 : (scenes >= 16 ? 10 : 0); }
 
 struct SceneSlot {
@@ -117,7 +117,6 @@ int prepare_scenes(sd_ensemble* e, float dt) {
         sd_sim* s = sl.sim;
         if (!graphable(s))
             return fail(SD_E_STATE, "ensemble: scenes must sort every step or never, without hydro add-ons");
-        s->dep_mult = scene_share(e->scenes.size());
         if (s->cfg.integrator == SD_INT_KDK && !s->lf_open) {
             if (int rc = do_step(s, dt, sort_due(s), false)) return rc;
         }
@@ -136,7 +135,9 @@ int capture_step(sd_ensemble* e, float dt, int par, cudaGraphExec_t* out) {
         if (rc) break;
         sd_sim* s = sl.sim;
         rc = SD_CUDA(cudaStreamWaitEvent(s->stream, e->fork, 0));
+        s->dep_mult = scene_share(e->scenes.size());  // not for steps that the scene takes alone
         if (!rc) rc = do_step(s, dt, s->cfg.sort_interval == 1, false);
+        s->dep_mult = 0;
         if (!rc) rc = SD_CUDA(cudaEventRecord(sl.join, s->stream));
         if (!rc) rc = SD_CUDA(cudaStreamWaitEvent(e->stream, sl.join, 0));
         sl.pos_after[par] = s->pos;
@@ -376,6 +377,7 @@ int sd_ensemble_autotune(sd_ensemble* e, float dt, int reps) {
                     s->cfg.order = orders[o];
                     s->dep_split = orders[o] == SD_ORDER_TILED ? deposit_split(s->N, s->G, mults[m]) : 0;
                     s->gather_blocks = caps[c];
+                    s->dep_mult = scene_share(e->scenes.size());  // the row-major share that the graphs take
                     rc = restore_snapshot(s, sn);
                     float ms = 0.f;
                     if (!rc) rc = time_scene(s, dt, reps, a, b, &ms);
@@ -386,6 +388,7 @@ int sd_ensemble_autotune(sd_ensemble* e, float dt, int reps) {
                         best_split = s->dep_split;
                     }
                 }
+        s->dep_mult = 0;
         s->cfg.order = best_order;
         s->gather_blocks = best_cap;
         s->dep_split = best_split;

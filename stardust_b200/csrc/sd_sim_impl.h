@@ -100,7 +100,7 @@ struct sd_sim {
 
     int gather_blocks = 0;   // cap of the gather grid (0: the default); set by the ensemble autotuner
     int dep_split = 0;       // window particles per CTA share of the fused deposit (0: deposit_split of dep_mult)
-    int dep_mult = 0;        // ... times a window's mean count (0: by the grid's side); set by the ensemble
+    int dep_mult = 0;        // ... times a window's mean count (0: deposit_shares); set while the ensemble captures or tunes
 
     // per-step FP64 diagnostics ring (cfg.diagnostics): kDiagCap records of 8 doubles
     double* diag_rec = nullptr;
