@@ -57,7 +57,10 @@ struct PoissonPlan {
     float* gexp = nullptr;   // exp(-(2 pi soft / G)^2 k^2 / 2), k = 0..G/2 (FP64-built)
     float scale = 0.f;       // 1 / (4 pi^2 G^3)
 };
-int poisson_plan_build(PoissonPlan& p, int G, float soft);
+// what the plan's kernels will be launched for: a density grid (periodic), a periodic or an
+// isolated simulation (G: the transform box)
+enum class PoissonUse { kGrid, kPeriodic, kIsolated };
+int poisson_plan_build(PoissonPlan& p, int G, float soft, PoissonUse use);
 void poisson_plan_free(PoissonPlan& p);
 size_t poisson_spectrum_elems(int G);  // complex elements of the (bricked, padded) spectrum buffer
 // rho_fixed != nullptr: the first pass reads the int64 fixed-point grid and

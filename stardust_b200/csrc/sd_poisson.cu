@@ -1149,7 +1149,10 @@ struct Launcher {
 
     static constexpr bool kIsoBox = G >= 32;  // the transform box of an isolated grid of side G / 2 >= 16
 
-    static int configure() {
+    // The kernels that a plan's use launches, and no others: setting an attribute loads the
+    // kernel. All fifteen took a process's first simulation from 11.0 to 13.6 ms (2,000,000
+    // on 128^3), an isolated one from 13.3 to 14.9; these take 12.5 and 13.4.
+    static int configure(PoissonUse use) {
         int rc = SD_OK;
         // prefer the largest shared-memory carveout so several 70 KB CTAs fit per SM
         auto set = [&rc](auto* kernel, size_t smem) {
@@ -1157,22 +1160,27 @@ struct Launcher {
                                                (int)cudaSharedmemCarveoutMaxShared));
             rc |= SD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         };
-        set(k_pass_a<G, 0>, smem_a());
-        set(k_pass_a<G, 1>, smem_a());
+        if (use != PoissonUse::kPeriodic) set(k_pass_a<G, 0>, smem_a());
+        if (use != PoissonUse::kGrid) set(k_pass_a<G, 1>, smem_a());
         set(k_pass_y<G, false, false>, smem_bd());
-        set(k_pass_y<G, true, false>, smem_bd());
-        set(k_pass_c<G, 0, false>, smem_c());
-        set(k_pass_c<G, 1, false>, smem_c());
-        set(k_pass_e<G, false>, smem_ae());
-        set(k_pass_a_deposit_bal<G, false, false>, smem_bal<false>());
-        set(k_pass_a_deposit_bal<G, false, true>, smem_bal<false>());
-        if constexpr (kIsoBox) {
-            set(k_pass_y<G, false, true>, smem_bd());
-            set(k_pass_y<G, true, true>, smem_bd());
-            set(k_pass_c<G, 2, true>, smem_ct());
-            set(k_pass_e<G, true>, smem_ae());
-            set(k_pass_a_deposit_bal<G, true, false>, smem_bal<true>());
-            set(k_pass_a_deposit_bal<G, true, true>, smem_bal<true>());
+        if (use == PoissonUse::kIsolated) {
+            if constexpr (kIsoBox) {
+                set(k_pass_c<G, 1, false>, smem_c());
+                set(k_pass_y<G, false, true>, smem_bd());
+                set(k_pass_y<G, true, true>, smem_bd());
+                set(k_pass_c<G, 2, true>, smem_ct());
+                set(k_pass_e<G, true>, smem_ae());
+                set(k_pass_a_deposit_bal<G, true, false>, smem_bal<true>());
+                set(k_pass_a_deposit_bal<G, true, true>, smem_bal<true>());
+            }
+        } else {
+            set(k_pass_y<G, true, false>, smem_bd());
+            set(k_pass_c<G, 0, false>, smem_c());
+            set(k_pass_e<G, false>, smem_ae());
+        }
+        if (use == PoissonUse::kPeriodic) {
+            set(k_pass_a_deposit_bal<G, false, false>, smem_bal<false>());
+            set(k_pass_a_deposit_bal<G, false, true>, smem_bal<false>());
         }
         return rc == SD_OK ? SD_OK : SD_E_CUDA;
     }
@@ -1264,14 +1272,14 @@ int fill_gexp(float* gexp, int G, float soft, cudaStream_t st) {
     return SD_OK;
 }
 
-int poisson_configure(int G) {
+int poisson_configure(int G, PoissonUse use) {
     switch (G) {
-        case 16: return Launcher<16>::configure();
-        case 32: return Launcher<32>::configure();
-        case 64: return Launcher<64>::configure();
-        case 128: return Launcher<128>::configure();
-        case 256: return Launcher<256>::configure();
-        case 512: return Launcher<512>::configure();
+        case 16: return Launcher<16>::configure(use);
+        case 32: return Launcher<32>::configure(use);
+        case 64: return Launcher<64>::configure(use);
+        case 128: return Launcher<128>::configure(use);
+        case 256: return Launcher<256>::configure(use);
+        case 512: return Launcher<512>::configure(use);
         default: return fail(SD_E_UNSUPPORTED, "poisson: grid size %d not supported", G);
     }
 }
@@ -1324,11 +1332,11 @@ void deposit_shares(DepositWork& w, int n, int G) {
 
 size_t poisson_spectrum_elems(int G) { return (size_t)G * G * (size_t)(G / 2 + 4); }
 
-int poisson_plan_build(PoissonPlan& p, int G, float soft) {
+int poisson_plan_build(PoissonPlan& p, int G, float soft, PoissonUse use) {
     if (p.G == G && p.soft == soft && p.tw) return SD_OK;
     poisson_plan_free(p);
     // kernel attributes are set here, outside any stream capture
-    if (int rc = poisson_configure(G)) return rc;
+    if (int rc = poisson_configure(G, use)) return rc;
     std::vector<float2> tw((size_t)G);
     const double two_pi = 6.283185307179586476925286766559;
     for (int m = 0; m < G; ++m) {
@@ -1497,7 +1505,7 @@ int noalloc_setup(int dev) {
             const double a = -two_pi * (double)m / (double)G;
             row[m] = make_float2((float)cos(a), (float)sin(a));
         }
-        if (int rc = poisson_configure(G)) return rc;
+        if (int rc = poisson_configure(G, PoissonUse::kGrid)) return rc;
     }
     if (SD_CUDA(cudaMemcpy(d.tw, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice))) return SD_E_CUDA;
     d.ready = true;

@@ -107,6 +107,7 @@ int key_bits_for(int G, int order) {
 }
 
 bool isolated(const sd_sim* s) { return s->cfg.boundary == SD_BOUNDARY_ISOLATED; }
+PoissonUse poisson_use(const sd_sim* s) { return isolated(s) ? PoissonUse::kIsolated : PoissonUse::kPeriodic; }
 
 // Side of the Poisson transform box: G (periodic) or 2G (isolated, Sim.cu:3100).
 int box_of(int G, int boundary) { return boundary == SD_BOUNDARY_ISOLATED ? 2 * G : G; }
@@ -233,7 +234,7 @@ int allocate(sd_sim* s) {
         free_buffers(s);
         return rc;
     }
-    rc = poisson_plan_build(s->plan, S, s->cfg.softening_cells);
+    rc = poisson_plan_build(s->plan, S, s->cfg.softening_cells, poisson_use(s));
     // the isolated Green spectrum, with phi and the spectrum as scratch (buildGreen, Sim.cu:3569-3576)
     if (!rc && isolated(s)) rc = build_green_table(s->plan, s->cfg.softening_cells, s->phi, s->spec, s->green, s->stream);
     if (rc) {
@@ -775,7 +776,7 @@ int reconfigure(sd_sim* s, const sd_config* c) {
         if (c->keep_density && !s->rho && (rc = alloc_dev(s->rho, (size_t)s->G * s->G * s->G))) return rc;
         if ((rc = ensure_hydro(s)) || (rc = ensure_resort(s))) return rc;
         if (!soft_changed) return SD_OK;
-        rc = poisson_plan_build(s->plan, box_of(s->G, s->cfg.boundary), s->cfg.softening_cells);
+        rc = poisson_plan_build(s->plan, box_of(s->G, s->cfg.boundary), s->cfg.softening_cells, poisson_use(s));
         if (!rc && isolated(s))
             rc = build_green_table(s->plan, s->cfg.softening_cells, s->phi, s->spec, s->green, s->stream);
         return rc;
@@ -1788,7 +1789,7 @@ int sd_poisson(const float* rho, int G, float soft, float* phi, void* ws, size_t
             if (p->G == G && p->soft == soft) plan = p;
         if (!plan) {
             plan = new PoissonPlan();
-            int rc = poisson_plan_build(*plan, G, soft);
+            int rc = poisson_plan_build(*plan, G, soft, PoissonUse::kGrid);
             if (rc) {
                 delete plan;
                 return rc;
