@@ -23,19 +23,27 @@ __device__ __forceinline__ void wait_previous() { cudaGridDependencySynchronize(
 __device__ __forceinline__ void cic_axis(float p, int G, int& i, float& f) {
     const float g = __fmaf_rn(p, (float)G, -0.5f);
     const float fl = floorf(g);
-    i = (int)fl;
+    i = __float2int_rz(fl);  // saturates
     f = __fsub_rn(g, fl);
 }
 
 // Containing cell along one axis, clamped (kCellKey, Sim.cu:2482-2485).
 __device__ __forceinline__ int cell_axis(float p, int G) {
-    return min(max((int)__fmul_rn(p, (float)G), 0), G - 1);
+    return min(max(__float2int_rz(__fmul_rn(p, (float)G)), 0), G - 1);
 }
 
 // Cell index of a CIC corner: wrapped (periodic) or clamped to the edge cell
 // (isolated; gidx3, Sim.cu:96-100 -- weights past the edge land on it).
 __device__ __forceinline__ int cic_cell(int i, int G, bool periodic) {
     return periodic ? (i & (G - 1)) : min(max(i, 0), G - 1);
+}
+
+// Cell of corner o (0 or 1) of a stencil at base i. The sum is one of unsigned values: the
+// base of a coordinate beyond 2^31 cells is 2^31 - 1, and where the compiler may take a sum
+// not to overflow it clamps before it adds, and a corner of such a particle, or of one
+// at infinity, lies outside the box's memory.
+__device__ __forceinline__ int cic_corner(int i, int o, int G, bool periodic) {
+    return cic_cell((int)((unsigned)i + (unsigned)o), G, periodic);
 }
 
 // Weight of corner k = ox | oy<<1 | oz<<2, as (wx*wy)*wz (Sim.cu:515).
@@ -64,9 +72,9 @@ __device__ __forceinline__ void deposit_particle(float4 p, int G, unsigned long 
     cic_axis(p.z, G, iz, fz);
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-        const int cx = cic_cell(ix + (k & 1), G, periodic);
-        const int cy = cic_cell(iy + ((k >> 1) & 1), G, periodic);
-        const int cz = cic_cell(iz + ((k >> 2) & 1), G, periodic);
+        const int cx = cic_corner(ix, k & 1, G, periodic);
+        const int cy = cic_corner(iy, (k >> 1) & 1, G, periodic);
+        const int cz = cic_corner(iz, (k >> 2) & 1, G, periodic);
         const long long q = fixed_weight(cic_weight(k, fx, fy, fz));
         atomicAdd(acc + ((size_t)cz * G + cy) * G + cx, (unsigned long long)q);
     }

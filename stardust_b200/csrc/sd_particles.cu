@@ -161,9 +161,9 @@ __device__ __forceinline__ float3 gather_accel_iso(const float* __restrict__ phi
     float f = 0.f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-        const int cx = cic_cell(ix + (k & 1), G, false);
-        const int cy = cic_cell(iy + ((k >> 1) & 1), G, false);
-        const int cz = cic_cell(iz + ((k >> 2) & 1), G, false);
+        const int cx = cic_corner(ix, k & 1, G, false);
+        const int cy = cic_corner(iy, (k >> 1) & 1, G, false);
+        const int cz = cic_corner(iz, (k >> 2) & 1, G, false);
         const int xm = max(cx - 1, 0), xp = min(cx + 1, G - 1);
         const int ym = max(cy - 1, 0), yp = min(cy + 1, G - 1);
         const int zm = max(cz - 1, 0), zp = min(cz + 1, G - 1);
@@ -192,7 +192,7 @@ __device__ __forceinline__ float3 accel_at(const float* __restrict__ phi, int G,
     using Off = typename OffsetOf<BIG>::type;
     if (!ISO) return gather_accel<Off, true>(phi, G, G, h, ix, iy, iz, fx, fy, fz, phi_at);
     const unsigned inner = G - 3;  // 1 <= i <= G - 3 on every axis
-    if ((unsigned)(ix - 1) < inner && (unsigned)(iy - 1) < inner && (unsigned)(iz - 1) < inner)
+    if ((unsigned)ix - 1u < inner && (unsigned)iy - 1u < inner && (unsigned)iz - 1u < inner)
         return gather_accel<Off, false>(phi, G, S, h, ix, iy, iz, fx, fy, fz, phi_at);
     return gather_accel_iso(phi, G, S, h, ix, iy, iz, fx, fy, fz, phi_at);
 }
@@ -245,8 +245,8 @@ __device__ __forceinline__ float3 sample_field(const float4* __restrict__ f, int
     float3 a = make_float3(0.f, 0.f, 0.f);
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-        const int cx = cic_cell(ix + (k & 1), G, !ISO), cy = cic_cell(iy + ((k >> 1) & 1), G, !ISO),
-                  cz = cic_cell(iz + ((k >> 2) & 1), G, !ISO);
+        const int cx = cic_corner(ix, k & 1, G, !ISO), cy = cic_corner(iy, (k >> 1) & 1, G, !ISO),
+                  cz = cic_corner(iz, (k >> 2) & 1, G, !ISO);
         const float w = cic_weight(k, fx, fy, fz);
         const float4 g = f[((size_t)cz * G + cy) * G + cx];
         a.x = __fmaf_rn(g.x, w, a.x);
@@ -601,8 +601,8 @@ __global__ void __launch_bounds__(kGatherThreads) k_energy(const float* __restri
             const int R = per ? G : S;  // row stride of the potential
             double f = 0.0;
             for (int k = 0; k < 8; ++k) {
-                const int cx = cic_cell(ix + (k & 1), G, per), cy = cic_cell(iy + ((k >> 1) & 1), G, per),
-                          cz = cic_cell(iz + ((k >> 2) & 1), G, per);
+                const int cx = cic_corner(ix, k & 1, G, per), cy = cic_corner(iy, (k >> 1) & 1, G, per),
+                          cz = cic_corner(iz, (k >> 2) & 1, G, per);
                 f += (double)cic_weight(k, fx, fy, fz) * (double)phi[((size_t)cz * R + cy) * R + cx];
             }
             pe += 0.5 * f;

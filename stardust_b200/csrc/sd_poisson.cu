@@ -631,7 +631,7 @@ __device__ __forceinline__ void deposit_bundle(int b, int slice, int items, cons
             // the weights of cic_weight, scaled by 2^32 with their z factor (exact)
             const float wx[2] = {__fsub_rn(1.f, fx), fx}, wy[2] = {__fsub_rn(1.f, fy), fy};
             const float wz[2] = {__fmul_rn(__fsub_rn(1.f, fz), SD_FIXED_ONE), __fmul_rn(fz, SD_FIXED_ONE)};
-            const int x0 = cic_cell(ix, M, !ISO), x1 = cic_cell(ix + 1, M, !ISO);
+            const int x0 = cic_cell(ix, M, !ISO), x1 = cic_corner(ix, 1, M, !ISO);
             // the bundle's rows that the stencil reaches: yl + (0, 1), zl + (0, 1), each in
             // [0, 4) or not this bundle's. In the periodic box they lie at fixed distances
             // from the first one's address, whether that is in the bundle or not.
@@ -639,8 +639,8 @@ __device__ __forceinline__ void deposit_bundle(int b, int slice, int items, cons
             if (ISO) {
 #pragma unroll
                 for (int o = 0; o < 2; ++o) {
-                    yl[o] = cic_cell(iy + o, M, false) - 4 * by;
-                    zl[o] = cic_cell(iz + o, M, false) - 4 * bz;
+                    yl[o] = cic_corner(iy, o, M, false) - 4 * by;
+                    zl[o] = cic_corner(iz, o, M, false) - 4 * bz;
                 }
             } else {
                 yl[1] = (iy + 1 - 4 * by) & m;

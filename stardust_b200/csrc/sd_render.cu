@@ -19,6 +19,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "sd_common.cuh"
 #include "sd_internal.h"
 
 namespace sd {
@@ -249,11 +250,11 @@ __global__ void k_scatter_dispersion(const float4* __restrict__ pos, const float
     float ux = p.x, uy = p.y;
     if (v.rot_on && !rot_point(p.x, p.y, p.z, v, ux, uy)) return;
     const float gx = ux * G - 0.5f, gy = uy * G - 0.5f;
-    const int ix = (int)floorf(gx), iy = (int)floorf(gy);
+    const int ix = __float2int_rd(gx), iy = __float2int_rd(gy);
     const float fx = gx - ix, fy = gy - iy;
     for (int k = 0; k < 4; ++k) {
         const int ox = k & 1, oy = (k >> 1) & 1;
-        const int cx = min(max(ix + ox, 0), G - 1), cy = min(max(iy + oy, 0), G - 1);
+        const int cx = cic_corner(ix, ox, G, false), cy = cic_corner(iy, oy, G, false);
         const float w = (ox ? fx : 1.f - fx) * (oy ? fy : 1.f - fy);
         atomicAdd(reinterpret_cast<unsigned long long*>(num + cy * G + cx), (unsigned long long)to_fixed24(w * v2));
         atomicAdd(reinterpret_cast<unsigned long long*>(den + cy * G + cx), (unsigned long long)to_fixed24(w));

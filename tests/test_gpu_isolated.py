@@ -198,3 +198,31 @@ def test_isolated_deposit_of_a_pile_at_the_wall(cuda, G, n, pile, axes):
             rho[order] = s.density()
     for order in (L.SD_ORDER_ROWMAJOR, L.SD_ORDER_TILED):
         assert np.array_equal(rho[order].view(np.int32), rho[L.SD_ORDER_MORTON].view(np.int32))
+
+
+@pytest.mark.parametrize("order", [L.SD_ORDER_MORTON, L.SD_ORDER_ROWMAJOR, L.SD_ORDER_TILED])
+@pytest.mark.parametrize("G,n", [(16, 2_000), (64, 20_000)])
+def test_isolated_positions_beyond_the_integers(cuda, order, G, n):
+    """Loaded positions more than 2^31 cells outside the box are clamped onto the edge cells
+    like any outside it: the density is that of the last cell's centre, and the wall takes
+    the particles back in."""
+    pos, vel = random_particles(n, G)
+    pos[:, :3] = 0.1 + 0.8 * pos[:, :3]
+    vel[:, :3] = 0.0
+    far, near = pos.copy(), pos.copy()
+    for k, (axis, x) in enumerate([(0, 1e9), (1, 1e10), (2, 1e12), (0, 1e30), (1, 1e36), (2, 3e35)]):
+        far[97 * (k + 1), axis], near[97 * (k + 1), axis] = x, (G - 0.5) / G
+    far[700, 1], near[700, 1] = -1e30, 0.5 / G
+    far[701, :3], near[701, :3] = 1e20, (G - 0.5) / G
+    rho = []
+    for p in (near, far):
+        with iso_sim(n, G, order=order) as s:
+            s.set_particles(p, vel)
+            s.step(1e-4)
+            rho.append(s.density())
+            p1, v1 = s.get_particles()
+            assert np.isfinite(p1).all() and np.isfinite(v1).all()
+            assert p1[:, :3].min() >= 0.002 and p1[:, :3].max() <= 0.998
+            s.step(1e-4)
+            assert s.density().sum(dtype=np.float64) == pytest.approx(n, rel=1e-6)
+    assert np.array_equal(rho[0].view(np.int32), rho[1].view(np.int32))
