@@ -122,17 +122,24 @@ __host__ __device__ __forceinline__ uint32_t row_of(uint32_t key, int shift) {
     return shift < 0 ? key : (key ? ((key - 1u) >> shift) + 1u : 0u);
 }
 
-// Whether the fused deposit's windows miss a live particle: its stencil's base row is
-// not where its key's row says (only positions outside the box; see k_deposit_plan).
-__device__ __forceinline__ bool stray_row(float p, int G, int order, bool periodic) {
+// Whether the fused deposit would not add a live particle as k_deposit_fixed does (see
+// k_deposit_plan): along y or z its stencil's base row is not where its key's row says
+// (positions outside the box), or along any axis its weight is no number, which
+// two 32-bit sums do not hold. The periodic tiled order leaves such weights out.
+__device__ __forceinline__ bool stray_axis(float p, int G, int order, bool periodic, bool row) {
     int i;
     float f;
     cic_axis(p, G, i, f);
-    if (order == 0 && periodic) {
-        const int c = cell_axis(p, G);
-        return i != c && i != c - 1;
-    }
-    return order == 2 && !periodic && (i < -1 || i >= G);
+    if (order == 1 || (order == 2 && periodic)) return false;
+    if (f != f) return true;
+    if (!row || (order == 0 && !periodic)) return false;
+    if (order == 2) return i < -1 || i >= G;
+    const int c = cell_axis(p, G);
+    return i != c && i != c - 1;
+}
+__device__ __forceinline__ bool stray_particle(float4 p, int G, int order, bool periodic) {
+    return !(p.x < 0.f) && (stray_axis(p.x, G, order, periodic, false) || stray_axis(p.y, G, order, periodic, true) ||
+                            stray_axis(p.z, G, order, periodic, true));
 }
 
 __device__ __forceinline__ unsigned lanemask_lt() {

@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(kPassAThreads<G>, G == 512 ? 3 : 0)
 //   plan_done    blocks of the plan kernel done (zero between uses)
 //   ticket       next work item of the deposit's CTAs, past their first ones
 //   use          nonzero: this use deposits from the fixed-point grid (see stray)
-//   stray        nonzero: a particle sits where its row's windows do not reach (set where
+//   stray        nonzero: a particle that the bundles' sums would miss (stray_particle; set where
 //                keys are made, launch_cell_keys; cleared by the next plan)
 template <int G>
 struct DepPlan {
@@ -436,7 +436,11 @@ __device__ __forceinline__ int block_excl_scan256(int v, int* total) {
 // keys were made from such a position the stray flag is set, and this kernel deposits
 // every particle into the fixed-point grid itself, which the bundles read instead of
 // particles. Steps leave positions inside the box, so this is at most the first step
-// after a load; its speed does not matter, its not costing the others a launch does.
+// after a load; its speed does not matter, its not costing the others a launch does. A
+// position that is no number sets the flag too: its weights are, to the 64-bit sums, one
+// large value, and a step takes it as lost.
+template <bool WIDE, bool ISO>
+constexpr bool kMayStray = WIDE || ISO;
 template <int G, bool WIDE, bool ISO>
 __global__ void __launch_bounds__(256) k_deposit_plan(const int* __restrict__ rs, int* __restrict__ w, int split,
                                                       int piece, const float4* __restrict__ pos, int n,
@@ -445,9 +449,8 @@ __global__ void __launch_bounds__(256) k_deposit_plan(const int* __restrict__ rs
     using P = DepPlan<G>;
     const int b = blockIdx.x * 256 + threadIdx.x;
     int extra = 0;
-    constexpr bool kMayStray = WIDE != ISO;  // row-major periodic, tiled isolated
-    const int stray = kMayStray ? w[P::kStray] : 0;
-    if (kMayStray && stray) {
+    const int stray = kMayStray<WIDE, ISO> ? w[P::kStray] : 0;
+    if (kMayStray<WIDE, ISO> && stray) {
         split = 0x7fffffff;  // no shared bundles
         for (long long i = b; i < n; i += (long long)gridDim.x * 256) deposit_particle(pos[i], G, acc, !ISO);
     }
@@ -472,7 +475,7 @@ __global__ void __launch_bounds__(256) k_deposit_plan(const int* __restrict__ rs
             w[P::kCtaPre] = 0;
             w[P::kCtaPre + 1] = sum;
             w[P::kTicket] = 0;
-            if (kMayStray) {  // every thread has read the flag
+            if (kMayStray<WIDE, ISO>) {  // every thread has read the flag
                 w[P::kUse] = stray;
                 w[P::kStray] = 0;
             }
@@ -496,7 +499,7 @@ __global__ void __launch_bounds__(256) k_deposit_plan(const int* __restrict__ rs
         w[P::kCtaPre + P::NC] = all;
         w[P::kDone] = 0;
         w[P::kTicket] = 0;
-        if (kMayStray) {  // every block has read the flag
+        if (kMayStray<WIDE, ISO>) {  // every block has read the flag
             w[P::kUse] = stray;
             w[P::kStray] = 0;
         }
@@ -836,7 +839,7 @@ __global__ void __launch_bounds__(kDepositThreads, kDepositPerSm<G>)
     const int* xpre = w.ints + P::kXpre;
     const int* cta_pre = w.ints + P::kCtaPre;
     unsigned* arrive = reinterpret_cast<unsigned*>(w.ints + P::kArrive);
-    const bool from_grid = WIDE != ISO && w.ints[P::kUse] != 0;
+    const bool from_grid = kMayStray<WIDE, ISO> && w.ints[P::kUse] != 0;
     const int extras = cta_pre[P::NC];
     if ((int)blockIdx.x >= extras + P::NB) return;  // fewer extra shares than there can be
     for (int i = threadIdx.x; i < G; i += kDepositThreads) sm[i] = tw_g[i];  // ordered by a later barrier

@@ -52,7 +52,7 @@ constexpr int kColThreads = 256;
 constexpr int kColSegs = kColThreads / 32;  // 8 segments of a column per CTA
 
 // stray (optional): set where a particle's key does not lead the fused deposit to its
-// stencil (positions outside the box).
+// stencil, or its weights are no numbers (stray_particle).
 __global__ void __launch_bounds__(256) k_cell_keys(const float4* __restrict__ pos, int n, int G, int order,
                                                    uint32_t* __restrict__ keys, int* __restrict__ stray,
                                                    int periodic) {
@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(256) k_cell_keys(const float4* __restrict__ po
     if (i >= n) return;
     const float4 p = pos[i];
     keys[i] = order_key(p, G, order);
-    if (stray && p.x >= 0.f && (stray_row(p.y, G, order, periodic) || stray_row(p.z, G, order, periodic))) *stray = 1;
+    if (stray && stray_particle(p, G, order, periodic)) *stray = 1;
 }
 
 // Exclusive scan across a 256-thread block (of two 32-bit sums packed in 64 bits, or

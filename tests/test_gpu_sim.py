@@ -642,3 +642,32 @@ def test_deposit_shares_of_small_grids(cuda, boundary, G, n, pile):
             rho[order] = s.density()
     for order in (L.SD_ORDER_ROWMAJOR, L.SD_ORDER_TILED):
         assert np.array_equal(rho[order].view(np.int32), rho[L.SD_ORDER_MORTON].view(np.int32))
+
+
+@pytest.mark.parametrize("boundary", [L.SD_BOUNDARY_PERIODIC, L.SD_BOUNDARY_ISOLATED])
+@pytest.mark.parametrize("G,n", [(16, 4_000), (64, 50_000)])
+@pytest.mark.parametrize("rows", [False, True])
+def test_positions_that_are_no_numbers(cuda, boundary, G, n, rows):
+    """Loaded positions that are infinite or no numbers reach the density as the 64-bit
+    atomics add them (the Morton order), in the row-major order and the isolated box too,
+    and the step takes those particles as lost."""
+    pos, vel = random_particles(n, G)
+    bad = [(0, np.nan), (0, np.inf), (0, 1e38), (1, np.nan), (2, np.nan)]
+    if rows:  # and some whose rows are elsewhere
+        bad += [(1, np.inf), (1, -np.inf), (2, 1e38), (1, 1e30)]
+    for k, (axis, x) in enumerate(bad):
+        pos[37 * (k + 1), axis] = x
+    out = []
+    for order in (L.SD_ORDER_MORTON, L.SD_ORDER_ROWMAJOR) + ((L.SD_ORDER_TILED,) if boundary == L.SD_BOUNDARY_ISOLATED else ()):
+        with make_sim(cuda, n, G, gravity=1.0, softening_cells=1.0, order=order, boundary=boundary) as s:
+            s.set_particles(pos, vel)
+            s.step(1e-4)
+            rho = s.density()
+            s.step(1e-4)
+            p, v = s.get_particles()
+            key = np.argsort(v[:, 3], kind="stable")
+            out.append((rho, s.density(), p[key]))
+    assert np.abs(out[0][0]).max() > 1e9  # the bad weights are there
+    for got in out[1:]:
+        for a, b in zip(out[0], got):
+            assert np.array_equal(a.view(np.int32), b.view(np.int32))
