@@ -52,8 +52,8 @@ struct SceneSlot {
     sd_scene_tuning tuning{};
     // what the graphs were captured with; any difference makes them stale
     const float4* expect_pos = nullptr;
-    int order = 0, gather_blocks = 0, dep_split = 0, N = 0, G = 0;
-    bool mlp_on = false;
+    int order = 0, gather_blocks = 0, dep_split = 0;
+    unsigned settings = 0;
 };
 
 }  // namespace
@@ -181,9 +181,7 @@ int build_graphs(sd_ensemble* e, float dt) {
         sl.order = s->cfg.order;
         sl.gather_blocks = s->gather_blocks;
         sl.dep_split = s->dep_split;
-        sl.N = s->N;
-        sl.G = s->G;
-        sl.mlp_on = s->mlp_on;
+        sl.settings = s->settings;
     }
     return SD_OK;
 }
@@ -193,7 +191,7 @@ bool graphs_current(const sd_ensemble* e, float dt) {
     for (const auto& sl : e->scenes) {
         const sd_sim* s = sl.sim;
         if (s->pos != sl.expect_pos || s->cfg.order != sl.order || s->gather_blocks != sl.gather_blocks ||
-            s->dep_split != sl.dep_split || s->N != sl.N || s->G != sl.G || s->mlp_on != sl.mlp_on || !graphable(s))
+            s->dep_split != sl.dep_split || s->settings != sl.settings || !graphable(s))
             return false;
     }
     return true;

@@ -755,6 +755,7 @@ int reconfigure(sd_sim* s, const sd_config* c) {
     if (c->order != s->cfg.order) invalidate_keys(s);
     s->cfg = *c;
     s->cfg.grid_size = G;
+    ++s->settings;
     if (!requested || shrink) {
         if (shrink) {
             s->req_n = c->particle_count;
@@ -1177,6 +1178,7 @@ int sd_set_mlp(sd_sim* s, const float* params_device, float out_scale) {
     if (int rc_settle = settle(s)) return rc_settle;
     if (s->graph) cudaGraphExecDestroy(s->graph);  // replays must see the new setting
     s->graph = nullptr;
+    ++s->settings;
     if (!params_device) {
         s->mlp_on = false;
         return SD_OK;

@@ -106,6 +106,8 @@ struct sd_sim {
     double* diag_rec = nullptr;
     unsigned long long* diag_count = nullptr;
 
+    unsigned settings = 0;   // counts the changes that captured steps do not see (reconfigure, set_mlp)
+
     // captured steps for sd_steps
     cudaGraphExec_t graph = nullptr;
     float graph_dt = 0.f;

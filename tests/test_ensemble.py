@@ -194,3 +194,42 @@ def test_ensemble_scenes_used_between_replays(cuda, order, ask):
             sp, sv = s.get_particles()
         assert np.array_equal(p.view(np.int32), sp.view(np.int32))
         assert np.array_equal(v.view(np.int32), sv.view(np.int32))
+
+
+@pytest.mark.gpu
+def test_ensemble_scene_reconfigured_between_replays(cuda):
+    """The graphs hold a scene's gravity, softening tables and outputs: a scene that is
+    reconfigured between replays steps as a simulation with the new settings does."""
+    from stardust_b200.ensemble import Ensemble, member_config
+    from stardust_b200.scenes import disk_galaxy
+    from stardust_b200.sim import Sim
+
+    dt, scenes = 1e-3, [(20_000, 32, 1), (30_000, 64, 2)]
+
+    def config(i, changed):
+        n, G, _ = scenes[i]
+        c = member_config({"n": n, "grid": G}, keep_density=1)
+        if changed:
+            c.gravity, c.softening_cells, c.diagnostics = 3.0, 2.5, 1
+        return c
+
+    with Ensemble(0) as ens:
+        for i, (n, _, seed) in enumerate(scenes):
+            ens.add(config(i, False), *disk_galaxy(n, seed))
+        ens.steps(dt, 2)
+        ens.scene(0).reconfigure(config(0, True))
+        ens.steps(dt, 2)
+        ens.synchronize()
+        got = [ens.scene(i).get_particles() for i in range(2)]
+        assert len(ens.scene(0).diagnostics_history()) == 2
+    for i, (n, _, seed) in enumerate(scenes):
+        with Sim(0) as s:
+            s.init(config(i, False))
+            s.set_particles(*disk_galaxy(n, seed))
+            for k in range(4):
+                if k == 2 and i == 0:
+                    s.reconfigure(config(0, True))
+                s.step(dt)
+            want = s.get_particles()
+        for a, b in zip(got[i], want):
+            assert np.array_equal(a.view(np.int32), b.view(np.int32))
