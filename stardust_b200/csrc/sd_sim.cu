@@ -671,6 +671,12 @@ int do_step(sd_sim* s, float dt, bool sort, bool timed) {
     return SD_OK;
 }
 
+// The next leapfrog kick is not dt: it opens with a half kick, or the last step had another
+// size. Captured steps hold the kick of steps of one size.
+bool kick_differs(const sd_sim* s, float dt) {
+    return s->cfg.integrator == SD_INT_KDK && (!s->lf_open || s->lf_dt_prev != dt);
+}
+
 bool sort_due(const sd_sim* s) {
     return s->cfg.sort_interval > 0 && (s->step_count % s->cfg.sort_interval) == 0;
 }
@@ -1392,8 +1398,8 @@ int sd_steps(sd_sim* s, float dt, int nsteps) {
                            (!hydro_on(s) || cooling_period(s) == 2);
     int done = 0;
     update_merge_policy(s);
-    // leapfrog opening kick and odd counts run eagerly
-    while (done < nsteps && (!graphable || (s->cfg.integrator == SD_INT_KDK && !s->lf_open))) {
+    // leapfrog opening kick, a step whose kick joins half steps of two sizes, and odd counts run eagerly
+    while (done < nsteps && (!graphable || kick_differs(s, dt))) {
         int rc = do_step(s, dt, sort_due(s), false);
         if (rc) return rc;
         ++done;

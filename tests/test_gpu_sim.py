@@ -671,3 +671,25 @@ def test_positions_that_are_no_numbers(cuda, boundary, G, n, rows):
     for got in out[1:]:
         for a, b in zip(out[0], got):
             assert np.array_equal(a.view(np.int32), b.view(np.int32))
+
+
+def test_leapfrog_steps_of_changing_size(cuda):
+    """The first leapfrog step of another size kicks by half of each: replayed steps equal
+    eager ones when the size changes between calls, back to an earlier one too."""
+    G, n = 32, 30_000
+    pos, vel = random_particles(n, 8, clustered=True)
+    plan = [(1e-3, 5), (4e-4, 4), (1e-3, 4), (2e-3, 2), (1e-3, 3)]
+    outs = []
+    for eager in (True, False):
+        with make_sim(cuda, n, G, gravity=200.0, softening_cells=1.0, integrator=L.SD_INT_KDK) as s:
+            s.set_particles(pos, vel)
+            for dt, k in plan:
+                if eager:
+                    for _ in range(k):
+                        s.step(dt)
+                else:
+                    s.steps(dt, k)
+            outs.append(s.get_particles())
+            assert s.step_count() == sum(k for _, k in plan)
+    for a, b in zip(*outs):
+        assert np.array_equal(a.view(np.int32), b.view(np.int32))
