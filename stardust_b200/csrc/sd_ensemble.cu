@@ -108,18 +108,12 @@ void restore_counters(sd_sim* s, const HostCounters& c) {
     s->rho_valid = c.rho_valid;
 }
 
-// Everything a step needs that must not be inside the graph: leapfrog opening
-// kicks, and keys and first-pass sort counts where the last step's are not there any
-// more (particles loaded, a field on 512^3 that sorted for itself). Before every replay:
-// a scene may have been used on its own since the last one.
-int prepare_scenes(sd_ensemble* e, float dt) {
+// Keys and first-pass sort counts must not be inside the graph: made here where the last
+// step's are not there any more (particles loaded, a field on 512^3 that sorted for
+// itself). Before every replay: a scene may have been used on its own since the last one.
+int prepare_scenes(sd_ensemble* e) {
     for (auto& sl : e->scenes) {
         sd_sim* s = sl.sim;
-        if (!graphable(s))
-            return fail(SD_E_STATE, "ensemble: scenes must sort every step or never, without hydro add-ons");
-        if (s->cfg.integrator == SD_INT_KDK && !s->lf_open) {
-            if (int rc = do_step(s, dt, sort_due(s), false)) return rc;
-        }
         if (s->cfg.sort_interval == 1) {
             if (int rc = ensure_sort_inputs(s)) return sim_error(s, rc);
         }
@@ -414,7 +408,19 @@ int sd_ensemble_steps(sd_ensemble* e, float dt, int nsteps) {
     if (nsteps < 0) return fail(SD_E_ARG, "ensemble_steps: negative count");
     if (e->scenes.empty() || nsteps == 0) return SD_OK;
     DeviceGuard g(e->device);
-    if (int rc = prepare_scenes(e, dt)) return rc;
+    bool eager = false;
+    for (auto& sl : e->scenes) {
+        if (!graphable(sl.sim))
+            return fail(SD_E_STATE, "ensemble: scenes must sort every step or never, without hydro add-ons");
+        eager = eager || kick_differs(sl.sim, dt);
+    }
+    // a leapfrog kick other than the graphs': every scene takes this step on its own stream
+    if (eager) {
+        for (auto& sl : e->scenes)
+            if (int rc = do_step(sl.sim, dt, sort_due(sl.sim), false)) return rc;
+        --nsteps;
+    }
+    if (int rc = prepare_scenes(e)) return rc;
     // the graphs are stale when dt changed or a scene was stepped or changed on its own
     if (e->graph[0] && !graphs_current(e, dt)) drop_graphs(e);
     // work issued on the scenes' own streams so far (particle uploads, opening
@@ -423,7 +429,7 @@ int sd_ensemble_steps(sd_ensemble* e, float dt, int nsteps) {
         if (SD_CUDA(cudaEventRecord(sl.join, sl.sim->stream)) || SD_CUDA(cudaStreamWaitEvent(e->stream, sl.join, 0)))
             return SD_E_CUDA;
     }
-    if (!e->graph[0]) {
+    if (!e->graph[0] && nsteps > 0) {
         if (int rc = build_graphs(e, dt)) return rc;
     }
     for (int k = 0; k < nsteps; ++k) {

@@ -128,6 +128,7 @@ struct DeviceGuard {
 
 int sim_error(sd_sim* s, int rc);
 bool sort_due(const sd_sim* s);
+bool kick_differs(const sd_sim* s, float dt);  // the next leapfrog kick is not one of captured steps of dt
 int ensure_sort_inputs(sd_sim* s);
 void invalidate_keys(sd_sim* s);
 bool incr_possible(const sd_sim* s);

@@ -233,3 +233,46 @@ def test_ensemble_scene_reconfigured_between_replays(cuda):
             want = s.get_particles()
         for a, b in zip(got[i], want):
             assert np.array_equal(a.view(np.int32), b.view(np.int32))
+
+
+@pytest.mark.gpu
+def test_ensemble_of_leapfrog_scenes(cuda):
+    """The opening leapfrog step is one of the steps asked for, and after a closing half
+    kick or a change of the step's size the kicks are those of the scenes alone."""
+    from stardust_b200.ensemble import Ensemble, member_config
+    from stardust_b200.scenes import disk_galaxy
+    from stardust_b200.sim import Sim
+
+    scenes = [(20_000, 32, 3, L.SD_INT_KDK), (15_000, 32, 4, L.SD_INT_KD), (30_000, 64, 5, L.SD_INT_KDK)]
+
+    def config(n, G, kind):
+        c = member_config({"n": n, "grid": G})
+        c.integrator = kind
+        return c
+
+    plan = [(1e-3, 3), "synchronize", (1e-3, 1), (1e-3, 2), (5e-4, 4)]
+    with Ensemble(0) as ens:
+        for n, G, seed, kind in scenes:
+            ens.add(config(n, G, kind), *disk_galaxy(n, seed))
+        for p in plan:
+            if p == "synchronize":
+                ens.scene(0).synchronize()
+            else:
+                ens.steps(*p)
+        ens.synchronize()
+        assert [ens.scene(i).step_count() for i in range(3)] == [10, 10, 10]
+        got = [ens.scene(i).get_particles() for i in range(3)]
+    for i, (n, G, seed, kind) in enumerate(scenes):
+        with Sim(0) as s:
+            s.init(config(n, G, kind))
+            s.set_particles(*disk_galaxy(n, seed))
+            for p in plan:
+                if p == "synchronize":
+                    if i == 0:
+                        s.synchronize()
+                else:
+                    for _ in range(p[1]):
+                        s.step(p[0])
+            want = s.get_particles()
+        for a, b in zip(got[i], want):
+            assert np.array_equal(a.view(np.int32), b.view(np.int32))
