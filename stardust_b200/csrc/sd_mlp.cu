@@ -385,7 +385,6 @@ struct Smem {
     float colsum[kWarps][2 * kH + kOut + 1];
 };
 
-
 // acc (16 x 64) += A (16 x 16 KS, fragments) * W[k][n] (rows of kS elements)
 template <int KS>
 __device__ __forceinline__ void mul_w(float (&acc)[8][4], const unsigned (&a)[KS][4], const __nv_bfloat16* w,
@@ -674,8 +673,7 @@ __global__ void __launch_bounds__(256) k_train_reduce(const float* __restrict__ 
     }
 }
 
-__global__ void k_adam(
-float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
+__global__ void k_adam(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
                        const float* __restrict__ grad, int n, float lr, float b1, float b2, float eps, float c1,
                        float c2) {
     wait_previous();
@@ -701,13 +699,13 @@ int launch_mlp_infer(const float* params, const float4* pos, const int* perm, in
     if (table) {
         const size_t quads = (size_t)G * G * G / 4;
         launch(k_feature_table, (unsigned)((quads + 255) / 256), 256, 0, s, reinterpret_cast<const float4*>(rho), quads,
-                                                                        inv_mean, reinterpret_cast<uint2*>(table));
+               inv_mean, reinterpret_cast<uint2*>(table));
         SD_LAUNCHED(s);
         launch(k_mlp_infer<true>, blocks, inf::kThreads, 0, s, params, pos, perm, n, rho, table, G, inv_mean, out_scale,
-                                                           out);
+               out);
     } else {
         launch(k_mlp_infer<false>, blocks, inf::kThreads, 0, s, params, pos, perm, n, rho, nullptr, G, inv_mean, out_scale,
-                                                            out);
+               out);
     }
     SD_LAUNCHED(s);
     return SD_OK;
@@ -738,7 +736,7 @@ int sd_mlp_features(const float* pos, const int32_t* perm, int n, const float* r
     if (n == 0) return SD_OK;
     cudaStream_t st = (cudaStream_t)stream;
     launch(k_features, (n + 255) / 256, 256, 0, st, reinterpret_cast<const float4*>(pos), perm, n, rho, G, inv_mean,
-                                                 reinterpret_cast<__nv_bfloat16*>(features_bf16));
+           reinterpret_cast<__nv_bfloat16*>(features_bf16));
     SD_LAUNCHED(st);
     return SD_OK;
 }
@@ -771,7 +769,7 @@ int sd_mlp_loss_grad(const float* params, const void* features_bf16, const float
     if (SD_CUDA(cudaFuncSetAttribute(k_train_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(tr::Smem))))
         return SD_E_CUDA;
     launch(k_train_tile, ctas, tr::kThreads, sizeof(tr::Smem), st,
-        params, reinterpret_cast<const __nv_bfloat16*>(features_bf16), targets, rows, part);
+           params, reinterpret_cast<const __nv_bfloat16*>(features_bf16), targets, rows, part);
     SD_LAUNCHED(st);
     launch(k_train_reduce, (kParams + 1 + 63) / 64, 256, 0, st, part, ctas, grad, sse);
     SD_LAUNCHED(st);

@@ -523,7 +523,8 @@ __global__ void k_apply_mean(float4* __restrict__ vel, const float4* __restrict_
 
 // Largest |v| of the live particles into *out (zeroed before). Grid-stride with two
 // particles in flight per thread, one atomic per CTA: with one per warp, 65,536 atomics
-// on one address took most of 52 us at 2,000,000 particles; now 10.9 us (64 MB read). The square root is monotone, so it is taken once, of the largest |v|^2.
+// on one address took most of 52 us at 2,000,000 particles; now 10.9 us (64 MB read). The
+// square root is monotone, so it is taken once, of the largest |v|^2.
 constexpr int kSpeedCtasPerSm = 8;
 __global__ void __launch_bounds__(256) k_max_speed(const float4* __restrict__ pos, const float4* __restrict__ vel,
                                                    int n, const float* __restrict__ mean_vel,
@@ -725,7 +726,7 @@ size_t deposit_workspace_bytes(int G) { return align_up(sizeof(long long) * (siz
 int launch_deposit_fixed(const float4* pos, int n, int G, long long* acc, cudaStream_t s, int periodic) {
     if (n <= 0) return SD_OK;
     launch(k_deposit_fixed, (n + 255) / 256, 256, 0, s, pos, n, G, reinterpret_cast<unsigned long long*>(acc),
-                                                     periodic);
+           periodic);
     SD_LAUNCHED(s);
     return SD_OK;
 }
@@ -791,7 +792,7 @@ int launch_gather_kick_drift(const float* phi, int G, float pot_scale, const flo
     const int cap = max_blocks > 0 ? max_blocks : gather_wave();
     if (blocks > cap) blocks = cap;
     const bool dg = diag && partials;
-    // change bits serve the merge sort of the periodic tiled order only
+    // change bits serve the merge sort, which the isolated box does without
     if (chg_words && (iso_S || tile_counts || !keys_out))
         return fail(SD_E_ARG, "gather: change bits need keys, no tile counts and the periodic box");
     const int keys_mode = chg_words ? kKeysChanged : (tile_counts ? kKeysCounts : kKeysPlain);
@@ -809,8 +810,8 @@ int launch_gather_kick_drift(const float* phi, int G, float pot_scale, const flo
     if (!iso_S && G > 1024) {  // the simulation's grids end at 512: a stage call, plain
         if (dg || press || keys_mode != kKeysPlain) return fail(SD_E_UNSUPPORTED, "gather: grid %d above 1024", G);
         launch(k_gather_kick_drift<false, false, false, kKeysPlain, true>, blocks, kGatherThreads, 0, s,
-            phi, G, h, pos_in, vel_in, perm, pos_out, vel_out, keys_out, order, n, dt_kick, dt_drift, c2, mean_vel,
-            partials, extra, iso_S, tile_counts, count_bits, press, chg_words);
+               phi, G, h, pos_in, vel_in, perm, pos_out, vel_out, keys_out, order, n, dt_kick, dt_drift, c2, mean_vel,
+               partials, extra, iso_S, tile_counts, count_bits, press, chg_words);
     } else if (iso_S) {
         if (dg) { SD_GATHER_P(true, true); }
         else { SD_GATHER_P(false, true); }
@@ -824,7 +825,7 @@ int launch_gather_kick_drift(const float* phi, int G, float pot_scale, const flo
     SD_LAUNCHED(s);
     if (dg) {
         launch(k_finalize_mean<6>, 1, 256, 0, s, partials, blocks, mom_out, mean_out, diag->rec, diag->count, diag->cap,
-                                            diag->mass, (double)pot_scale);
+               diag->mass, (double)pot_scale);
         SD_LAUNCHED(s);
     } else if (partials && (mom_out || mean_out)) {
         launch(k_finalize_mean<4>, 1, 256, 0, s, partials, blocks, mom_out, mean_out, nullptr, nullptr, 1, 0.0, 0.0);

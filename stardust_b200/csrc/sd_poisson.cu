@@ -337,7 +337,8 @@ struct DepPlan {
     static constexpr int NB = G * G / 16;
     static constexpr int NC = (NB + 255) / 256;
     static constexpr int kItems = 0, kXpre = NB, kArrive = 2 * NB, kCtaSum = 3 * NB, kCtaPre = 3 * NB + NC,
-                         kDone = 3 * NB + 2 * NC + 1, kTicket = kDone + 1, kUse = kTicket + 1, kStray = kUse + 1, kInts = kStray + 1;
+                         kDone = 3 * NB + 2 * NC + 1, kTicket = kDone + 1, kUse = kTicket + 1, kStray = kUse + 1,
+                         kInts = kStray + 1;
 };
 
 // Where the particles of a bundle's window sit among the sorted ones, as kRanges
@@ -1145,7 +1146,7 @@ struct Launcher {
         const long long extra = 4ll * dw.n / piece, wave = 148 * kDepositPerSm<G>;
         const long long ctas = P::NB + (extra < 8 ? 8 : extra);
         launch(k_pass_a_deposit_bal<G, ISO, WIDE>, (unsigned)(kDepositLoop<G> && ctas > wave ? wave : ctas), kDepositThreads,
-                                             smem_bal<ISO>(), s, pos, perm, row_start, keep, spec, p.tw, dw);
+               smem_bal<ISO>(), s, pos, perm, row_start, keep, spec, p.tw, dw);
         SD_LAUNCHED(s);
         return SD_OK;
     }
@@ -1199,7 +1200,8 @@ struct Launcher {
         // full box's traffic (a 256^3 box: A 39 -> 19 us, B 27 -> 13, C 42 -> 29, D 27 -> 13,
         // E 33 -> 9; a 512^3 box: 266 -> 90, 210 -> 112, 402 -> 253, 210 -> 88, 234 -> 55).
         const bool half = kIsoBox && iso && iso->table && 2 * src_g == G;
-        if (iso && iso->table && !half) return fail(SD_E_ARG, "poisson: the isolated density has half the box's side");
+        if (iso && iso->table && !half)
+            return fail(SD_E_ARG, "poisson: the isolated density has half the box's side");
         const int hy = half ? T::NBY / 2 : T::NBY, hz = half ? T::NBZ / 2 : T::NBZ;
         const dim3 grid_rows(hy, hz), grid_y(T::NBX, hz), grid_z(T::NBX, T::NBY);
         if (pos) {
@@ -1217,7 +1219,7 @@ struct Launcher {
         } else {
             if (acc)
                 launch(k_pass_a<G, 1>, grid_rows, kPassAThreads<G>, smem_a(), s, nullptr, const_cast<long long*>(acc), keep,
-                                                                         spec, p.tw, src_g);
+                       spec, p.tw, src_g);
             else
                 launch(k_pass_a<G, 0>, grid_rows, kPassAThreads<G>, smem_a(), s, rho, nullptr, keep, spec, p.tw, src_g);
             SD_LAUNCHED(s);
@@ -1229,7 +1231,7 @@ struct Launcher {
                 SD_LAUNCHED(s);
                 if (ev) cudaEventRecord(ev[1], s);
                 launch(k_pass_c<G, 2, true>, grid_z, kFftThreads, smem_ct(), s, spec, p.tw, p.gexp, p.scale, iso->table,
-                                                                           iso->table_scale);
+                       iso->table_scale);
                 SD_LAUNCHED(s);
                 if (ev) cudaEventRecord(ev[2], s);
                 launch(k_pass_y<G, true, true>, grid_y, kFftThreads, smem_bd(), s, spec, p.tw);

@@ -376,7 +376,7 @@ int launch_resort(const ResortBufs& r, const uint32_t* keys, int n, int G, int o
     launch(k_chg_count, chunks, kChgThreads, 0, s, r.words, r.chunk_cnt);
     SD_LAUNCHED(s);
     launch(k_chg_compact, chunks, kCompactThreads, 0, s, r.words, r.chunk_cnt, keys, r.word_pre, r.ck_in, r.ci_in,
-                                                 r.n_changed);
+           r.n_changed);
     SD_LAUNCHED(s);
     // C by key, stable: the radix sort with the count on the device
     int rc = launch_sort_pairs(r.ck_in, r.ci_in, r.ck_out, r.ci_out, r.ck_tmp, r.ci_tmp, n, key_bits, sort_ws,
@@ -384,15 +384,15 @@ int launch_resort(const ResortBufs& r, const uint32_t* keys, int n, int G, int o
     if (rc) return rc;
     auto changed = shift < 0 ? k_merge_changed<false> : k_merge_changed<true>;
     launch(changed, 148 * 4, 256, 0, s, r.ck_out, r.ci_out, r.n_changed, keys, shift, row_start, r.words, r.word_pre,
-                                    vals_out);
+           vals_out);
     SD_LAUNCHED(s);
     launch(k_rows, (rows + 1 + 255) / 256, 256, 0, s, r.ck_out, r.n_changed, rows, shift, r.words, r.word_pre, r.c_rows,
-                                                   row_start);
+           row_start);
     SD_LAUNCHED(s);
     const int warps = (n + 255) / 256;
     auto unchanged = shift < 0 ? k_merge_unchanged<false> : k_merge_unchanged<true>;
     launch(unchanged, (warps + kMergeThreads / 32 - 1) / (kMergeThreads / 32), kMergeThreads, 0, s,
-        keys, r.words, r.word_pre, r.c_rows, shift, r.ck_out, r.ci_out, n, vals_out);
+           keys, r.words, r.word_pre, r.c_rows, shift, r.ck_out, r.ci_out, n, vals_out);
     SD_LAUNCHED(s);
     return SD_OK;
 }

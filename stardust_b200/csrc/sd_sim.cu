@@ -189,7 +189,7 @@ size_t estimate_bytes(int n, int G, int boundary) {
     b += sizeof(float) * (box + cells);                // phi, kept density
     if (S != G) b += sizeof(float) * green_table_elems(S);
     b += sizeof(double) * 8 * (gather_partials((int)N) + 1024);
-    if (S == G) b += resort_bytes((int)N, G);  // the merge sort (periodic box, tiled order)
+    if (S == G) b += resort_bytes((int)N, G);  // the merge sort (periodic box; made from merge_min_particles up)
     return b;
 }
 
@@ -497,9 +497,13 @@ int do_sort(sd_sim* s, int32_t* perm_out_dev) {
 
 // Field for the current positions: deposit + Poisson -> phi (computeAccel, Sim.cu:3605-3633).
 // On a 512^3 grid the particles are sorted by tiled row for it, so that pass A deposits
-// them itself: the int64 grid, 1 GB to read and clear again, costs more than the sort
-// (2,097,152 particles: atomics and pass A 0.64 ms, keys, sort and fused deposit 0.46).
-// Smaller grids come out even or worse.
+// them itself: the int64 grid, 1 GB to read and clear again, costs more than the sort at any
+// count. Forces with the grid and with the sort, in ms: 1,000 particles 1.44 and 1.24;
+// 131,072 1.53 and 1.30; 2,097,152 in no order 2.50 and 1.94, after a step 1.80 and 1.40;
+// 16,777,216 9.7 and 7.0, after a step 2.6 and 2.1. On 256^3 it depends on the particles: 1,000
+// 0.20 and 0.23; 2,097,152 evenly spread 0.59 and 0.48, in eight clumps 0.44 and 0.50;
+// 16,777,216 in clumps 2.06 and 2.66, after a step 1.30 and 0.90. On 128^3 the sort loses nearly
+// everywhere (2,097,152 evenly spread 0.27 and 0.34).
 int do_field(sd_sim* s, bool keep) {
     int rc = SD_OK;
     const bool fused = !isolated(s) && s->G == 512;

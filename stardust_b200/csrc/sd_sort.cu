@@ -650,7 +650,7 @@ static int scan_offsets(unsigned* counts, int tiles, int radix, const SortWs& w,
     const int chunks = col_chunks(tiles);
     if (!sums_ready) {
         launch(k_col_sums, dim3(chunks, (radix + kColThreads - 1) / kColThreads), kColThreads, 0, s, counts, tiles, radix,
-                                                                                               w.S);
+               w.S);
         SD_LAUNCHED(s);
     }
     launch(k_col_prefix, slabs, kColThreads, 0, s, w.S, chunks, radix, w.T, w.done);
