@@ -1205,7 +1205,8 @@ struct Launcher {
         const int hy = half ? T::NBY / 2 : T::NBY, hz = half ? T::NBZ / 2 : T::NBZ;
         const dim3 grid_rows(hy, hz), grid_y(T::NBX, hz), grid_z(T::NBX, T::NBY);
         if (pos) {
-            if (!dw || !dw->acc || !dw->ints || dw->split <= 0 || dw->piece <= 0) return fail(SD_E_ARG, "fused deposit: no work plan");
+            if (!dw || !dw->acc || !dw->ints || dw->split <= 0 || dw->piece <= 0)
+                return fail(SD_E_ARG, "fused deposit: no work plan");
             int rc = SD_OK;
             if constexpr (kIsoBox) {
                 if (half)
