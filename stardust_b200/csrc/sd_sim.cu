@@ -1228,11 +1228,9 @@ int sd_step_host(sd_sim* s, const float* pos_in, const float* vel_in, int n, flo
         return fail(SD_E_ARG, "step_host: bad arguments (n=%d)", n);
     DeviceGuard g(s->device);
     if (int rc_settle = settle(s)) return rc_settle;
-    if (!s->io_stream) {
-        if (SD_CUDA(cudaStreamCreateWithFlags(&s->io_stream, cudaStreamNonBlocking))) return SD_E_CUDA;
-        for (auto& e : s->io_ev)
-            if (SD_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming))) return SD_E_CUDA;
-    }
+    if (!s->io_stream && SD_CUDA(cudaStreamCreateWithFlags(&s->io_stream, cudaStreamNonBlocking))) return SD_E_CUDA;
+    for (auto& e : s->io_ev)  // the stream may be there without them (sd_step_host_async)
+        if (!e && SD_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming))) return SD_E_CUDA;
     const size_t bytes = sizeof(float4) * (size_t)n;
     cudaStream_t st = s->stream, io = s->io_stream;
     // Inputs: the positions first, at the link's full speed, on the handle's

@@ -693,3 +693,21 @@ def test_leapfrog_steps_of_changing_size(cuda):
             assert s.step_count() == sum(k for _, k in plan)
     for a, b in zip(*outs):
         assert np.array_equal(a.view(np.int32), b.view(np.int32))
+
+
+def test_offload_step_after_pipelined_ones(cuda):
+    """The two offload calls share a stream: either may come first."""
+    import torch
+
+    G, n, dt = 32, 20_000, 1e-3
+    pos, vel = (torch.from_numpy(a).pin_memory() for a in random_particles(n, 3))
+    out = [tuple(torch.empty_like(pos).pin_memory() for _ in range(2)) for _ in range(3)]
+    with make_sim(cuda, n, G, gravity=10.0, softening_cells=1.0) as s:
+        s.step_host_async(pos, vel, dt, out[0])
+        s.step_host_wait()
+        s.step_host(pos, vel, dt, out[1])
+        s.step_host_async(pos, vel, dt, out[2])
+        s.step_host_wait()
+    for o in out[1:]:
+        for a, b in zip(out[0], o):
+            assert np.array_equal(a.numpy().view(np.int32), b.numpy().view(np.int32))
